@@ -55,6 +55,8 @@ enum Ctl : int {
   C_CHECKSUM = 11,
   C_AUX = 12,
   C_EDGES = 13,    // edge slots scanned by push levels (work counter)
+  C_BND0 = 14,     // bound on the values in queue 0: none of them is better than this
+  C_BND1 = 15,     // ... in queue 1
   // device-driven level loop (written by k_level_begin, read by level kernels)
   C_LEVEL = 16,    // levels run in the current loop
   C_STAMP = 17,    // frontier dedup stamp of the current level
@@ -255,6 +257,21 @@ struct HistNode {
   uint64_t value;
 };
 
+// Row counts and slice bounds of the sliced-ELL in-edge copy.  Rows are sorted
+// by length, longest first, so everything about the slices follows from the
+// number of rows of each length: slices [slice[L], slice[L - 1]) are L entries
+// wide and start at entry base[L] of the copy.
+constexpr uint32_t PULL_HUB = 576;  // longest row
+constexpr int SELL_BINS = (int)PULL_HUB + 1;
+struct SellPlan {
+  unsigned long long hubs, pieces;      // vertices cut into pieces, and their pieces
+  unsigned long long rows, slices, total;  // non-empty rows, slices, entries (padding included)
+  unsigned long long base[SELL_BINS];   // first entry of the slices of width L
+  uint32_t count[SELL_BINS];            // rows of length L
+  uint32_t cursor[SELL_BINS];           // where the next row of length L goes
+  uint32_t slice[SELL_BINS];            // first slice of width <= L
+};
+
 // A cached, instantiated level-loop graph.
 struct LoopGraph {
   cudaGraphExec_t exec = nullptr;
@@ -310,11 +327,9 @@ struct Graph {
   uint64_t sell_piece_cap = 0;
   ulonglong2 *sell_piece_best = nullptr;  // best {value, parent | w << 32} of each piece in a pull level
   uint64_t sell_best_cap = 0;
-  unsigned long long *sell_cnt = nullptr;
-  uint64_t sell_hubs = 0, sell_rows = 0, sell_slices = 0, sell_epoch = 0;
-  uint64_t sell_cls[3] = {0, 0, 0};  // first slice of width <= 8, 4, 2
-  uint64_t sell_split = 0;           // first slice of the second launch of a pull level
-  std::vector<uint64_t> sell_off_host;  // host copy of sell_off (launch bounds of grouped pull levels)
+  SellPlan *sell_plan = nullptr;     // row counts and slice bounds of the copy, on the device ...
+  SellPlan *sell_plan_host = nullptr;  // ... and pinned on the host
+  uint64_t sell_epoch = 0;  // bumped when cached loop graphs hold old addresses of the copy
   uint64_t pull_groups = 2;          // launches of a split pull level (RG_OPT_PULL_GROUPS)
   uint64_t pull_div = 64;
   int pull_split = 2;  // two-launch pull levels: 1 always, 0 never, 2 SSSP and WCC

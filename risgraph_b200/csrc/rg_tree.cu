@@ -610,7 +610,6 @@ __global__ void __launch_bounds__(DN_TPB, 3) k_push_dense(DevGraph g, const uint
 // no atomics on labels: a vertex row is written only by its own lane; a piece
 // leaves its best in a side array and k_pull_hub_fix combines the pieces of
 // each hub.
-constexpr uint32_t PULL_HUB = 576;
 constexpr int PS_TPB = 256;
 // Split pull levels (RG_OPT_PULL_SPLIT): a level runs in two launches, first
 // the slices of the longest in-lists (width >= PULL_SPLIT: the hubs and their
@@ -632,13 +631,9 @@ constexpr int PS_TPB = 256;
 constexpr uint32_t PULL_SPLIT = 288;
 // every hub piece (at least PULL_HUB / 2 entries) must fall in the first launch
 static_assert(PULL_SPLIT <= PULL_HUB / 2, "hub pieces must be pulled before k_pull_hub_fix");
-// In-list entries a lane keeps in flight: 16 for 8-byte weighted entries; 8 for
-// 4-byte ones, plus the next 8 prefetched (measured best on RMAT-22).
-template <bool W>
-struct PullDepth {
-  static constexpr int N = W ? 16 : 8;
-  static constexpr bool prefetch = !W;
-};
+// Entries of a row that a lane reads at a time.
+constexpr int PULL_DEPTH = 8;
+constexpr int PULL_CTAS = 4;  // resident CTAs per SM that the pull kernel's registers allow
 
 template <bool W>
 struct SellE;
@@ -662,305 +657,572 @@ struct SellE<false> {
 // Pieces of a hub of in-list length len: equal lengths of at most PULL_HUB.
 __device__ __forceinline__ uint32_t hub_pieces(uint32_t len) { return (len + PULL_HUB - 1) / PULL_HUB; }
 
-// Hubs (in-list longer than PULL_HUB) with their piece counts.
-__global__ void k_sell_hubs(DevGraph g, uint32_t *hub_v, uint64_t *hub_np, unsigned long long *cnt) {
+// The copy is laid out in three passes over the vertices' list lengths: count
+// the rows of each length (k_sell_count), turn the counts into row and slice
+// positions (k_sell_plan, one block), and put each row in its place
+// (k_sell_rows).  Lengths are at most PULL_HUB, so a histogram in shared memory
+// replaces a sort of all vertices, and the host waits once, for the plan, to
+// size the arrays.  (RMAT-20, 16M weighted edges: the whole preparation takes
+// 0.25 ms; 8.0 ms with a radix sort, five host synchronisations, temporary
+// allocations and one thread copying each row.)
+__global__ void __launch_bounds__(1024) k_sell_count(DevGraph g, uint32_t *hub_v, uint64_t *hub_pc, SellPlan *plan) {
+  __shared__ uint32_t s_n[SELL_BINS];
+  for (int b = threadIdx.x; b < SELL_BINS; b += blockDim.x) s_n[b] = 0;
+  __syncthreads();
   const uint64_t V = g.V;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += stride) {
     const uint32_t d = seg_len(g.in, (uint32_t)v);
     if (d > PULL_HUB) {
-      const unsigned long long h = atomicAdd(cnt, 1ull);
+      const uint32_t np = hub_pieces(d), base = d / np, extra = d % np;
+      const unsigned long long h = atomicAdd(&plan->hubs, 1ull);
       hub_v[h] = (uint32_t)v;
-      hub_np[h] = hub_pieces(d);
+      hub_pc[h] = atomicAdd(&plan->pieces, (unsigned long long)np) | ((uint64_t)np << 32);
+      atomicAdd(&s_n[base], np - extra);
+      if (extra) atomicAdd(&s_n[base + 1], extra);
+    } else if (d) {
+      atomicAdd(&s_n[d], 1u);
     }
   }
+  __syncthreads();
+  for (int b = threadIdx.x; b < SELL_BINS; b += blockDim.x)
+    if (s_n[b]) atomicAdd(&plan->count[b], s_n[b]);
 }
 
-// Row keys of the vertices: in-list length, 0 for hubs (their rows are pieces).
-__global__ void k_sell_keys(DevGraph g, uint32_t *key, uint32_t *id) {
-  const uint64_t V = g.V;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += stride) {
-    const uint32_t d = seg_len(g.in, (uint32_t)v);
-    key[v] = d > PULL_HUB ? 0u : d;
-    id[v] = (uint32_t)v;
+// Rows of length L take the positions after all longer ones; slices are 32
+// consecutive rows, as wide as their first.
+__global__ void __launch_bounds__(1024) k_sell_plan(SellPlan *plan) {
+  using Scan = cub::BlockScan<uint64_t, 1024>;
+  __shared__ typename Scan::TempStorage tmp;
+  const int t = threadIdx.x, L = (int)PULL_HUB - t;  // longest first
+  const uint64_t n = L >= 1 ? plan->count[L] : 0;
+  uint64_t row, rows;
+  Scan(tmp).ExclusiveSum(n, row, rows);
+  const uint64_t s0 = (row + 31) / 32, s1 = (row + n + 31) / 32;
+  __syncthreads();
+  uint64_t base, total;
+  Scan(tmp).ExclusiveSum(L >= 1 ? 32 * (uint64_t)L * (s1 - s0) : 0, base, total);
+  if (L >= 1) {
+    plan->cursor[L] = (uint32_t)row;
+    plan->slice[L] = (uint32_t)s0;
+    plan->base[L] = base;
+  }
+  if (t == 0) {
+    plan->rows = rows;
+    plan->slices = (rows + 31) / 32;
+    plan->total = total;
+    plan->slice[0] = (uint32_t)((rows + 31) / 32);
   }
 }
 
-// Piece rows of every hub (id V + piece index), their keys and the piece table.
-__global__ void k_sell_pieces(DevGraph g, const uint32_t *hub_v, const uint64_t *piece_off, uint64_t nh, uint32_t *key,
-                              uint32_t *id, uint32_t *piece_v, uint32_t *piece_start, uint32_t *piece_len) {
+// Row ids (a vertex, or |V| + a piece of a hub) in their places, the piece
+// table, and the slice offsets.  A block reserves the places of its rows of
+// one length together, which keeps rows of near vertices near each other.
+constexpr int SR_TPB = 512, SR_ITEMS = 8;
+
+__global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
+                                                      SellPlan *plan, uint32_t *row_id, uint32_t *piece_v,
+                                                      uint32_t *piece_start, uint32_t *piece_len, uint64_t *off) {
+  __shared__ uint32_t s_n[SELL_BINS], s_at[SELL_BINS];
   const uint64_t V = g.V;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t h = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; h < nh; h += stride) {
+  constexpr uint64_t TILE = SR_TPB * SR_ITEMS;
+  for (uint64_t b0 = blockIdx.x * TILE; b0 < V; b0 += gridDim.x * TILE) {
+    for (int b = threadIdx.x; b < SELL_BINS; b += SR_TPB) s_n[b] = 0;
+    __syncthreads();
+    uint32_t d[SR_ITEMS], at[SR_ITEMS];
+#pragma unroll
+    for (int k = 0; k < SR_ITEMS; k++) {
+      const uint64_t v = b0 + (uint64_t)k * SR_TPB + threadIdx.x;
+      d[k] = v < V ? seg_len(g.in, (uint32_t)v) : 0u;
+      if (d[k] > PULL_HUB) d[k] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < SR_ITEMS; k++) at[k] = d[k] ? atomicAdd(&s_n[d[k]], 1u) : 0u;
+    __syncthreads();
+    for (int b = threadIdx.x; b < SELL_BINS; b += SR_TPB)
+      s_at[b] = s_n[b] ? atomicAdd(&plan->cursor[b], s_n[b]) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SR_ITEMS; k++)
+      if (d[k]) row_id[s_at[d[k]] + at[k]] = (uint32_t)(b0 + (uint64_t)k * SR_TPB + threadIdx.x);
+    __syncthreads();
+  }
+  // one warp per hub writes its pieces
+  const int lane = lane_id();
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t nh = plan->hubs;
+  for (uint64_t h = warp; h < nh; h += nwarps) {
     const uint32_t v = hub_v[h];
-    const uint32_t d = seg_len(g.in, v);
-    const uint64_t p0 = piece_off[h];
-    const uint32_t np = hub_pieces(d), base = d / np, extra = d % np;
-    uint32_t start = 0;
-    for (uint32_t k = 0; k < np; k++) {
-      const uint32_t n = base + (k < extra ? 1u : 0u);
-      key[V + p0 + k] = n;
-      id[V + p0 + k] = (uint32_t)(V + p0 + k);
+    const uint32_t dv = seg_len(g.in, v);
+    const uint64_t pc = hub_pc[h];
+    const uint32_t p0 = (uint32_t)pc, np = (uint32_t)(pc >> 32), base = dv / np, extra = dv % np;
+    uint32_t a1 = 0, a0 = 0;  // the first `extra` pieces are one longer
+    if (lane == 0) {
+      if (extra) a1 = atomicAdd(&plan->cursor[base + 1], extra);
+      a0 = atomicAdd(&plan->cursor[base], np - extra);
+    }
+    a1 = __shfl_sync(FULL, a1, 0);
+    a0 = __shfl_sync(FULL, a0, 0);
+    for (uint32_t k = lane; k < np; k += 32) {
       piece_v[p0 + k] = v;
-      piece_start[p0 + k] = start;
-      piece_len[p0 + k] = n;
-      start += n;
+      piece_start[p0 + k] = k * base + min(k, extra);
+      piece_len[p0 + k] = base + (k < extra ? 1u : 0u);
+      row_id[k < extra ? a1 + k : a0 + (k - extra)] = (uint32_t)(V + p0 + k);
     }
   }
-}
-
-__global__ void k_sell_count(const uint32_t *key, uint64_t n, unsigned long long *rows) {
+  const uint64_t ns = plan->slices;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += stride) {
-    const uint64_t i = base + threadIdx.x;
-    const unsigned b = __ballot_sync(FULL, i < n && key[i] > 0);
-    if (lane_id() == 0 && b) atomicAdd(rows, (unsigned long long)__popc(b));
+  for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s <= ns; s += stride) {
+    int lo = 1, hi = (int)PULL_HUB;  // the narrowest width L with slice[L] <= s
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (plan->slice[mid] <= s) hi = mid;
+      else lo = mid + 1;
+    }
+    off[s] = s < ns ? plan->base[lo] + (s - plan->slice[lo]) * 32 * lo : plan->total;
   }
 }
 
-// Slice sizes (entries): 32 x the length of the slice's first (longest) row.
-__global__ void k_sell_sizes(const uint32_t *sorted_key, uint64_t slices, uint64_t *size) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s <= slices; s += stride)
-    size[s] = s < slices ? 32ull * sorted_key[s * 32] : 0;
+// Weight classes of the entry order: 0 to 127 exactly, then sixteen to each
+// power of two (device weights are below 2^31, so there are 512).  w_floor /
+// w_ceil: the smallest / largest weight of w's class.
+constexpr int W_CLASSES = 512;
+__device__ __forceinline__ uint32_t w_class(uint32_t w) {
+  if (w < 128) return w;
+  const uint32_t e = 31 - __clz(w);
+  return (128 + 16 * (e - 7) + ((w >> (e - 4)) & 15)) & (W_CLASSES - 1);
+}
+__device__ __forceinline__ uint32_t w_floor(uint32_t w) {
+  return w < 128 ? w : w & ~((1u << (27 - __clz(w))) - 1u);
+}
+__device__ __forceinline__ uint32_t w_ceil(uint32_t w) {
+  return w < 128 ? w : w | ((1u << (27 - __clz(w))) - 1u);
 }
 
-// Copy the live in-entries of each row into its column; pad with NONE.
+// Where row r's entries come from.
+struct RowSrc {
+  uint64_t from;
+  uint32_t n;
+};
+__device__ __forceinline__ RowSrc sell_row_src(const DevGraph &g, const uint32_t *row_id, uint64_t r, uint64_t rows,
+                                               const uint32_t *piece_v, const uint32_t *piece_start,
+                                               const uint32_t *piece_len) {
+  RowSrc s = {0, 0};
+  if (r < rows) {
+    const uint32_t id = row_id[r];
+    if (id < g.V) {
+      s.from = g.in.off[id];
+      s.n = seg_len(g.in, id);
+    } else {
+      const uint32_t p = id - g.V;
+      s.from = g.in.off[piece_v[p]] + piece_start[p];
+      s.n = piece_len[p];
+    }
+  }
+  return s;
+}
+
+// Copy the live in-entries of each row of slices [s_lo, s_hi) into its column;
+// pad with NONE.  One thread per row, in the order of the pool: for narrow
+// rows, and for rows without weights.
 template <bool W>
-__global__ void k_sell_fill(DevGraph g, const uint32_t *row_id, uint64_t rows, uint64_t slices, const uint64_t *off,
-                            const uint32_t *piece_v, const uint32_t *piece_start, const uint32_t *piece_len,
-                            typename SellE<W>::E *ent) {
+__global__ void k_sell_fill(DevGraph g, const uint32_t *row_id, uint64_t rows, uint64_t s_lo, uint64_t s_hi,
+                            const uint64_t *off, const uint32_t *piece_v, const uint32_t *piece_start,
+                            const uint32_t *piece_len, typename SellE<W>::E *ent) {
   using P_ = PoolT<W>;
   using S_ = SellE<W>;
   const typename P_::E *pool = reinterpret_cast<const typename P_::E *>(g.in.pool);
-  const uint64_t V = g.V;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < slices * 32; r += stride) {
+  for (uint64_t r = s_lo * 32 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < s_hi * 32; r += stride) {
     const uint64_t s = r >> 5, lane = r & 31;
-    const uint64_t o0 = off[s], width = (off[s + 1] - o0) >> 5;
-    uint64_t j = 0;
-    if (r < rows) {
-      const uint32_t id = row_id[r];
-      uint32_t v, k0, n;
-      if (id < V) {
-        v = id;
-        k0 = 0;
-        n = seg_len(g.in, v);
-      } else {
-        v = piece_v[id - V];
-        k0 = piece_start[id - V];
-        n = piece_len[id - V];
-      }
-      const uint64_t so = g.in.off[v] + k0;
-      for (uint32_t k = 0; k < n && j < width; k++) {
-        const typename P_::E e = pool[so + k];
-        const uint32_t u = P_::nbr(e);
-        if (u & DEAD) continue;
-        ent[o0 + j * 32 + lane] = S_::make(u, P_::wt(e));
-        j++;
+    const uint64_t o0 = off[s];
+    const uint32_t width = (uint32_t)((off[s + 1] - o0) >> 5);
+    typename S_::E *col = ent + o0 + lane;
+    const RowSrc src = sell_row_src(g, row_id, r, rows, piece_v, piece_start, piece_len);
+    uint32_t j = 0;
+    for (uint32_t k0 = 0; k0 < src.n; k0 += 8) {
+      typename P_::E e[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k0 + k < src.n) e[k] = pool[src.from + k0 + k];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k0 + k < src.n && !(P_::nbr(e[k]) & DEAD)) col[(uint64_t)j++ * 32] = S_::make(P_::nbr(e[k]), P_::wt(e[k]));
+    }
+    for (; j < width; j++) col[(uint64_t)j * 32] = S_::none();
+  }
+}
+
+// The same for weighted rows of more than 8 entries, each row's live entries
+// by weight class, lightest first, so that a pull can stop inside the row.
+// One CTA per slice and one warp per row: a lane keeps its K entries in
+// registers (one round trip to the pool), the row's class counts and the
+// sorted slice are in shared memory, and the slice leaves it column-major in
+// coalesced stores.  A row of the tile is padded to an odd number of entries,
+// so that a column of 32 rows touches every bank pair once.
+constexpr int SF_TPB = 1024;
+constexpr size_t sell_fill_smem(int K) { return 32 * (32 * (size_t)K + 1) * 8 + 32 * W_CLASSES * 2; }
+
+template <int K>
+__global__ void __launch_bounds__(SF_TPB) k_sell_fill_sorted(DevGraph g, const uint32_t *row_id, uint64_t rows,
+                                                             uint64_t s_lo, uint64_t s_hi, const uint64_t *off,
+                                                             const uint32_t *piece_v, const uint32_t *piece_start,
+                                                             const uint32_t *piece_len, uint2 *ent) {
+  extern __shared__ uint2 s_tile[];  // [32 rows][32 K + 1], then [32 rows][W_CLASSES] u16 in pairs
+  constexpr int RS = 32 * K + 1;
+  const int lane = lane_id(), row = threadIdx.x >> 5;
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(s_tile + 32 * RS) + row * (W_CLASSES / 2);  // two classes per word
+  constexpr int CW = W_CLASSES / 64;  // words of classes per lane
+  const uint2 *pool = reinterpret_cast<const uint2 *>(g.in.pool);
+  for (uint64_t s = s_lo + blockIdx.x; s < s_hi; s += gridDim.x) {
+    const uint64_t o0 = off[s];
+    const uint32_t width = (uint32_t)((off[s + 1] - o0) >> 5);
+    const RowSrc src = sell_row_src(g, row_id, s * 32 + row, rows, piece_v, piece_start, piece_len);
+    uint2 e[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t i = 32 * k + lane;
+      e[k] = i < src.n ? pool[src.from + i] : make_uint2(NONE, 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < CW; k++) cnt[32 * k + lane] = 0;
+    __syncwarp();
+    uint32_t at[K];  // rank within the class
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      at[k] = 0;
+      if (!(e[k].x & DEAD)) {  // (NONE has the bit too)
+        const uint32_t c = w_class(e[k].y);
+        at[k] = (atomicAdd(&cnt[c >> 1], 1u << (16 * (c & 1))) >> (16 * (c & 1))) & 0xFFFFu;
       }
     }
-    for (; j < width; j++) ent[o0 + j * 32 + lane] = S_::none();
+    __syncwarp();
+    // exclusive prefix over the classes, each lane the words CW l .. CW l + CW - 1
+    uint32_t c2[CW], sum = 0;
+#pragma unroll
+    for (int k = 0; k < CW; k++) {
+      c2[k] = cnt[CW * lane + k];
+      sum += (c2[k] & 0xFFFFu) + (c2[k] >> 16);
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const uint32_t live = __shfl_sync(FULL, incl, 31);
+    uint32_t run = incl - sum;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < CW; k++) {
+      const uint32_t a = run, b = run + (c2[k] & 0xFFFFu);
+      cnt[CW * lane + k] = a | (b << 16);
+      run = b + (c2[k] >> 16);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      if (!(e[k].x & DEAD)) {
+        const uint32_t c = w_class(e[k].y);
+        s_tile[row * RS + ((cnt[c >> 1] >> (16 * (c & 1))) & 0xFFFFu) + at[k]] = e[k];
+      }
+    }
+    for (uint32_t j = live + lane; j < width; j += 32) s_tile[row * RS + j] = make_uint2(NONE, 0u);
+    __syncthreads();
+    for (uint32_t j = row; j < width; j += 32) ent[o0 + (uint64_t)j * 32 + lane] = s_tile[lane * RS + j];
+    __syncthreads();
   }
 }
 
-// Writes v's pulled best when it improves v's value (single writer per vertex).
+// Values in 32 bits (every hook's fit): update_func's value and its order.
 template <int A>
-__device__ __forceinline__ bool pull_commit(const DevGraph &g, bool has, uint32_t v, uint64_t best, uint32_t bsrc,
-                                            uint32_t bw) {
-  if (!has || !Hook<A>::better(best, ld_v32(g.val32, v))) return false;
-  g.lab[v] = make_ulonglong2(best, pack_parent(bsrc, bw));
-  g.val32[v] = (uint32_t)best;
-  return true;
+__device__ __forceinline__ uint32_t combine32(uint32_t s, uint32_t w) {
+  return (uint32_t)Hook<A>::combine(s, w);
+}
+template <int A>
+__device__ __forceinline__ bool better32(uint32_t a, uint32_t b) {
+  return A == RG_SSWP ? a > b : a < b;
 }
 
-// Commit of one pulled row (all lanes of the warp call it).
+// What a pull may leave out.  No vertex in the level's frontier has a value
+// better than the level's bound m (the best value that the level before
+// committed, or the best possible one), and neither has any vertex that changes
+// in this level; a source that is in neither set was relaxed over all its edges
+// after its last change.  So an in-edge of weight w can only improve v if
+// combine(m, w) does, and since rows are in order of weight (lightest first;
+// SSWP reads them from the other end), the first weight class that cannot
+// improve v ends its row.  With weights of 1 to 255 that leaves a few entries
+// of each list: a hub of value 5 reads the entries lighter than 5.  The values
+// after the level are those of the full pull.
+// (RMAT-22 SSSP, four pull levels: 0.17, 0.13, 0.11 and 0.09 ms and 0.7 E
+// entries read in all; over every entry 0.31 to 0.34 ms each and 4.0 E.)
 template <int A>
-__device__ __forceinline__ void pull_row_done(const DevGraph &g, bool active, uint32_t id, bool has, uint64_t best,
-                                              uint32_t bsrc, uint32_t bw, ulonglong2 *piece_best, uint32_t *fout,
-                                              unsigned long long *fout_n, uint32_t mst, unsigned long long &local) {
-  bool upd = false;
-  if (active && id < g.V) {
-    upd = pull_commit<A>(g, has, id, best, bsrc, bw);
-  } else if (active) {
-    // a hub piece: its best waits for k_pull_hub_fix
-    piece_best[id - g.V] = make_ulonglong2(best, has ? pack_parent(bsrc, bw) : ~0ull);
+__device__ __forceinline__ bool pull_open(uint32_t m, uint32_t w, uint32_t best) {
+  return better32<A>(combine32<A>(m, w), best);
+}
+// the remaining entries of a row after one of weight w
+template <int A>
+__device__ __forceinline__ bool pull_more(uint32_t m, uint32_t w, uint32_t best) {
+  return pull_open<A>(m, A == RG_SSWP ? w_ceil(w) : w_floor(w), best);
+}
+
+// One row's pull: the value it improves (its vertex's, or for a piece its
+// hub's), the best candidate so far and where that came from.
+struct PullRow {
+  uint32_t best, bsrc, bw;
+  bool has;
+};
+
+template <int A, bool W>
+__device__ __forceinline__ void pull_take(const typename SellE<W>::E &e, uint32_t sv, bool on, PullRow &p) {
+  using S_ = SellE<W>;
+  const uint32_t c = combine32<A>(sv, S_::wt(e));
+  if (on && better32<A>(c, p.best)) {
+    p.has = true;
+    p.best = c;
+    p.bsrc = S_::nbr(e);
+    p.bw = S_::wt(e);
+  }
+}
+
+// A warp's new frontier entries, collected in shared memory and written to the
+// queue PQ_CAP at a time: one atomic on the queue's counter and one round trip
+// for a buffer instead of for every slice.
+constexpr uint32_t PQ_CAP = 128;
+struct PullQueue {
+  uint32_t *buf;  // this warp's PQ_CAP entries
+  uint32_t n;     // entries held (the same in every lane)
+};
+
+__device__ __forceinline__ void pull_flush(PullQueue &q, uint32_t *fout, unsigned long long *fout_n) {
+  const uint32_t lane = (uint32_t)lane_id();
+  unsigned long long base = 0;
+  if (lane == 0 && q.n) base = atomicAdd(fout_n, (unsigned long long)q.n);
+  base = __shfl_sync(FULL, base, 0);
+  __syncwarp();
+  for (uint32_t i = lane; i < q.n; i += 32) fout[base + i] = q.buf[i];
+  __syncwarp();
+  q.n = 0;
+}
+
+// Commit of one pulled row (all lanes of the warp call it): a vertex has a
+// single writer, so its label needs no atomic; a piece leaves its best for
+// k_pull_hub_fix.  fb: the best value committed by this thread.
+template <int A>
+__device__ __forceinline__ void pull_row_done(const DevGraph &g, bool active, uint32_t id, const PullRow &p,
+                                              ulonglong2 *piece_best, PullQueue &q, uint32_t *fout,
+                                              unsigned long long *fout_n, uint32_t mst, uint32_t &local, uint32_t &fb) {
+  const bool upd = active && id < g.V && p.has;
+  if (upd) {
+    g.lab[id] = make_ulonglong2(p.best, pack_parent(p.bsrc, p.bw));
+    g.val32[id] = p.best;
+    if (better32<A>(p.best, fb)) fb = p.best;
+  } else if (active && id >= g.V) {
+    piece_best[id - g.V] = make_ulonglong2(p.best, p.has ? pack_parent(p.bsrc, p.bw) : ~0ull);
   }
   local += upd;
-  warp_append(upd, id, fout, fout_n, FULL);
+  const unsigned b = __ballot_sync(FULL, upd);
+  if (b) {
+    if (upd) q.buf[q.n + __popc(b & ((1u << lane_id()) - 1))] = id;
+    q.n += __popc(b);
+    if (q.n > PQ_CAP - 32) pull_flush(q, fout, fout_n);
+  }
   if (mst) mark_modified(g, upd, id, mst);
 }
 
-template <int A, bool W>
-__device__ __forceinline__ void pull_take(const typename SellE<W>::E &e, uint32_t sv, bool &has, uint64_t &best,
-                                          uint32_t &bsrc, uint32_t &bw) {
-  using S_ = SellE<W>;
-  if (S_::nbr(e) == NONE) return;
-  const uint64_t c = Hook<A>::combine(sv, S_::wt(e));
-  if (!has || Hook<A>::better(c, best)) {
-    has = true;
-    best = c;
-    bsrc = S_::nbr(e);
-    bw = S_::wt(e);
+// The best value committed by the warp, into the bound of the next frontier.
+template <int A>
+__device__ __forceinline__ void pull_bound_out(uint32_t fb, unsigned long long *bout) {
+  const uint32_t b = A == RG_SSWP ? __reduce_max_sync(FULL, fb) : __reduce_min_sync(FULL, fb);
+  if (lane_id() == 0 && better32<A>(b, (uint32_t)__ldcg(bout))) {
+    if (A == RG_SSWP) atomicMax(bout, (unsigned long long)b);
+    else atomicMin(bout, (unsigned long long)b);
   }
+}
+template <int A>
+__device__ __forceinline__ uint32_t pull_worst() {
+  return A == RG_SSWP ? 0u : 0xFFFFFFFFu;
 }
 
 // Source values through L1: the values of popular sources stay there.  A value
 // cached before its owner improved in this level is only older, and that owner
 // is in the next frontier anyway.
-__device__ __forceinline__ uint32_t pull_src_val(const DevGraph &g, uint32_t u) {
-  return u != NONE ? __ldca(&g.val32[u]) : 0u;
-}
+__device__ __forceinline__ uint32_t pull_src_val(const DevGraph &g, uint32_t u) { return __ldca(&g.val32[u]); }
 
-// Slices are sorted by width (the length of their longest row).  Wide slices
-// (more than 8 entries per row) take a warp each and stream their rows 16 (or
-// 8 + 8 prefetched) entries at a time; narrower slices are taken G at a time
-// (G = 2, 4, 8 for widths up to 8, 4, 2) so that every lane still keeps 16
-// entries in flight per round trip.  cls[0..2]: first slice of width <= 8, 4, 2.
-struct PullClasses {
-  uint64_t c8, c4, c2;
-};
-
+// Slices are sorted by width (the length of their longest row).  A warp takes
+// one slice and reads its rows PULL_DEPTH entries at a time; slices at most 4,
+// 2 and 1 entries wide are taken G = 2, 4 and 8 at a time, so that every lane
+// still keeps eight entries in flight per round trip.  (Sixteen took 112
+// registers a thread and left a quarter of the warps resident.)
 template <int A, bool W, int G>
 __device__ __forceinline__ void pull_narrow(const DevGraph &g, const typename SellE<W>::E *ent, const uint64_t *off,
-                                            const uint32_t *row_id, uint64_t rows, uint64_t lo, uint64_t hi,
-                                            ulonglong2 *piece_best, uint32_t *fout, unsigned long long *fout_n,
-                                            uint32_t mst, unsigned long long &local, uint64_t warp, uint64_t nwarps) {
+                                            const uint32_t *row_id, uint32_t rows, uint32_t lo, uint32_t hi, uint32_t m,
+                                            PullQueue &q, uint32_t *fout, unsigned long long *fout_n, uint32_t mst,
+                                            uint32_t &local, uint32_t &fb, uint32_t warp, uint32_t nwarps) {
   using S_ = SellE<W>;
-  constexpr int NP = 16 / G;
+  constexpr int NP = PULL_DEPTH / G;
   const int lane = lane_id();
-  for (uint64_t s0 = lo + warp * G; s0 < hi; s0 += nwarps * G) {
-    typename S_::E e[16];
+  for (uint32_t s0 = lo + warp * G; s0 < hi; s0 += nwarps * G) {
+    typename S_::E e[PULL_DEPTH];
+    uint32_t id[G];
 #pragma unroll
     for (int gi = 0; gi < G; gi++) {
-      const uint64_t s = s0 + gi;
-      const uint64_t o = s < hi ? off[s] : 0, w = s < hi ? (off[s + 1] - o) >> 5 : 0;
+      const uint32_t s = s0 + gi;
+      const uint64_t o = s < hi ? off[s] : 0;
+      const uint32_t w = s < hi ? (uint32_t)((off[s + 1] - o) >> 5) : 0u;
+      id[gi] = s < hi && s * 32 + lane < rows ? row_id[s * 32 + lane] : NONE;
 #pragma unroll
       for (int k = 0; k < NP; k++) e[gi * NP + k] = k < w ? __ldcs(&ent[o + (uint64_t)k * 32 + lane]) : S_::none();
     }
-    uint32_t sv[16];
+    uint32_t cur[G];
 #pragma unroll
-    for (int k = 0; k < 16; k++) sv[k] = pull_src_val(g, S_::nbr(e[k]));
+    for (int gi = 0; gi < G; gi++) cur[gi] = id[gi] != NONE ? __ldcg(&g.val32[id[gi]]) : 0u;
+    uint32_t sv[PULL_DEPTH];
+    bool on[PULL_DEPTH];
+#pragma unroll
+    for (int k = 0; k < PULL_DEPTH; k++) {
+      on[k] = S_::nbr(e[k]) != NONE && pull_open<A>(m, S_::wt(e[k]), cur[k / NP]);
+      sv[k] = on[k] ? pull_src_val(g, S_::nbr(e[k])) : 0u;
+    }
 #pragma unroll
     for (int gi = 0; gi < G; gi++) {
-      const uint64_t s = s0 + gi;
-      const uint64_t r = s * 32 + lane;
-      const bool active = s < hi && r < rows;
-      bool has = false;
-      uint64_t best = 0;
-      uint32_t bsrc = 0, bw = 0;
+      PullRow p = {cur[gi], 0u, 0u, false};
 #pragma unroll
-      for (int k = 0; k < NP; k++) pull_take<A, W>(e[gi * NP + k], sv[gi * NP + k], has, best, bsrc, bw);
-      pull_row_done<A>(g, active, active ? row_id[r] : 0u, has, best, bsrc, bw, piece_best, fout, fout_n, mst, local);
+      for (int k = 0; k < NP; k++) pull_take<A, W>(e[gi * NP + k], sv[gi * NP + k], on[gi * NP + k], p);
+      // (a row this narrow is a vertex)
+      pull_row_done<A>(g, id[gi] != NONE, id[gi], p, nullptr, q, fout, fout_n, mst, local, fb);
     }
   }
 }
 
-// One launch covers the wide slices [s_lo, s_hi), and the narrow classes
-// when `rest` is set.
+// What one launch of a pull level covers: the slices of the hubs and their
+// pieces (PART_HUBS), every slice after them (PART_REST), all slices
+// (PART_ALL), none (PART_NONE), or the wide slices [s_lo, s_hi), and with
+// `rest` the narrow ones too (PART_RANGE, grouped pull levels).  The bounds of
+// the named parts come from the plan in device memory, so that the cached loop
+// graph outlives the copy it was captured for.
+enum PullPart : int { PART_HUBS, PART_REST, PART_ALL, PART_NONE, PART_RANGE };
+
 template <int A, bool W>
-__global__ void __launch_bounds__(PS_TPB) k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off,
-                                                      const uint32_t *row_id, uint64_t rows, uint64_t slices,
-                                                      PullClasses cls, uint64_t s_lo, uint64_t s_hi, int rest,
-                                                      ulonglong2 *piece_best, uint32_t *fout,
-                                                      unsigned long long *fout_n, uint32_t mst) {
-  if (g.ctl[C_MODE] != M_PULL) return;
+__global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
+    k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off, const uint32_t *row_id,
+                const uint32_t *piece_v, const SellPlan *plan, int part, uint32_t s_lo, uint32_t s_hi, int rest,
+                const unsigned long long *bin, unsigned long long *bout, ulonglong2 *piece_best, uint32_t *fout,
+                unsigned long long *fout_n, uint32_t mst) {
+  if (g.ctl[C_MODE] != M_PULL || part == PART_NONE) return;
   using S_ = SellE<W>;
+  constexpr bool rev = A == RG_SSWP;  // heaviest entries first
+  constexpr bool by_w = W && (A == RG_SSSP || A == RG_SSWP);
+  constexpr int N = PULL_DEPTH;
+  __shared__ uint32_t s_q[PS_TPB / 32][PQ_CAP];
+  const uint32_t rows = (uint32_t)plan->rows, c4 = plan->slice[4];
+  if (part != PART_RANGE) {
+    const uint32_t mid = plan->slice[PULL_SPLIT - 1];
+    s_lo = part == PART_REST ? mid : 0;
+    s_hi = part == PART_HUBS ? mid : c4;
+    rest = part != PART_HUBS;
+  }
   const int lane = lane_id();
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long local = 0;
-  for (uint64_t s = s_lo + warp; s < s_hi; s += nwarps) {
-    const uint64_t r = s * 32 + lane;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t m = (uint32_t)*bin;
+  PullQueue q = {s_q[threadIdx.x >> 5], 0u};
+  uint32_t fb = pull_worst<A>();
+  uint32_t local = 0, chunks = 0;
+  for (uint32_t s = s_lo + warp; s < s_hi; s += nwarps) {
+    const uint32_t r = s * 32 + lane;
     const bool active = r < rows;
     const uint32_t id = active ? row_id[r] : 0u;
-    const uint64_t o0 = off[s], width = (off[s + 1] - o0) >> 5;
+    const uint64_t o0 = off[s];
+    const uint32_t width = (uint32_t)((off[s + 1] - o0) >> 5);
     const typename S_::E *col = ent + o0 + lane;
-    bool has = false;
-    uint64_t best = 0;
-    uint32_t bsrc = 0, bw = 0;
-    constexpr int N = PullDepth<W>::N;
-    typename S_::E ne[N];
-    if constexpr (PullDepth<W>::prefetch) {
+    typename S_::E e[N];
 #pragma unroll
-      for (int k = 0; k < N; k++) ne[k] = k < width ? __ldcs(&col[(uint64_t)k * 32]) : S_::none();
-    }
-    for (uint64_t j = 0; j < width; j += N) {
-      typename S_::E e[N];
+    for (int k = 0; k < N; k++)  // (the first entries travel with the row's value)
+      e[k] = active && k < width ? __ldcs(&col[(rev ? width - 1 - k : k) * 32]) : S_::none();
+    PullRow p = {0u, 0u, 0u, false};
+    if (active) p.best = __ldcg(&g.val32[id < g.V ? id : piece_v[id - g.V]]);
+    bool live = active && pull_open<A>(m, A == RG_SSWP ? 0xFFFFFFFFu : 0u, p.best);
+    for (uint32_t j = N;; j += N) {
+      uint32_t sv[N];
+      bool on[N];
 #pragma unroll
       for (int k = 0; k < N; k++) {
-        if constexpr (PullDepth<W>::prefetch) {
-          e[k] = ne[k];
-          ne[k] = j + N + k < width ? __ldcs(&col[(j + N + k) * 32]) : S_::none();
-        } else {
-          e[k] = j + k < width ? __ldcs(&col[(j + k) * 32]) : S_::none();
-        }
+        on[k] = live && S_::nbr(e[k]) != NONE && pull_open<A>(m, S_::wt(e[k]), p.best);
+        sv[k] = on[k] ? pull_src_val(g, S_::nbr(e[k])) : 0u;
       }
-      uint32_t sv[N];  // every hook's values fit 32 bits
 #pragma unroll
-      for (int k = 0; k < N; k++) sv[k] = pull_src_val(g, S_::nbr(e[k]));
+      for (int k = 0; k < N; k++) pull_take<A, W>(e[k], sv[k], on[k], p);
+      chunks += live;
+      if (j >= width) break;
+      if constexpr (by_w) {
+        // padding ends a row read forwards and comes first in one read backwards
+        if (S_::nbr(e[N - 1]) == NONE) live = live && rev;
+        else live = live && pull_more<A>(m, S_::wt(e[N - 1]), p.best);
+      } else {
+        live = live && pull_open<A>(m, 0u, p.best);
+      }
+      if (!__any_sync(FULL, live)) break;
 #pragma unroll
-      for (int k = 0; k < N; k++) pull_take<A, W>(e[k], sv[k], has, best, bsrc, bw);
+      for (int k = 0; k < N; k++)
+        e[k] = live && j + k < width ? __ldcs(&col[(rev ? width - 1 - (j + k) : j + k) * 32]) : S_::none();
     }
-    pull_row_done<A>(g, active, id, has, best, bsrc, bw, piece_best, fout, fout_n, mst, local);
+    pull_row_done<A>(g, active, id, p, piece_best, q, fout, fout_n, mst, local, fb);
   }
-  if (!rest) {
-    warp_add_result(local, &g.ctl[C_RESULT]);
-    return;
+  unsigned long long scanned = (unsigned long long)chunks * N;
+  if (rest) {
+    const uint32_t c2 = plan->slice[2], c1 = plan->slice[1], slices = (uint32_t)plan->slices;
+    pull_narrow<A, W, 2>(g, ent, off, row_id, rows, c4, c2, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
+    pull_narrow<A, W, 4>(g, ent, off, row_id, rows, c2, c1, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
+    pull_narrow<A, W, 8>(g, ent, off, row_id, rows, c1, slices, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
+    if (blockIdx.x == 0 && threadIdx.x == 0) scanned += off[slices] - off[c4];
   }
-  pull_narrow<A, W, 2>(g, ent, off, row_id, rows, cls.c8, cls.c4, piece_best, fout, fout_n, mst, local, warp, nwarps);
-  pull_narrow<A, W, 4>(g, ent, off, row_id, rows, cls.c4, cls.c2, piece_best, fout, fout_n, mst, local, warp, nwarps);
-  pull_narrow<A, W, 8>(g, ent, off, row_id, rows, cls.c2, slices, piece_best, fout, fout_n, mst, local, warp, nwarps);
+  pull_flush(q, fout, fout_n);
+  pull_bound_out<A>(fb, bout);
   warp_add_result(local, &g.ctl[C_RESULT]);
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g.ctl[C_EDGES], off[slices]);
-}
-
-// First slice whose width is at most 8, 4, 2 (slice widths never increase).
-__global__ void k_sell_classes(const uint32_t *sorted_key, uint64_t slices, unsigned long long *cls) {
-  // cls[3]: first slice narrower than PULL_SPLIT
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < slices; s += stride) {
-    const uint32_t w = sorted_key[s * 32], wp = s ? sorted_key[(s - 1) * 32] : 0xFFFFFFFFu;
-    if (w <= 8 && wp > 8) cls[0] = s;
-    if (w <= 4 && wp > 4) cls[1] = s;
-    if (w <= 2 && wp > 2) cls[2] = s;
-    if (w < PULL_SPLIT && wp >= PULL_SPLIT) cls[3] = s;
-  }
+  warp_add_result(scanned, &g.ctl[C_EDGES]);
 }
 
 // One warp per hub: best of its pieces, one write.
 template <int A>
-__global__ void k_pull_hub_fix(DevGraph g, const uint32_t *hub_v, const uint64_t *piece_off, uint64_t nh,
-                               const ulonglong2 *piece_best, uint32_t *fout, unsigned long long *fout_n, uint32_t mst) {
+__global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
+                                                      const SellPlan *plan, const ulonglong2 *piece_best,
+                                                      unsigned long long *bout, uint32_t *fout,
+                                                      unsigned long long *fout_n, uint32_t mst) {
   if (g.ctl[C_MODE] != M_PULL) return;
   const int lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long local = 0;
-  for (uint64_t h0 = warp * 32; h0 < nh; h0 += nwarps * 32) {
-    // lane l owns hub h0 + l; the warp scans the pieces of its 32 hubs
-    const uint64_t h = h0 + lane;
-    bool has = false;
-    uint64_t best = 0, meta = 0;
-    uint32_t v = 0;
-    if (h < nh) {
-      v = hub_v[h];
-      for (uint64_t p = piece_off[h]; p < piece_off[h + 1]; p++) {
-        const ulonglong2 b = piece_best[p];
-        if (b.y == ~0ull) continue;
-        if (!has || Hook<A>::better(b.x, best)) {
-          has = true;
-          best = b.x;
-          meta = b.y;
-        }
+  const uint64_t nh = plan->hubs;
+  uint32_t local = 0;
+  uint32_t fb = pull_worst<A>();
+  for (uint64_t h = warp; h < nh; h += nwarps) {
+    const uint32_t v = hub_v[h];
+    const uint64_t pc = hub_pc[h];
+    const uint32_t p0 = (uint32_t)pc, np = (uint32_t)(pc >> 32);
+    uint32_t best = pull_worst<A>();
+    uint64_t meta = ~0ull;
+    for (uint32_t k = lane; k < np; k += 32) {
+      const ulonglong2 b = piece_best[p0 + k];
+      if (b.y != ~0ull && (meta == ~0ull || better32<A>((uint32_t)b.x, best))) {
+        best = (uint32_t)b.x;
+        meta = b.y;
       }
     }
-    const bool upd = h < nh && pull_commit<A>(g, has, v, best, (uint32_t)meta, (uint32_t)(meta >> 32));
+    const uint32_t top = A == RG_SSWP ? __reduce_max_sync(FULL, best) : __reduce_min_sync(FULL, best);
+    const unsigned won = __ballot_sync(FULL, meta != ~0ull && best == top);
+    const bool upd = won && lane == __ffs(won) - 1;
+    if (upd) {
+      g.lab[v] = make_ulonglong2(best, meta);
+      g.val32[v] = best;
+      if (better32<A>(best, fb)) fb = best;
+    }
     local += upd;
     warp_append(upd, v, fout, fout_n, FULL);
     if (mst) mark_modified(g, upd, v, mst);
   }
+  pull_bound_out<A>(fb, bout);
   warp_add_result(local, &g.ctl[C_RESULT]);
 }
 
@@ -1330,6 +1592,7 @@ struct LevelCfg {
   uint64_t cl_v;         // frontier vertices a cluster stages (its CTAs x CL_TPB)
   int allow_pull;
   int bottom_up;
+  uint32_t bnd_best, bnd_worst;  // the best and the worst value of the hook's order
 };
 
 // Picks the level mode from the frontier size (the reference's push/pull rule
@@ -1390,6 +1653,10 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   else if (n >= cfg.lbs_min) mode = M_LBS;
   if (mode == M_DENSE_PUSH) c[C_ACT] += 1;
   c[C_MODE] = mode;
+  // bounds on the frontiers' values: pull levels collect theirs, others give none
+  const int half = fin_n == &c[C_QN0] ? 0 : 1;
+  if (lvl == 0) c[C_BND0 + half] = cfg.bnd_best;
+  c[C_BND0 + (half ^ 1)] = mode == M_PULL ? cfg.bnd_worst : cfg.bnd_best;
   if (use_switch) c[C_KLAUNCH] += 1 + mode_launches(mode) + (mode == M_PULL ? cfg.pull_groups - 2 : 0);
   if (n) {
     if (lvl < TRACE_CAP) {
@@ -2427,13 +2694,27 @@ int guard_counters(Graph &g) {
   return RG_OK;
 }
 
+template <int K>
+int sell_fill_sorted(Graph &g, uint64_t s_lo, uint64_t s_hi, const uint32_t *pv, const uint32_t *pst,
+                     const uint32_t *pln) {
+  if (s_lo >= s_hi) return RG_OK;
+  const size_t smem = sell_fill_smem(K);
+  RG_CUDA(cudaFuncSetAttribute(k_sell_fill_sorted<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  count_launch(g);
+  const uint64_t blocks = std::min<uint64_t>(s_hi - s_lo, (uint64_t)g.num_sms * 8);
+  k_sell_fill_sorted<K><<<(unsigned)blocks, SF_TPB, smem, g.stream>>>(g.d, g.sell_row, g.sell_plan_host->rows, s_lo, s_hi,
+                                                                      g.sell_off, pv, pst, pln,
+                                                                      reinterpret_cast<uint2 *>(g.sell_ent));
+  RG_CUDA(cudaGetLastError());
+  return RG_OK;
+}
+
 // Sliced-ELL copy of the in-edges for dense pull levels, rebuilt only after
-// the adjacency changed (one degree sort and one copy per version).
+// the adjacency changed (three passes over the list lengths, one host
+// synchronisation for the sizes, one copy of the entries per version).
 template <bool W>
 int prepare_pull_w(Graph &g) {
   const uint64_t V = g.V;
-  unsigned long long *cnt = g.sell_cnt;
-  unsigned long long h[2] = {0, 0};
   auto grow = [&](void **p, uint64_t &cap, uint64_t want, size_t esz) -> int {
     if (want <= cap && *p) return RG_OK;
     if (*p) {
@@ -2442,6 +2723,7 @@ int prepare_pull_w(Graph &g) {
     }
     *p = nullptr;
     cap = 0;
+    g.sell_epoch++;  // cached loop graphs hold the old address
     const uint64_t c = want + want / 8 + 64;
     if (cudaMalloc(p, c * esz) != cudaSuccess) {
       cudaGetLastError();
@@ -2453,105 +2735,53 @@ int prepare_pull_w(Graph &g) {
     return RG_OK;
   };
   int rc = RG_OK;
-  // 1. hubs and their piece offsets (the hub arrays are sized for every vertex
-  //    once, so their addresses stay fixed for the cached level-loop graph)
+  // the hub arrays are sized for every vertex once, so their addresses stay
+  // fixed for the cached level-loop graph
   if ((rc = grow((void **)&g.sell_hub, g.sell_hub_cap, V + 1, 4))) return rc;
-  uint64_t off_cap = g.sell_hub_cap;
   if (!g.sell_hub_off) {
-    if (cudaMalloc(&g.sell_hub_off, off_cap * 8) != cudaSuccess) {
+    if (cudaMalloc(&g.sell_hub_off, g.sell_hub_cap * 8) != cudaSuccess) {
       cudaGetLastError();
       set_error("device allocation failed: pull preparation");
       return RG_ENOMEM_HBM;
     }
-    g.bytes += off_cap * 8;
+    g.bytes += g.sell_hub_cap * 8;
   }
-  RG_CUDA(cudaMemsetAsync(cnt, 0, 16, g.stream));
-  count_launch(g);
-  k_sell_hubs<<<g.num_sms * 8, TPB, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, cnt);
-  RG_CUDA(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, g.stream));
+  RG_CUDA(cudaMemsetAsync(g.sell_plan, 0, sizeof(SellPlan), g.stream));
+  count_launch(g, 2);
+  k_sell_count<<<g.num_sms * 2, 1024, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan);
+  k_sell_plan<<<1, 1024, 0, g.stream>>>(g.sell_plan);
+  RG_CUDA(cudaMemcpyAsync(g.sell_plan_host, g.sell_plan, sizeof(SellPlan), cudaMemcpyDeviceToHost, g.stream));
   RG_CUDA(cudaStreamSynchronize(g.stream));
-  const uint64_t nh = h[0];
-  RG_CUDA(cudaMemsetAsync(g.sell_hub_off + nh, 0, 8, g.stream));
-  size_t tb = g.cub_tmp_bytes;
-  RG_CUDA(cub::DeviceScan::ExclusiveSum(g.cub_tmp, tb, g.sell_hub_off, g.sell_hub_off, nh + 1, g.stream));
-  uint64_t P = 0;
-  RG_CUDA(cudaMemcpyAsync(&P, g.sell_hub_off + nh, 8, cudaMemcpyDeviceToHost, g.stream));
-  RG_CUDA(cudaStreamSynchronize(g.stream));
-  const uint64_t n = V + P;
-  // 2. piece table, piece results and row ids
+  const SellPlan &plan = *g.sell_plan_host;
+  const uint64_t P = plan.pieces;
   if ((rc = grow((void **)&g.sell_piece, g.sell_piece_cap, 3 * (P + 1), 4))) return rc;
   if ((rc = grow((void **)&g.sell_piece_best, g.sell_best_cap, P + 1, 16))) return rc;
-  if ((rc = grow((void **)&g.sell_row, g.sell_row_cap, n, 4))) return rc;
+  if ((rc = grow((void **)&g.sell_row, g.sell_row_cap, V + P, 4))) return rc;
+  if ((rc = grow((void **)&g.sell_off, g.sell_off_cap, plan.slices + 1, 8))) return rc;
+  if ((rc = grow(&g.sell_ent, g.sell_cap, plan.total, W ? 8 : 4))) return rc;
   uint32_t *pv = g.sell_piece, *pst = pv + (P + 1), *pln = pst + (P + 1);
-  // 3. keys and ids of all rows (vertices, then pieces), sorted by length
-  uint32_t *key0 = nullptr;
-  void *tmp = nullptr;
-  if (cudaMalloc(&key0, n * 4 * 3 + 64) != cudaSuccess) {
-    cudaGetLastError();
-    set_error("device allocation failed: pull preparation");
-    return RG_ENOMEM_HBM;
-  }
-  uint32_t *id0 = key0 + n, *key1 = id0 + n;
-  count_launch(g, nh ? 2 : 1);
-  k_sell_keys<<<g.num_sms * 8, TPB, 0, g.stream>>>(g.d, key0, id0);
-  if (nh) k_sell_pieces<<<g.num_sms * 2, TPB, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, nh, key0, id0, pv, pst, pln);
-  cudaError_t e = cudaGetLastError();
-  tb = 0;
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, key0, key1, id0, g.sell_row, (int)n, 0, 32, g.stream);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tb + 256);
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairsDescending(tmp, tb, key0, key1, id0, g.sell_row, (int)n, 0, 32, g.stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(cnt + 1, 0, 8, g.stream);
-  if (e == cudaSuccess) {
-    count_launch(g);
-    k_sell_count<<<g.num_sms * 4, TPB, 0, g.stream>>>(key1, n, cnt + 1);
-    e = cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, g.stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
-  cudaFree(tmp);
-  const uint64_t rows = h[1], slices = (rows + 31) / 32;
-  // 4. slice offsets (rows count hub pieces too, so there can be more than |V|)
-  uint64_t total = 0;
-  if (e == cudaSuccess && (rc = grow((void **)&g.sell_off, g.sell_off_cap, slices + 1, 8))) {
-    cudaFree(key0);
-    return rc;
-  }
-  if (e == cudaSuccess) {
-    count_launch(g);
-    k_sell_sizes<<<g.num_sms * 4, TPB, 0, g.stream>>>(key1, slices, g.scratch64);
-    tb = g.cub_tmp_bytes;
-    e = cub::DeviceScan::ExclusiveSum(g.cub_tmp, tb, g.scratch64, g.sell_off, slices + 1, g.stream);
-  }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&total, g.sell_off + slices, 8, cudaMemcpyDeviceToHost, g.stream);
-  unsigned long long cls[4] = {slices, slices, slices, slices};
-  if (e == cudaSuccess) e = cudaMemcpyAsync(g.sell_cnt + 2, cls, 32, cudaMemcpyHostToDevice, g.stream);
-  if (e == cudaSuccess) {
-    count_launch(g);
-    k_sell_classes<<<g.num_sms * 4, TPB, 0, g.stream>>>(key1, slices, g.sell_cnt + 2);
-    e = cudaMemcpyAsync(cls, g.sell_cnt + 2, 32, cudaMemcpyDeviceToHost, g.stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
-  cudaFree(key0);
-  if (e != cudaSuccess) return cuda_fail(e, "pull preparation");
-  // 5. the entries
-  if ((rc = grow(&g.sell_ent, g.sell_cap, total, W ? 8 : 4))) return rc;
   count_launch(g);
-  k_sell_fill<W><<<g.num_sms * 8, TPB, 0, g.stream>>>(g.d, g.sell_row, rows, slices, g.sell_off, pv, pst, pln,
-                                                      reinterpret_cast<typename SellE<W>::E *>(g.sell_ent));
+  k_sell_rows<<<g.num_sms * 4, SR_TPB, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan, g.sell_row, pv, pst,
+                                                      pln, g.sell_off);
   RG_CUDA(cudaGetLastError());
-  g.sell_hubs = nh;
-  g.sell_rows = rows;
-  g.sell_slices = slices;
-  // classes are nested: a slice of width <= 2 is also <= 4 and <= 8
-  g.sell_cls[2] = cls[2];
-  g.sell_cls[1] = std::min<uint64_t>(cls[1], g.sell_cls[2]);
-  g.sell_cls[0] = std::min<uint64_t>(cls[0], g.sell_cls[1]);
-  g.sell_split = std::min<uint64_t>(cls[3], g.sell_cls[0]);
-  g.sell_off_host.resize(slices + 1);
-  RG_CUDA(cudaMemcpyAsync(g.sell_off_host.data(), g.sell_off, (slices + 1) * 8, cudaMemcpyDeviceToHost, g.stream));
-  RG_CUDA(cudaStreamSynchronize(g.stream));
-  g.sell_epoch++;
+  uint64_t plain_lo = 0;
+  if constexpr (W) {
+    // the rows that a pull reads in pieces, by weight; K = ceil(width / 32)
+    const uint32_t *sl = plan.slice;
+    if ((rc = sell_fill_sorted<18>(g, 0, sl[256], pv, pst, pln))) return rc;
+    if ((rc = sell_fill_sorted<8>(g, sl[256], sl[128], pv, pst, pln))) return rc;
+    if ((rc = sell_fill_sorted<4>(g, sl[128], sl[64], pv, pst, pln))) return rc;
+    if ((rc = sell_fill_sorted<2>(g, sl[64], sl[32], pv, pst, pln))) return rc;
+    if ((rc = sell_fill_sorted<1>(g, sl[32], sl[8], pv, pst, pln))) return rc;
+    plain_lo = sl[8];
+  }
+  if (plain_lo < plan.slices) {
+    count_launch(g);
+    k_sell_fill<W><<<g.num_sms * 16, TPB, 0, g.stream>>>(g.d, g.sell_row, plan.rows, plain_lo, plan.slices,
+                                                         g.sell_off, pv, pst, pln,
+                                                         reinterpret_cast<typename SellE<W>::E *>(g.sell_ent));
+    RG_CUDA(cudaGetLastError());
+  }
   g.pull_version = g.adj_version;
   return RG_OK;
 }
@@ -2570,24 +2800,41 @@ int prepare_pull(Graph &g) {
   return g.weighted ? prepare_pull_w<true>(g) : prepare_pull_w<false>(g);
 }
 
+// First entry of slice s (or the entries in all).
+uint64_t sell_offset(const Graph &g, uint64_t s) {
+  const SellPlan &p = *g.sell_plan_host;
+  if (s >= p.slices) return p.total;
+  int lo = 1, hi = (int)PULL_HUB;  // the narrowest width L with slice[L] <= s
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (p.slice[mid] <= s) hi = mid;
+    else lo = mid + 1;
+  }
+  return p.base[lo] + (s - p.slice[lo]) * 32 * lo;
+}
+
 // Slice bounds of the launches that follow the hub launch of a split pull
-// level: [mid, b1), [b1, b2), ..., [b_k, c8), the narrow classes with the last
+// level: [mid, b1), [b1, b2), ..., [b_k, c4), the narrow slices with the last
 // launch; groups - 1 launches holding about equal shares of the entries of
 // slices [mid, end).
-std::vector<uint64_t> pull_group_bounds(const Graph &g, uint64_t mid, uint64_t c8, uint64_t groups) {
+std::vector<uint64_t> pull_group_bounds(const Graph &g, uint64_t mid, uint64_t c4, uint64_t groups) {
   std::vector<uint64_t> b{mid};
   const uint64_t k = groups > 2 ? groups - 1 : 1;
-  const std::vector<uint64_t> &off = g.sell_off_host;
-  if (k > 1 && off.size() == g.sell_slices + 1 && mid <= c8 && c8 <= g.sell_slices) {
-    const uint64_t e0 = off[mid], e1 = off[g.sell_slices];
+  if (k > 1 && mid <= c4) {
+    const uint64_t e0 = sell_offset(g, mid), e1 = g.sell_plan_host->total;
     for (uint64_t i = 1; i < k; i++) {
       const uint64_t target = e0 + (e1 - e0) * i / k;
-      uint64_t s = (uint64_t)(std::lower_bound(off.begin() + mid, off.begin() + c8, target) - off.begin());
-      s = std::min(std::max(s, b.back()), c8);
-      if (s > b.back() && s < c8) b.push_back(s);
+      uint64_t lo = mid, hi = c4;  // first slice at or past the target
+      while (lo < hi) {
+        const uint64_t m = (lo + hi) / 2;
+        if (sell_offset(g, m) < target) lo = m + 1;
+        else hi = m;
+      }
+      const uint64_t s = std::min(std::max(lo, b.back()), c4);
+      if (s > b.back() && s < c4) b.push_back(s);
     }
   }
-  b.push_back(c8);
+  b.push_back(c4);
   return b;
 }
 
@@ -2609,22 +2856,26 @@ int enqueue_mode(Graph &g, cudaStream_t s, int half, unsigned long long mode) {
       break;
     case M_PULL: {
       const auto *ent = reinterpret_cast<const typename SellE<W>::E *>(g.sell_ent);
-      const PullClasses cls{g.sell_cls[0], g.sell_cls[1], g.sell_cls[2]};
       const bool split = pull_split_on(g, A);
-      const uint64_t mid = split ? g.sell_split : cls.c8;  // end of the first launch's wide slices
-      k_pull_sell<A, W><<<g.num_sms * 8, PS_TPB, 0, s>>>(g.d, ent, g.sell_off, g.sell_row, g.sell_rows, g.sell_slices,
-                                                         cls, 0, mid, split ? 0 : 1, g.sell_piece_best, fout, fout_n,
-                                                         mst);
-      k_pull_hub_fix<A><<<(unsigned)std::max<uint64_t>(1, (g.sell_hubs + 255) / 256), 256, 0, s>>>(
-          g.d, g.sell_hub, g.sell_hub_off, g.sell_hubs, g.sell_piece_best, fout, fout_n, mst);
-      // the other rows, in widest-first groups of equal entries: each group
-      // reads the values the groups before it set in this level
-      const std::vector<uint64_t> b = pull_group_bounds(g, mid, cls.c8, split ? g.pull_groups : 2);
-      for (size_t i = 0; i + 1 < b.size(); i++)
-        k_pull_sell<A, W><<<g.num_sms * 8, PS_TPB, 0, s>>>(g.d, ent, g.sell_off, g.sell_row, g.sell_rows,
-                                                           g.sell_slices, cls, b[i], b[i + 1],
-                                                           (split && i + 2 == b.size()) ? 1 : 0, g.sell_piece_best,
-                                                           fout, fout_n, mst);
+      const unsigned long long *bin = &g.d.ctl[C_BND0 + half];
+      unsigned long long *bout = &g.d.ctl[C_BND0 + (half ^ 1)];
+      auto pull = [&](int part, uint32_t lo, uint32_t hi, int rest) {
+        k_pull_sell<A, W><<<g.num_sms * 8, PS_TPB, 0, s>>>(g.d, ent, g.sell_off, g.sell_row, g.sell_piece, g.sell_plan,
+                                                           part, lo, hi, rest, bin, bout, g.sell_piece_best, fout,
+                                                           fout_n, mst);
+      };
+      pull(split ? PART_HUBS : PART_ALL, 0, 0, 0);
+      k_pull_hub_fix<A><<<g.num_sms * 2, 256, 0, s>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan, g.sell_piece_best,
+                                                      bout, fout, fout_n, mst);
+      if (!split || g.pull_groups <= 2) {
+        pull(split ? PART_REST : PART_NONE, 0, 0, 0);
+      } else {
+        // the other rows, in widest-first groups of equal entries: each group
+        // reads the values the groups before it set in this level
+        const std::vector<uint64_t> b = pull_group_bounds(g, g.sell_plan_host->slice[PULL_SPLIT - 1],
+                                                          g.sell_plan_host->slice[4], g.pull_groups);
+        for (size_t i = 0; i + 1 < b.size(); i++) pull(PART_RANGE, (uint32_t)b[i], (uint32_t)b[i + 1], i + 2 == b.size() ? 1 : 0);
+      }
       break;
     }
     case M_DENSE_PUSH:
@@ -2700,6 +2951,8 @@ LevelCfg level_cfg(const Graph &g, int A, bool build_variant) {
   cfg.pull_groups = cfg.pull_split ? std::max<uint64_t>(2, g.pull_groups) : 2;
   cfg.cl_edges = g.cl_ctas ? std::min<uint64_t>(g.cluster_edges, CL_EDGES) : 0;
   cfg.cl_v = (uint64_t)g.cl_ctas * CL_TPB;
+  cfg.bnd_best = A == RG_SSWP ? 0xFFFFFFFFu : 0u;
+  cfg.bnd_worst = ~cfg.bnd_best;
   return cfg;
 }
 
@@ -2887,7 +3140,9 @@ template <int A, bool W>
 int loop_exec(Graph &g, bool build_variant, cudaGraphExec_t *out) {
   const LevelCfg cfg = level_cfg(g, A, build_variant);
   LoopGraph &slot = g.loops[(A * 2 + (W ? 1 : 0)) * 2 + (build_variant ? 1 : 0)];
-  const uint64_t key = cfg_key(cfg) ^ splitmix64(g.layout_version) ^ splitmix64(build_variant ? g.sell_epoch + 5 : 0);
+  // (the launches of grouped pull levels hold slice bounds of the current copy)
+  const uint64_t key = cfg_key(cfg) ^ splitmix64(g.layout_version) ^ splitmix64(build_variant ? g.sell_epoch + 5 : 0) ^
+                       splitmix64(build_variant && cfg.pull_groups > 2 ? g.pull_version + 23 : 0);
   if (slot.exec && slot.key == key) {
     *out = slot.exec;
     return RG_OK;
@@ -3219,7 +3474,8 @@ int tree_alloc(Graph &g) {
   if ((rc = alloc((void **)&g.lb_P, V * 8 + 16, "frontier degree prefix"))) return rc;
   if ((rc = alloc((void **)&g.act, V * 4 + 4, "dense-level activity"))) return rc;
   if ((rc = alloc((void **)&g.lb_sums, SC_BLOCKS * 8, "scan block sums"))) return rc;
-  if ((rc = alloc((void **)&g.sell_cnt, 64, "pull counters"))) return rc;
+  if ((rc = alloc((void **)&g.sell_plan, sizeof(SellPlan), "pull plan"))) return rc;
+  RG_CUDA(cudaHostAlloc(&g.sell_plan_host, sizeof(SellPlan), cudaHostAllocDefault));
   RG_CUDA(cudaMemset(g.act, 0, V * 4 + 4));
   if ((rc = alloc((void **)&g.lb_tile, (g.d.out.pool_cap / LB_TILE + 4) * 4, "tile partition"))) return rc;
   g.cub_tmp_bytes = 0;
