@@ -348,6 +348,9 @@ struct Graph {
   int phase_trace = 0;            // RG_OPT_PHASE_TRACE
   uint64_t inline_max = 16;       // RG_OPT_INLINE_MAX: largest fused batch passed in the launch parameters
   uint64_t cluster_edges = 65536;  // RG_OPT_CLUSTER_EDGES: out-slot limit of a cluster level (0: off)
+  int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
+  unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
+  bool ctl_on_host = false;         // the last launch writes the control block to h_ctl itself
   int cl_ctas = 0;                  // CTAs of the cluster kernel (16 where the GPU schedules it, else 8)
   unsigned long long *ptrace_buf = nullptr;  // its device buffer (allocated with the labels)
   int bfs_bottom_up = 1;
@@ -395,6 +398,17 @@ struct Graph {
 constexpr uint64_t W_RAW_MAX = 1ull << 27;
 constexpr uint64_t W_CODE_BASE = W_RAW_MAX + 1, W_CODE_END = 1ull << 31;
 constexpr uint64_t W_LIMIT = 0ull - (1ull << 27);
+
+// Words of the grid engine's barrier block, on lines of their own: arrivals,
+// generation, a third queue counter, bounds of three frontiers, two counts
+// each of the heavy vertices queued by the rescue and expand passes, and the
+// level and stamp that CTA 0's own levels reached, twice.
+enum EngWord : int {
+  EB_COUNT = 0, EB_GEN = 16, EB_QN2 = 32, EB_BND = 48, EB_HVR = 64, EB_HVE = 66, EB_LVL = 80, EB_WORDS = 96
+};
+
+// C_KLAUNCH of the host's control block until the engine has written it.
+constexpr unsigned long long CTL_PENDING = ~0ull;
 
 // Kernel launch bookkeeping (every launch site calls count_launch).
 inline void count_launch(Graph &g, int n = 1) { g.launches += (uint64_t)n; }

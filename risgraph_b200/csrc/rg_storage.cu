@@ -414,6 +414,12 @@ int storage_copy_old(Graph &g, uint64_t n) {
 const uint64_t *storage_old_host(Graph &g) { return reinterpret_cast<const uint64_t *>(g.stage_host); }
 
 int sync_ctl(Graph &g) {
+  if (g.ctl_on_host) {
+    g.ctl_on_host = false;
+    RG_CUDA(cudaStreamSynchronize(g.stream));
+    if (g.h_ctl[C_KLAUNCH] != CTL_PENDING) return RG_OK;
+    // (the engine gave up before its end: the reason is in the device's copy)
+  }
   RG_CUDA(cudaMemcpyAsync(g.h_ctl, g.d.ctl, sizeof(unsigned long long) * C_COUNT, cudaMemcpyDeviceToHost, g.stream));
   RG_CUDA(cudaStreamSynchronize(g.stream));
   return RG_OK;
@@ -427,6 +433,7 @@ int storage_error(Graph &g) {
                                 : "device error");
   cudaMemsetAsync(&g.d.ctl[C_ERR], 0, 8, g.stream);
   cudaMemsetAsync(&g.d.ctl[C_AUX], 0, 8, g.stream);
+  if (code == RG_ETIMEOUT) cudaMemsetAsync(g.eng_bar, 0, EB_WORDS * 8, g.stream);  // (left half counted)
   return code;
 }
 

@@ -1104,18 +1104,19 @@ __device__ __forceinline__ void pull_narrow(const DevGraph &g, const typename Se
 // graph outlives the copy it was captured for.
 enum PullPart : int { PART_HUBS, PART_REST, PART_ALL, PART_NONE, PART_RANGE };
 
+// (q_buf: this warp's PQ_CAP words of shared memory)
 template <int A, bool W>
-__global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
-    k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off, const uint32_t *row_id,
-                const uint32_t *piece_v, const SellPlan *plan, int part, uint32_t s_lo, uint32_t s_hi, int rest,
-                const unsigned long long *bin, unsigned long long *bout, ulonglong2 *piece_best, uint32_t *fout,
-                unsigned long long *fout_n, uint32_t mst) {
-  if (g.ctl[C_MODE] != M_PULL || part == PART_NONE) return;
+__device__ __forceinline__ void pull_part(const DevGraph &g, const typename SellE<W>::E *ent, const uint64_t *off,
+                                          const uint32_t *row_id, const uint32_t *piece_v, const SellPlan *plan,
+                                          int part, uint32_t s_lo, uint32_t s_hi, int rest, uint32_t m,
+                                          unsigned long long *bout, ulonglong2 *piece_best, uint32_t *q_buf,
+                                          uint32_t *fout, unsigned long long *fout_n, uint32_t mst,
+                                          unsigned long long &updates, unsigned long long &scanned, uint32_t warp,
+                                          uint32_t nwarps) {
   using S_ = SellE<W>;
   constexpr bool rev = A == RG_SSWP;  // heaviest entries first
   constexpr bool by_w = W && (A == RG_SSSP || A == RG_SSWP);
   constexpr int N = PULL_DEPTH;
-  __shared__ uint32_t s_q[PS_TPB / 32][PQ_CAP];
   const uint32_t rows = (uint32_t)plan->rows, c4 = plan->slice[4];
   if (part != PART_RANGE) {
     const uint32_t mid = plan->slice[PULL_SPLIT - 1];
@@ -1124,10 +1125,7 @@ __global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
     rest = part != PART_HUBS;
   }
   const int lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t m = (uint32_t)*bin;
-  PullQueue q = {s_q[threadIdx.x >> 5], 0u};
+  PullQueue q = {q_buf, 0u};
   uint32_t fb = pull_worst<A>();
   uint32_t local = 0, chunks = 0;
   for (uint32_t s = s_lo + warp; s < s_hi; s += nwarps) {
@@ -1170,7 +1168,7 @@ __global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
     }
     pull_row_done<A>(g, active, id, p, piece_best, q, fout, fout_n, mst, local, fb);
   }
-  unsigned long long scanned = (unsigned long long)chunks * N;
+  scanned += (unsigned long long)chunks * N;
   if (rest) {
     const uint32_t c2 = plan->slice[2], c1 = plan->slice[1], slices = (uint32_t)plan->slices;
     pull_narrow<A, W, 2>(g, ent, off, row_id, rows, c4, c2, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
@@ -1180,22 +1178,33 @@ __global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
   }
   pull_flush(q, fout, fout_n);
   pull_bound_out<A>(fb, bout);
+  updates += local;
+}
+
+template <int A, bool W>
+__global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
+    k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off, const uint32_t *row_id,
+                const uint32_t *piece_v, const SellPlan *plan, int part, uint32_t s_lo, uint32_t s_hi, int rest,
+                const unsigned long long *bin, unsigned long long *bout, ulonglong2 *piece_best, uint32_t *fout,
+                unsigned long long *fout_n, uint32_t mst) {
+  if (g.ctl[C_MODE] != M_PULL || part == PART_NONE) return;
+  __shared__ uint32_t s_q[PS_TPB / 32][PQ_CAP];
+  unsigned long long local = 0, scanned = 0;
+  pull_part<A, W>(g, ent, off, row_id, piece_v, plan, part, s_lo, s_hi, rest, (uint32_t)*bin, bout, piece_best,
+                  s_q[threadIdx.x >> 5], fout, fout_n, mst, local, scanned,
+                  (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
   warp_add_result(local, &g.ctl[C_RESULT]);
   warp_add_result(scanned, &g.ctl[C_EDGES]);
 }
 
 // One warp per hub: best of its pieces, one write.
 template <int A>
-__global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
-                                                      const SellPlan *plan, const ulonglong2 *piece_best,
-                                                      unsigned long long *bout, uint32_t *fout,
-                                                      unsigned long long *fout_n, uint32_t mst) {
-  if (g.ctl[C_MODE] != M_PULL) return;
+__device__ __forceinline__ void pull_hub_fix(const DevGraph &g, const uint32_t *hub_v, const uint64_t *hub_pc,
+                                             const SellPlan *plan, const ulonglong2 *piece_best,
+                                             unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n,
+                                             uint32_t mst, unsigned long long &local, uint32_t warp, uint32_t nwarps) {
   const int lane = lane_id();
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint64_t nh = plan->hubs;
-  uint32_t local = 0;
   uint32_t fb = pull_worst<A>();
   for (uint64_t h = warp; h < nh; h += nwarps) {
     const uint32_t v = hub_v[h];
@@ -1204,7 +1213,7 @@ __global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t
     uint32_t best = pull_worst<A>();
     uint64_t meta = ~0ull;
     for (uint32_t k = lane; k < np; k += 32) {
-      const ulonglong2 b = piece_best[p0 + k];
+      const ulonglong2 b = __ldcg(&piece_best[p0 + k]);
       if (b.y != ~0ull && (meta == ~0ull || better32<A>((uint32_t)b.x, best))) {
         best = (uint32_t)b.x;
         meta = b.y;
@@ -1223,6 +1232,17 @@ __global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t
     if (mst) mark_modified(g, upd, v, mst);
   }
   pull_bound_out<A>(fb, bout);
+}
+
+template <int A>
+__global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
+                                                      const SellPlan *plan, const ulonglong2 *piece_best,
+                                                      unsigned long long *bout, uint32_t *fout,
+                                                      unsigned long long *fout_n, uint32_t mst) {
+  if (g.ctl[C_MODE] != M_PULL) return;
+  unsigned long long local = 0;
+  pull_hub_fix<A>(g, hub_v, hub_pc, plan, piece_best, bout, fout, fout_n, mst, local,
+                  (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
   warp_add_result(local, &g.ctl[C_RESULT]);
 }
 
@@ -1231,37 +1251,53 @@ __global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t
 // its in-edges and takes the first in-neighbour at depth d as its parent,
 // stopping there.  Used when the frontier is large; each vertex is written
 // only by its own thread, so no atomics on labels.
+// The in-list is read four entries at a time: the search is a chain of dependent
+// loads, and most vertices find a parent in the first few entries.
 template <bool W>
-__global__ void k_bfs_bottom_up(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
-  if (g.ctl[C_MODE] != M_BOTTOM_UP) return;
-  const uint64_t d = g.ctl[C_DEPTH];
+__device__ __forceinline__ void bottom_up(const DevGraph &g, uint64_t d, uint32_t *fout, unsigned long long *fout_n,
+                                          uint64_t gtid, uint64_t gthreads, unsigned long long &local,
+                                          unsigned long long &scanned) {
   using P_ = PoolT<W>;
   const typename P_::E *pool = reinterpret_cast<const typename P_::E *>(g.in.pool);
   const uint64_t V = g.V;
-  unsigned long long local = 0, scanned = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < V; base += stride) {
-    const uint64_t v = base + threadIdx.x;
+  const int lane = lane_id();
+  for (uint64_t v0 = gtid - lane; v0 < V; v0 += gthreads) {
+    const uint64_t v = v0 + lane;
     bool found = false;
     if (v < V && ld_v32(g.val32, (uint32_t)v) == BFS_MAXL) {
       const uint32_t len = seg_len(g.in, (uint32_t)v);
       const uint64_t off = g.in.off[v];
-      for (uint32_t k = 0; k < len; k++) {
-        const typename P_::E e = __ldg(&pool[off + k]);
-        const uint32_t u = P_::nbr(e);
-        scanned++;
-        if (u & DEAD) continue;
-        if (__ldca(&g.val32[u]) == d) {  // a stale value only hides a parent found this level
-          g.lab[v] = make_ulonglong2(d + 1, pack_parent(u, P_::wt(e)));
-          g.val32[v] = (uint32_t)(d + 1);
-          found = true;
-          break;
+      for (uint32_t k = 0; k < len && !found; k += 4) {
+        typename P_::E e[4];
+        uint32_t sv[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (k + i < len) e[i] = pool[off + k + i];
+#pragma unroll
+        for (int i = 0; i < 4; i++)  // a stale value only hides a parent found this level
+          sv[i] = k + i < len && !(P_::nbr(e[i]) & DEAD) ? __ldca(&g.val32[P_::nbr(e[i])]) : NONE;
+        scanned += min(4u, len - k);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          if (!found && sv[i] == d) {
+            g.lab[v] = make_ulonglong2(d + 1, pack_parent(P_::nbr(e[i]), P_::wt(e[i])));
+            g.val32[v] = (uint32_t)(d + 1);
+            found = true;
+          }
         }
       }
     }
     local += found;
     warp_append(found, (uint32_t)v, fout, fout_n, FULL);
   }
+}
+
+template <bool W>
+__global__ void k_bfs_bottom_up(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
+  if (g.ctl[C_MODE] != M_BOTTOM_UP) return;
+  unsigned long long local = 0, scanned = 0;
+  bottom_up<W>(g, g.ctl[C_DEPTH], fout, fout_n, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+               (uint64_t)gridDim.x * blockDim.x, local, scanned);
   warp_add_result(local, &g.ctl[C_RESULT]);
   warp_add_result(scanned, &g.ctl[C_EDGES]);
 }
@@ -1352,7 +1388,7 @@ __device__ __forceinline__ void tiny_levels(const DevGraph &g, uint32_t *q_in, u
           if (s_pref[mid] <= e) lo = mid;
           else hi = mid - 1;
         }
-        const typename P_::E ent = __ldg(&pool[s_off[lo] + (e - s_pref[lo])]);
+        const typename P_::E ent = pool[s_off[lo] + (e - s_pref[lo])];
         v = P_::nbr(ent);
         scanned++;
         if (!(v & DEAD)) upd = relax_lab<A>(g, s_v[lo], s_su[lo], v, P_::wt(ent));
@@ -1541,9 +1577,8 @@ __global__ void __launch_bounds__(CL_TPB, 1)
 // host round trip happens between levels (the reference's driver decides
 // between levels on the host, core/graph.hpp:898-983, :1013-1111).
 
-// stamp: the control block's C_STAMP when the caller read it already.
-__device__ __forceinline__ void prologue_ctl(unsigned long long *c, unsigned long long inv_tag,
-                                             const unsigned long long *stamp = nullptr) {
+// (all of it but the frontier stamp)
+__device__ __forceinline__ void prologue_words(unsigned long long *c, unsigned long long inv_tag) {
   c[C_INVTAG] = inv_tag;
   c[C_INVITER] = 0;
   c[C_OVER] = 0;
@@ -1560,6 +1595,12 @@ __device__ __forceinline__ void prologue_ctl(unsigned long long *c, unsigned lon
   c[C_HVR] = 0;
   c[C_HVE] = 0;
   c[C_HVP] = 0;
+}
+
+// stamp: the control block's C_STAMP when the caller read it already.
+__device__ __forceinline__ void prologue_ctl(unsigned long long *c, unsigned long long inv_tag,
+                                             const unsigned long long *stamp = nullptr) {
+  prologue_words(c, inv_tag);
   c[C_STAMP] = (stamp ? *stamp : c[C_STAMP]) + 1;
 }
 
@@ -1723,14 +1764,19 @@ __global__ void k_copy_frontier(DevGraph g, const uint32_t *src, const unsigned 
 // build_tree init (core/graph.hpp:886-896): every label to init_label_func,
 // parent to empty; the active set is the root, or every vertex (WCC).
 template <int A>
-__global__ void k_init(DevGraph g, uint64_t root, uint32_t *fout) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.V; v += stride) {
+__device__ __forceinline__ void init_labels(const DevGraph &g, uint64_t root, uint32_t *fout, uint64_t gtid,
+                                            uint64_t stride) {
+  for (uint64_t v = gtid; v < g.V; v += stride) {
     g.lab[v] = make_ulonglong2(Hook<A>::init(v, root), pack_parent(NONE, 0));
     g.val32[v] = (uint32_t)Hook<A>::init(v, root);
     if (Hook<A>::all_active) fout[v] = (uint32_t)v;
     else if (v == root) fout[0] = (uint32_t)v;
   }
+}
+
+template <int A>
+__global__ void k_init(DevGraph g, uint64_t root, uint32_t *fout) {
+  init_labels<A>(g, root, fout, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     g.ctl[C_QN0] = Hook<A>::all_active ? g.V : 1;
     g.ctl[C_ROOT] = root;
@@ -1928,15 +1974,13 @@ __global__ void __launch_bounds__(TPB) k_rescue(DevGraph g, const uint32_t *fin,
 // Rescue of the queued heavy vertices: for each in turn, every warp scans a
 // 32-entry stride of its in-list; the first valid candidate wins the CAS.
 template <int A, bool W>
-__global__ void __launch_bounds__(TPB) k_rescue_heavy(DevGraph g, uint64_t limit) {
-  if (g.ctl[C_RECOMPUTE]) return;
+__device__ __forceinline__ void rescue_heavy_warps(const DevGraph &g, uint64_t queued, uint64_t limit, uint64_t warp,
+                                                   uint64_t nwarps) {
   const uint32_t tag_inv = (uint32_t)g.ctl[C_INVTAG];
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint64_t nh = min(g.ctl[C_HVR], (unsigned long long)g.heavy_cap);
+  const uint64_t nh = min(queued, g.heavy_cap);
   for (uint64_t h = 0; h < nh; h++) {
     const uint32_t d = g.heavy[h];
     const uint64_t sd = ld_v32(g.val32, d);
@@ -1962,6 +2006,13 @@ __global__ void __launch_bounds__(TPB) k_rescue_heavy(DevGraph g, uint64_t limit
       }
     }
   }
+}
+
+template <int A, bool W>
+__global__ void __launch_bounds__(TPB) k_rescue_heavy(DevGraph g, uint64_t limit) {
+  if (g.ctl[C_RECOMPUTE]) return;
+  rescue_heavy_warps<A, W>(g, g.ctl[C_HVR], limit, (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5,
+                           ((uint64_t)gridDim.x * blockDim.x) >> 5);
 }
 
 // Collect and expand (core/graph.hpp:1363-1417): a still-invalid vertex joins
@@ -2010,16 +2061,14 @@ __device__ __forceinline__ void expand_warps(const DevGraph &g, const uint32_t *
 // Expansion of the queued heavy vertices: their tree children, found by every
 // warp over a stride of the out-list.
 template <int A, bool W>
-__global__ void __launch_bounds__(TPB) k_expand_heavy(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
-  if (g.ctl[C_RECOMPUTE]) return;
+__device__ __forceinline__ void expand_heavy_warps(const DevGraph &g, uint64_t queued, uint32_t *fout,
+                                                   unsigned long long *fout_n, uint64_t warp, uint64_t nwarps) {
   const uint32_t tag_inv = (uint32_t)g.ctl[C_INVTAG];
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.out.pool);
   const int lane = lane_id();
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t *hv = g.heavy + g.heavy_cap;
-  const uint64_t nh = min(g.ctl[C_HVE], (unsigned long long)g.heavy_cap);
+  const uint64_t nh = min(queued, g.heavy_cap);
   for (uint64_t h = 0; h < nh; h++) {
     const uint32_t u = hv[h];
     const uint32_t len = seg_len(g.out, u);
@@ -2039,6 +2088,13 @@ __global__ void __launch_bounds__(TPB) k_expand_heavy(DevGraph g, uint32_t *fout
       warp_append(app, v, fout, fout_n, FULL);
     }
   }
+}
+
+template <int A, bool W>
+__global__ void __launch_bounds__(TPB) k_expand_heavy(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
+  if (g.ctl[C_RECOMPUTE]) return;
+  expand_heavy_warps<A, W>(g, g.ctl[C_HVE], fout, fout_n, (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5,
+                           ((uint64_t)gridDim.x * blockDim.x) >> 5);
 }
 
 template <int A, bool W>
@@ -2132,15 +2188,13 @@ __global__ void __launch_bounds__(TPB) k_pull(DevGraph g, const uint32_t *fin, c
 // The pull of the queued heavy reset vertices: every warp takes the best of a
 // stride of the in-list and relaxes the vertex with it (the CAS keeps the best).
 template <int A, bool W>
-__global__ void __launch_bounds__(TPB) k_pull_heavy(DevGraph g, uint32_t mst) {
-  if (g.ctl[C_RECOMPUTE]) return;
+__device__ __forceinline__ unsigned long long pull_heavy_warps(const DevGraph &g, uint32_t mst, uint64_t warp,
+                                                               uint64_t nwarps) {
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t *hv = g.heavy + 2 * g.heavy_cap;
-  const uint64_t nh = min(g.ctl[C_HVP], (unsigned long long)g.heavy_cap);
+  const uint64_t nh = min(__ldcg(&g.ctl[C_HVP]), (unsigned long long)g.heavy_cap);
   unsigned long long local = 0;
   for (uint64_t h = 0; h < nh; h++) {
     const uint32_t d = hv[h];
@@ -2170,6 +2224,15 @@ __global__ void __launch_bounds__(TPB) k_pull_heavy(DevGraph g, uint32_t mst) {
     local += upd;
     if (mst) mark_modified(g, __shfl_sync(FULL, upd, 0) && lane == 0, d, mst);
   }
+  return local;
+}
+
+template <int A, bool W>
+__global__ void __launch_bounds__(TPB) k_pull_heavy(DevGraph g, uint32_t mst) {
+  if (g.ctl[C_RECOMPUTE]) return;
+  const unsigned long long local =
+      pull_heavy_warps<A, W>(g, mst, (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5,
+                             ((uint64_t)gridDim.x * blockDim.x) >> 5);
   warp_add_result(local, &g.ctl[C_RESULT]);
 }
 
@@ -2512,7 +2575,10 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, sdev::OpView ops, 
   const bool left = over || (c[C_QN0] && !c[C_ERR]);
   __syncthreads();  // every thread has read the counts before the next batch resets them
   stamp(RG_PH_END);
-  if (tid == 0) c[C_OVER] = over ? 1 : 0;
+  if (tid == 0) {
+    c[C_OVER] = over ? 1 : 0;
+    c[C_QN1] = 0;  // (the engine's first output count)
+  }
   return left ? 1 : 0;
 }
 
@@ -2620,6 +2686,474 @@ __global__ void __launch_bounds__(FS_TPB)
   ctl_to_host(g, ctl_host);
 }
 
+// ---- the grid engine: levels and deletion repairs in one persistent launch ------
+// One CTA per SM, launched cooperatively, runs every level of a build or of a
+// repair, with a grid barrier where the graph-driven loop has kernel
+// boundaries, a level-begin kernel and a conditional node.  That loop spends
+// 15 to 25 us of a level on launches and conditions; a barrier is about 1.5 us.
+// Each CTA picks the level's mode from the same counters by the same rules, so
+// no decision has to be sent around:
+//   * a bottom-up or a pull level, as in the graph-driven loop;
+//   * a frontier of at most ENG_STAGE vertices is staged (offset, value, degree
+//     prefix) in every CTA's shared memory; with few out-slots CTA 0 runs
+//     successive levels alone (tiny_levels), else the slots are spread over
+//     all CTAs;
+//   * a larger frontier is prefix-summed piecewise, one contiguous piece per
+//     CTA, and after a barrier each CTA takes an equal share of the level's
+//     slots and stages the vertices that own them.
+// Queue counters rotate over three words (in, out, cleared for the next level),
+// so that clearing one needs no barrier of its own.  Served graphs keep the
+// graph-driven loop: the engine waits until every SM has room, which other
+// instances' epochs delay.
+constexpr int ENG_TPB = 1024;
+constexpr uint32_t ENG_STAGE = 1024;
+constexpr int ENG_MAX_CTAS = 256;
+constexpr uint32_t ENG_TINY = 4096;          // out-slots that CTA 0 relaxes alone
+constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
+constexpr uint32_t ENG_SPINS = 1u << 26;     // polls before a barrier gives up (tens of seconds)
+constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
+static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
+
+struct EngineArgs {
+  // sliced in-edge copy (pull levels)
+  const void *ent;
+  const uint64_t *off;
+  const uint32_t *row_id, *piece_v, *hub_v;
+  const uint64_t *hub_pc;
+  const SellPlan *plan;
+  ulonglong2 *piece_best;
+  // queues and scratch
+  uint32_t *q[2], *tree;
+  uint64_t *P;                  // frontier degree prefix, per CTA piece
+  unsigned long long *tot;      // slots of each CTA's piece
+  unsigned long long *bar;      // barrier words, third queue counter, bounds
+  unsigned long long *ctl_host;
+  uint64_t root;                // builds
+  uint64_t limit, big, max_iter;  // deletion repairs
+  LevelCfg cfg;
+  uint32_t mst;
+  int build;                    // initialise the labels first
+  int del;                      // repair deletions from the invalidated frontier in queue 0 first
+};
+
+struct GridBar {
+  unsigned long long *w;
+  unsigned gen;  // thread 0's
+};
+
+// All CTAs of the grid; false when the wait gave up (the caller returns).
+// A CTA may leave a barrier long before another one has looked at what it
+// decides on next, so a word that every CTA reads after a barrier is written
+// again only past the barrier after that: counters and flags of successive
+// levels alternate between words.
+__device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned *count = reinterpret_cast<unsigned *>(b.w + EB_COUNT), *gen = reinterpret_cast<unsigned *>(b.w + EB_GEN);
+    int ok = 1;
+    __threadfence();
+    if (atomicAdd(count, 1u) == gridDim.x - 1) {
+      atomicExch(count, 0u);
+      __threadfence();
+      atomicExch(gen, b.gen + 1);
+    } else {
+      unsigned x, spins = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(gen) : "memory");
+      } while (x == b.gen && ++spins < ENG_SPINS);
+      if (x == b.gen) {
+        atomicCAS(&g.ctl[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
+        ok = 0;
+      }
+    }
+    __threadfence();
+    b.gen++;
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+union EngShared {
+  struct {
+    uint64_t pref[ENG_STAGE + 1];  // first slot of each staged vertex, relative to the CTA's share
+    uint64_t base[ENG_STAGE];      // pool slot minus level slot
+    uint32_t u[ENG_STAGE], su[ENG_STAGE];
+    uint64_t tot[ENG_MAX_CTAS + 1];
+  } p;
+  uint32_t q[ENG_TPB / 32][PQ_CAP];
+};
+
+// Relax level slots [e0, e1) over the staged vertices (pref ascending; the
+// slots of vertex j start at pref[j]).  All threads of the CTA.
+template <int A, bool W>
+__device__ __noinline__ void eng_relax(const DevGraph &g, const EngShared &sh, uint32_t m, uint64_t e0, uint64_t e1,
+                                       uint32_t st, uint32_t *fout, unsigned long long *fout_n, uint32_t mst) {
+  unsigned long long local = 0;
+  using P_ = PoolT<W>;
+  const typename P_::E *pool = reinterpret_cast<const typename P_::E *>(g.out.pool);
+  for (uint64_t b = e0; b < e1; b += ENG_TPB * ENG_ITEMS) {
+    bool on[ENG_ITEMS];
+    uint32_t uu[ENG_ITEMS], vv[ENG_ITEMS], ww[ENG_ITEMS];
+    uint64_t su[ENG_ITEMS];
+#pragma unroll
+    for (int k = 0; k < ENG_ITEMS; k++) {
+      const uint64_t e = b + (uint64_t)k * ENG_TPB + threadIdx.x;
+      on[k] = e < e1;
+      uu[k] = vv[k] = ww[k] = 0;
+      su[k] = 0;
+      if (on[k]) {
+        uint32_t lo = 0, hi = m - 1;  // the last vertex that starts at or before e
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi + 1) >> 1;
+          if (sh.p.pref[mid] <= e) lo = mid;
+          else hi = mid - 1;
+        }
+        const typename P_::E ent = pool[sh.p.base[lo] + e];
+        uu[k] = sh.p.u[lo];
+        su[k] = sh.p.su[lo];
+        vv[k] = P_::nbr(ent);
+        ww[k] = P_::wt(ent);
+        on[k] = !(vv[k] & DEAD);
+      }
+    }
+    relax_batch<A, ENG_ITEMS>(g, on, uu, vv, ww, su, st, fout, fout_n, local, mst);
+  }
+  warp_add_result(local, &g.ctl[C_RESULT]);
+}
+
+// CTA r's share of S level slots.
+__device__ __forceinline__ void eng_share(uint64_t S, uint64_t &e0, uint64_t &e1) {
+  uint64_t per = (S + gridDim.x - 1) / gridDim.x;
+  if (per < 256) per = 256;
+  per = (per + 31) & ~31ull;
+  e0 = min(S, per * blockIdx.x);
+  e1 = min(S, e0 + per);
+}
+
+// Deletion repair over the whole grid (do_update_tree_del,
+// core/graph.hpp:1250-1511): the phases of k_rescue, k_expand, k_reset and
+// k_pull, and of their heavy-vertex passes when a vertex was queued for one.
+// Leaves the reset set in queue 0 with its count in ctl[C_QN0].
+template <int A, bool W>
+__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar) {
+  unsigned long long *c = g.ctl;
+  unsigned long long *hvr = a.bar + EB_HVR, *hve = a.bar + EB_HVE;  // two words each, by turns
+  auto cnt = [&](uint64_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
+  const uint64_t warp = (blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * ENG_TPB) >> 5;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  bool recompute = false;
+  for (uint64_t it = 0; it < a.max_iter; it++) {
+    const uint32_t *fin = a.q[it & 1];
+    uint32_t *fout = a.q[(it & 1) ^ 1];
+    const uint64_t n = __ldcg(cnt(it));
+    if (n == 0) break;
+    if (it <= 10 && __ldcg(&c[C_TREEN]) + n > a.big) {  // core/graph.hpp:1252
+      recompute = true;
+      break;
+    }
+    if (lead) {
+      *cnt(it + 2) = 0;
+      c[C_INVITER] = it + 1;
+    }
+    rescue_warps<A, W>(g, fin, n, a.limit, warp, nwarps, g.heavy, &hvr[it & 1], g.heavy_cap);
+    if (!grid_sync(g, bar)) return false;
+    const uint64_t nr = __ldcg(&hvr[it & 1]);
+    if (nr) {
+      rescue_heavy_warps<A, W>(g, nr, a.limit, warp, nwarps);
+      if (!grid_sync(g, bar)) return false;
+    }
+    if (__ldcg(&c[C_RECOMPUTE])) {  // a chain ran past the guard (nothing sets it before the next level's rescue)
+      recompute = true;
+      break;
+    }
+    if (lead) hvr[(it + 1) & 1] = hve[(it + 1) & 1] = 0;
+    expand_warps<A, W>(g, fin, n, a.tree, fout, cnt(it + 1), warp, nwarps, g.heavy + g.heavy_cap, &hve[it & 1],
+                       g.heavy_cap);
+    if (!grid_sync(g, bar)) return false;
+    const uint64_t ne = __ldcg(&hve[it & 1]);
+    if (ne) {
+      expand_heavy_warps<A, W>(g, ne, fout, cnt(it + 1), warp, nwarps);
+      if (!grid_sync(g, bar)) return false;
+    }
+  }
+  const uint64_t tn = __ldcg(&c[C_TREEN]);
+  if (!grid_sync(g, bar)) return false;  // (every CTA has read the last counts)
+  if (lead) {
+    c[C_QN0] = recompute ? 0 : tn;
+    c[C_QN1] = 0;
+    if (recompute) c[C_RECOMPUTE] = 1;
+  }
+  if (recompute) return grid_sync(g, bar);
+  // reset the invalid set; it is also the frontier of the push levels
+  reset_warps<A>(g, a.tree, tn, a.mst, warp, nwarps);
+  for (uint64_t i = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; i < tn; i += (uint64_t)gridDim.x * ENG_TPB)
+    a.q[0][i] = a.tree[i];
+  if (!grid_sync(g, bar)) return false;
+  unsigned long long local = pull_warps<A, W>(g, a.tree, tn, a.mst, warp, nwarps, g.heavy + 2 * g.heavy_cap, &c[C_HVP],
+                                              g.heavy_cap);
+  warp_add_result(local, &c[C_RESULT]);
+  if (!grid_sync(g, bar)) return false;
+  if (__ldcg(&c[C_HVP])) {
+    local = pull_heavy_warps<A, W>(g, a.mst, warp, nwarps);
+    warp_add_result(local, &c[C_RESULT]);
+    if (!grid_sync(g, bar)) return false;
+  }
+  return true;
+}
+
+// The level kinds as calls: each gets the registers of a thread for itself
+// (inlined into one function they spilled over a kilobyte per thread).
+template <int A, bool W>
+__device__ __noinline__ void eng_pull(const DevGraph &g, const EngineArgs &a, EngShared &sh, int what, uint32_t m,
+                                      unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n) {
+  unsigned long long local = 0, scanned = 0;
+  pull_part<A, W>(g, reinterpret_cast<const typename SellE<W>::E *>(a.ent), a.off, a.row_id, a.piece_v, a.plan, what, 0,
+                  0, 0, m, bout, a.piece_best, sh.q[threadIdx.x >> 5], fout, fout_n, a.mst, local, scanned,
+                  (blockIdx.x * ENG_TPB + threadIdx.x) >> 5, (gridDim.x * ENG_TPB) >> 5);
+  warp_add_result(local, &g.ctl[C_RESULT]);
+  warp_add_result(scanned, &g.ctl[C_EDGES]);
+}
+
+template <int A>
+__device__ __noinline__ void eng_hub_fix(const DevGraph &g, const EngineArgs &a, unsigned long long *bout,
+                                         uint32_t *fout, unsigned long long *fout_n) {
+  unsigned long long local = 0;
+  pull_hub_fix<A>(g, a.hub_v, a.hub_pc, a.plan, a.piece_best, bout, fout, fout_n, a.mst, local,
+                  (blockIdx.x * ENG_TPB + threadIdx.x) >> 5, (gridDim.x * ENG_TPB) >> 5);
+  warp_add_result(local, &g.ctl[C_RESULT]);
+}
+
+template <bool W>
+__device__ __noinline__ void eng_bottom_up(const DevGraph &g, uint64_t d, uint32_t *fout, unsigned long long *fout_n) {
+  unsigned long long local = 0, scanned = 0;
+  bottom_up<W>(g, d, fout, fout_n, blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB, local,
+               scanned);
+  warp_add_result(local, &g.ctl[C_RESULT]);
+  warp_add_result(scanned, &g.ctl[C_EDGES]);
+}
+
+template <int A, bool W>
+__device__ __noinline__ void eng_tiny(const DevGraph &g, const EngineArgs &a, uint32_t *q_in, unsigned long long *n_in,
+                                      uint32_t *q_out, unsigned long long *n_out, uint64_t max_levels) {
+  tiny_levels<A, W>(g, q_in, n_in, q_out, n_out, q_out, n_out, max_levels,
+                    min((uint64_t)ENG_TINY, (uint64_t)a.cfg.tiny_edges), a.mst, true);
+}
+
+using EngScan = cub::BlockScan<uint64_t, ENG_TPB>;
+
+// Stages a frontier of at most ENG_STAGE vertices and returns its out-slots.
+__device__ __noinline__ uint64_t eng_stage(const DevGraph &g, EngShared &sh, EngScan::TempStorage &tmp,
+                                           const uint32_t *fin, uint32_t n) {
+  const unsigned tid = threadIdx.x;
+  uint64_t d = 0, excl, S;
+  if (tid < n) {
+    const uint32_t u = fin[tid];
+    d = seg_len(g.out, u);
+    sh.p.u[tid] = u;
+    sh.p.base[tid] = g.out.off[u];
+    sh.p.su[tid] = (uint32_t)ld_v32(g.val32, u);
+  }
+  EngScan(tmp).ExclusiveSum(d, excl, S);
+  if (tid < n) {
+    sh.p.pref[tid] = excl;
+    sh.p.base[tid] -= excl;
+  }
+  __syncthreads();
+  return S;
+}
+
+// The degree prefix of this CTA's contiguous piece of a large frontier.
+__device__ __noinline__ void eng_prefix(const DevGraph &g, const EngineArgs &a, EngScan::TempStorage &tmp,
+                                        const uint32_t *fin, uint32_t n, uint32_t per) {
+  const uint32_t i0 = min(n, per * blockIdx.x), i1 = min(n, i0 + per);
+  uint64_t carry = 0;
+  for (uint32_t b = i0; b < i1; b += ENG_TPB) {
+    const uint32_t i = b + threadIdx.x;
+    uint64_t d = i < i1 ? seg_len(g.out, fin[i]) : 0, x, total;
+    EngScan(tmp).ExclusiveSum(d, x, total);
+    if (i < i1) a.P[i] = carry + x;
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) a.tot[blockIdx.x] = carry;
+}
+
+// Where every piece starts; returns the level's slots, and the first vertex of
+// this CTA's share [e0, e1) of them: its piece, then 32 probes at a time.
+__device__ __noinline__ uint64_t eng_first(const EngineArgs &a, EngShared &sh, EngScan::TempStorage &tmp, uint32_t n,
+                                           uint32_t per, uint64_t &e0, uint64_t &e1, uint32_t &first) {
+  __shared__ uint32_t s_first;
+  const unsigned tid = threadIdx.x, G = gridDim.x;
+  uint64_t t = tid < G ? __ldcg(&a.tot[tid]) : 0, x, S;
+  EngScan(tmp).ExclusiveSum(t, x, S);
+  if (tid < G) sh.p.tot[tid] = x;
+  __syncthreads();
+  eng_share(S, e0, e1);
+  if (tid < 32 && e0 < e1) {
+    uint32_t lo = 0, hi = G - 1;  // the last piece that starts at or before e0
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (sh.p.tot[mid] <= e0) lo = mid;
+      else hi = mid - 1;
+    }
+    const uint64_t want = e0 - sh.p.tot[lo];
+    uint32_t at = min(n, per * lo), len = min(n, at + per) - at;
+    while (len > 1) {
+      const uint32_t step = (len + 31) / 32, i = tid * step;
+      const bool le = i < len && __ldcg(&a.P[at + i]) <= want;
+      const uint32_t last = 31 - __clz(__ballot_sync(FULL, le));  // (lane 0 always passes)
+      at += last * step;
+      len = min(step, len - last * step);
+    }
+    if (tid == 0) s_first = at;
+  }
+  __syncthreads();
+  first = s_first;
+  return S;
+}
+
+// Stages up to ENG_STAGE vertices from i on; returns their number.
+__device__ __noinline__ uint32_t eng_stage_from(const DevGraph &g, const EngineArgs &a, EngShared &sh,
+                                                const uint32_t *fin, uint32_t n, uint32_t per, uint32_t i, uint64_t S) {
+  const uint32_t m = min(ENG_STAGE, n - i);
+  for (uint32_t j = threadIdx.x; j <= m; j += ENG_TPB) {
+    const uint32_t ij = i + j;
+    const uint64_t pj = ij < n ? sh.p.tot[ij / per] + __ldcg(&a.P[ij]) : S;
+    sh.p.pref[j] = pj;  // (entry m: where the next vertex starts)
+    if (j < m) {
+      const uint32_t u = fin[ij];
+      sh.p.u[j] = u;
+      sh.p.base[j] = g.out.off[u] - pj;
+      sh.p.su[j] = (uint32_t)ld_v32(g.val32, u);
+    }
+  }
+  __syncthreads();
+  return m;
+}
+
+template <int A, bool W>
+__global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ DevGraph g,
+                                                       const __grid_constant__ EngineArgs a) {
+  __shared__ EngScan::TempStorage scan_tmp;
+  extern __shared__ __align__(16) unsigned char eng_smem[];
+  EngShared &sh = *reinterpret_cast<EngShared *>(eng_smem);
+  unsigned long long *c = g.ctl;
+  unsigned long long *bnd = a.bar + EB_BND;
+  auto cnt = [&](uint32_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  GridBar bar = {a.bar, 0u};
+  if (threadIdx.x == 0) bar.gen = *reinterpret_cast<volatile unsigned *>(a.bar + EB_GEN);
+  // what the launch before left, read before anything below may change it
+  uint32_t st = (uint32_t)__ldcg(&c[C_STAMP]);
+  uint64_t lvl = a.build ? 0 : __ldcg(&c[C_LEVEL]);
+  if (lead) a.bar[EB_QN2] = a.bar[EB_HVR] = a.bar[EB_HVE] = 0;
+  if (a.build) {
+    init_labels<A>(g, a.root, a.q[0], blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB);
+    if (lead) {
+      prologue_words(c, 0ull);
+      c[C_QN0] = Hook<A>::all_active ? g.V : 1;
+      c[C_ROOT] = a.root;
+      bnd[1] = a.cfg.bnd_worst;  // (the first level's output bound; only builds pull)
+    }
+  }
+  if (!grid_sync(g, bar)) return;
+  if (a.del && !eng_del<A, W>(g, a, bar)) return;
+  bool pulled = false;
+  for (uint32_t k = 0;; k++) {
+    const uint32_t *fin = a.q[k & 1];
+    uint32_t *fout = a.q[(k & 1) ^ 1];
+    unsigned long long *fout_n = cnt(k + 1);
+    const uint64_t n = __ldcg(cnt(k));
+    if (n == 0) break;
+    if (lvl >= a.cfg.max_levels) {
+      if (lead) atomicCAS(&c[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
+      break;
+    }
+    st++;
+    if (lead) {
+      *cnt(k + 2) = 0;
+      bnd[(k + 2) % 3] = a.cfg.bnd_worst;
+      c[C_STAMP] = st;
+      c[C_DEPTH] = lvl;
+      if (lvl < TRACE_CAP) {
+        g.trace[lvl] = n;
+        g.trace[TRACE_CAP + lvl] = global_ns();
+      }
+      c[C_LEVEL] = lvl + 1;
+    }
+    // the mode rules of k_level_begin
+    const bool bu = a.cfg.bottom_up && n * a.cfg.bu_div >= g.V;
+    const bool pull = !bu && a.cfg.allow_pull && n * (pulled ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
+    if (bu) {
+      eng_bottom_up<W>(g, lvl, fout, fout_n);
+    } else if (pull) {
+      const uint32_t m = pulled ? (uint32_t)__ldcg(&bnd[k % 3]) : a.cfg.bnd_best;
+      unsigned long long *bout = &bnd[(k + 1) % 3];
+      eng_pull<A, W>(g, a, sh, a.cfg.pull_split ? PART_HUBS : PART_ALL, m, bout, fout, fout_n);
+      if (!grid_sync(g, bar)) return;
+      eng_hub_fix<A>(g, a, bout, fout, fout_n);
+      if (a.cfg.pull_split) {
+        if (!grid_sync(g, bar)) return;
+        eng_pull<A, W>(g, a, sh, PART_REST, m, bout, fout, fout_n);
+      }
+    } else if (n <= ENG_STAGE) {
+      const uint64_t S = eng_stage(g, sh, scan_tmp, fin, (uint32_t)n);
+      if (S <= a.cfg.tiny_edges && S <= ENG_TINY) {
+        if (!grid_sync(g, bar)) return;  // (every CTA has read the counts that CTA 0 now uses by turns)
+        unsigned long long *at = a.bar + EB_LVL + 2 * (k & 1);  // where CTA 0 got to
+        if (blockIdx.x == 0) {
+          eng_tiny<A, W>(g, a, a.q[k & 1], cnt(k), fout, fout_n,
+                         min((uint64_t)a.cfg.max_levels, lvl + ENG_TINY_LEVELS));
+          if (threadIdx.x == 0) {
+            at[0] = c[C_LEVEL];
+            at[1] = c[C_STAMP];
+          }
+        }
+        if (!grid_sync(g, bar)) return;
+        lvl = __ldcg(&at[0]);
+        st = (uint32_t)__ldcg(&at[1]);
+        pulled = false;
+        continue;
+      }
+      uint64_t e0, e1;
+      eng_share(S, e0, e1);
+      eng_relax<A, W>(g, sh, (uint32_t)n, e0, e1, st, fout, fout_n, a.mst);
+      if (lead) atomicAdd(&c[C_EDGES], (unsigned long long)S);
+    } else {
+      const uint32_t per = (uint32_t)((n + gridDim.x - 1) / gridDim.x);
+      eng_prefix(g, a, scan_tmp, fin, (uint32_t)n, per);
+      if (!grid_sync(g, bar)) return;
+      uint64_t e0, e1;
+      uint32_t i;
+      const uint64_t S = eng_first(a, sh, scan_tmp, (uint32_t)n, per, e0, e1, i);
+      for (uint64_t e = e0; e < e1;) {
+        const uint32_t m = eng_stage_from(g, a, sh, fin, (uint32_t)n, per, i, S);
+        const uint64_t end = min(e1, sh.p.pref[m]);
+        eng_relax<A, W>(g, sh, m, e, end, st, fout, fout_n, a.mst);
+        __syncthreads();
+        e = end;
+        i += m;
+      }
+      if (lead) atomicAdd(&c[C_EDGES], (unsigned long long)S);
+    }
+    pulled = pull;
+    lvl++;
+    if (!grid_sync(g, bar)) return;
+  }
+  if (!grid_sync(g, bar)) return;  // (every CTA has read the last counts)
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      c[C_QN0] = 0;
+      c[C_QN1] = 0;
+      if (lvl < TRACE_CAP) g.trace[TRACE_CAP + lvl] = global_ns();
+    }
+    ctl_to_host(g, a.ctl_host);
+  }
+}
+
 // need_update_tree_add (core/graph.hpp:987-1000) / need_update_tree_del
 // (:1220-1233) per edge.
 template <int A>
@@ -2670,7 +3204,10 @@ int grid_warps(const Graph &g, uint64_t warps) {
 
 uint32_t mod_stamp(Graph &g) { return g.trace ? 1u : 0u; }
 
+// Wait for the call's work and take the control block, which the last kernel
+// may have written to the host's copy itself.
 int read_ctl(Graph &g) {
+  if (g.ctl_on_host) return sync_ctl(g);
   RG_CUDA(cudaMemcpyAsync(g.h_ctl, g.d.ctl, sizeof(unsigned long long) * C_COUNT, cudaMemcpyDeviceToHost, g.stream));
   RG_CUDA(cudaStreamSynchronize(g.stream));
   return RG_OK;
@@ -3292,10 +3829,57 @@ int del_repair_stepped(Graph &g) {
   return RG_OK;
 }
 
+// The engine runs every tree call but those of served graphs (which run without
+// cluster levels, RG_OPT_CLUSTER_EDGES 0) and host-stepped ones.
+bool engine_on(const Graph &g) { return g.eng_ctas && g.cluster_edges && !g.profiling; }
+
+// One engine launch (see k_engine): build from scratch, or the levels of a
+// repair whose frontier is in queue 0, after the deletion repair when `del`.
+// It ends with the control block in the host's copy.
+template <int A, bool W>
+int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
+  EngineArgs a = {};
+  a.cfg = level_cfg(g, A, build);
+  if (a.cfg.allow_pull) {
+    int rc = prepare_pull(g);
+    if (rc) return rc;
+    a.ent = g.sell_ent;
+    a.off = g.sell_off;
+    a.row_id = g.sell_row;
+    a.piece_v = g.sell_piece;
+    a.hub_v = g.sell_hub;
+    a.hub_pc = g.sell_hub_off;
+    a.plan = g.sell_plan;
+    a.piece_best = g.sell_piece_best;
+  }
+  a.q[0] = g.q[0];
+  a.q[1] = g.q[1];
+  a.tree = g.tree;
+  a.P = g.lb_P;
+  a.tot = reinterpret_cast<unsigned long long *>(g.lb_sums);
+  a.bar = g.eng_bar;
+  a.ctl_host = g.h_ctl_dev;
+  a.root = root;
+  a.limit = (uint64_t)((double)g.V * 0.1);  // has_parents guard, core/graph.hpp:1900
+  a.big = recompute_threshold(g);
+  a.max_iter = (uint64_t)g.V + 2;
+  a.mst = mod_stamp(g);
+  a.build = build ? 1 : 0;
+  a.del = del ? 1 : 0;
+  g.h_ctl[C_KLAUNCH] = CTL_PENDING;
+  count_launch(g);
+  void *args[] = {(void *)&g.d, (void *)&a};
+  RG_CUDA(cudaLaunchCooperativeKernel((const void *)k_engine<A, W>, dim3((unsigned)g.eng_ctas), dim3(ENG_TPB), args,
+                                      sizeof(EngShared), g.stream));
+  g.ctl_on_host = true;
+  return RG_OK;
+}
+
 template <int A, bool W>
 int build_enqueue(Graph &g, uint64_t root) {
   int rc = guard_counters(g);
   if (rc) return rc;
+  if (engine_on(g)) return engine_launch<A, W>(g, true, false, root);
   count_launch(g, 2);
   k_prologue<<<1, 1, 0, g.stream>>>(g.d, 0ull);
   k_init<A><<<g.num_sms * 16, TPB, 0, g.stream>>>(g.d, root, g.q[0]);
@@ -3313,6 +3897,7 @@ int add_enqueue(Graph &g, uint64_t n_edges, int directed, bool from_cands) {
       g.d, op_src(g), op_dst(g), op_w(g), from_cands ? op_cand(g) : nullptr, &g.d.ctl[C_CANDN], n_edges, directed,
       g.q[0], &g.d.ctl[C_QN0], mod_stamp(g));
   RG_CUDA(cudaGetLastError());
+  if (engine_on(g)) return engine_launch<A, W>(g, false, false, 0);
   return push_levels<A, W>(g, false);
 }
 
@@ -3332,6 +3917,7 @@ int del_enqueue(Graph &g, uint64_t n_edges, int directed, bool from_cands) {
       g.d, op_src(g), op_dst(g), op_w(g), from_cands ? op_cand(g) : nullptr, &g.d.ctl[C_CANDN], n_edges, directed,
       g.q[0], &g.d.ctl[C_QN0]);
   RG_CUDA(cudaGetLastError());
+  if (engine_on(g)) return engine_launch<A, W>(g, false, true, 0);
   if (g.profiling) {
     rc = del_repair_stepped<A, W>(g);
   } else {
@@ -3350,6 +3936,8 @@ int after_sync(Graph &g, int what) {
   if (g.h_ctl[C_ERR]) {
     int code = (int)g.h_ctl[C_ERR];
     set_error(code == RG_ETIMEOUT ? "push levels did not converge" : "device error in tree update");
+    // (a barrier of the engine that gave up is left half counted)
+    cudaMemsetAsync(g.eng_bar, 0, EB_WORDS * 8, g.stream);
     cudaMemsetAsync(&g.d.ctl[C_ERR], 0, 8, g.stream);
     return code;
   }
@@ -3440,9 +4028,31 @@ static void cluster_setup(Graph &g) {
   cudaGetLastError();
 }
 
+template <int A, bool W>
+static bool engine_fits(const Graph &g) {
+  int n = 0;
+  return cudaFuncSetAttribute(k_engine<A, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EngShared)) ==
+             cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_engine<A, W>, ENG_TPB, sizeof(EngShared)) == cudaSuccess &&
+         n > 0;
+}
+
+// CTAs of the engine: one per SM where the GPU launches cooperatively.
+static void engine_setup(Graph &g) {
+  int coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g.device);
+  const bool fits = coop && engine_fits<RG_BFS, false>(g) && engine_fits<RG_BFS, true>(g) &&
+                    engine_fits<RG_SSSP, false>(g) && engine_fits<RG_SSSP, true>(g) &&
+                    engine_fits<RG_SSWP, false>(g) && engine_fits<RG_SSWP, true>(g) &&
+                    engine_fits<RG_WCC, false>(g) && engine_fits<RG_WCC, true>(g);
+  g.eng_ctas = fits ? std::min(g.num_sms, ENG_MAX_CTAS) : 0;
+  cudaGetLastError();
+}
+
 int tree_alloc(Graph &g) {
   uint64_t V = g.V;
   cluster_setup(g);
+  engine_setup(g);
   auto alloc = [&](void **p, size_t bytes, const char *what) -> int {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
@@ -3474,6 +4084,8 @@ int tree_alloc(Graph &g) {
   if ((rc = alloc((void **)&g.lb_P, V * 8 + 16, "frontier degree prefix"))) return rc;
   if ((rc = alloc((void **)&g.act, V * 4 + 4, "dense-level activity"))) return rc;
   if ((rc = alloc((void **)&g.lb_sums, SC_BLOCKS * 8, "scan block sums"))) return rc;
+  if ((rc = alloc((void **)&g.eng_bar, EB_WORDS * 8, "engine barrier"))) return rc;
+  RG_CUDA(cudaMemset(g.eng_bar, 0, EB_WORDS * 8));
   if ((rc = alloc((void **)&g.sell_plan, sizeof(SellPlan), "pull plan"))) return rc;
   RG_CUDA(cudaHostAlloc(&g.sell_plan_host, sizeof(SellPlan), cudaHostAllocDefault));
   RG_CUDA(cudaMemset(g.act, 0, V * 4 + 4));
@@ -3689,6 +4301,10 @@ int apply_exec(Graph &g, bool add, int directed, cudaGraphExec_t *out) {
 template <int A, bool W>
 int finish_left(Graph &g, unsigned long long left) {
   int rc = RG_OK;
+  if (engine_on(g)) {
+    rc = engine_launch<A, W>(g, false, left == 2 && g.h_ctl[C_OVER], 0);
+    return rc ? rc : read_ctl(g);
+  }
   if (left == 2) {
     cudaGraphExec_t de;
     if ((rc = del_exec<A, W>(g, true, &de))) return rc;
@@ -3698,6 +4314,21 @@ int finish_left(Graph &g, unsigned long long left) {
   if ((rc = loop_exec<A, W>(g, false, &le))) return rc;
   RG_CUDA(cudaGraphLaunch(le, g.stream));
   return read_ctl(g);
+}
+
+// The delete batch of an insert+delete submission in its own kernel, from the
+// staging buffer.
+template <int A, bool W>
+int launch_apply_second(Graph &g, int directed) {
+  const LevelCfg cfg = level_cfg(g, A, false);
+  char *base = reinterpret_cast<char *>(g.stage_host_dev);
+  k_apply_small<A, W><<<1, FS_TPB, 0, g.stream>>>(
+      g.d, sdev::op_view(g), reinterpret_cast<const ApplyHdr *>(base + APPLY_HDR2),
+      base + APPLY_DATA_OFF + apply_data2_off(), reinterpret_cast<uint64_t *>(base + apply_old_off()), op_cand(g), 0,
+      directed ? 1 : 0, g.q[0], mod_stamp(g), 1, fused_repair(g, cfg), reinterpret_cast<uint4 *>(g.stage_dev),
+      g.h_ctl_dev);
+  RG_CUDA(cudaGetLastError());
+  return RG_OK;
 }
 
 // An inline batch from the caller's edges (n <= INLINE_EDGES).
@@ -3843,10 +4474,16 @@ int apply_add_del_t(Graph &g, const rg_edge *adds, uint64_t n_add, const rg_edge
   unsigned long long left = g.h_ctl[C_LEFT];
   if (left == 1) {
     // the insert batch's level loop, then the delete batch in its own kernel
-    cudaGraphExec_t re;
-    if ((rc = rest_exec<A, W>(g, directed, &re))) return rc;
     count_launch(g);
-    RG_CUDA(cudaGraphLaunch(re, g.stream));
+    if (engine_on(g)) {
+      if ((rc = engine_launch<A, W>(g, false, false, 0))) return rc;
+      g.ctl_on_host = false;  // (the kernel after it writes the host's copy last)
+      if ((rc = launch_apply_second<A, W>(g, directed))) return rc;
+    } else {
+      cudaGraphExec_t re;
+      if ((rc = rest_exec<A, W>(g, directed, &re))) return rc;
+      RG_CUDA(cudaGraphLaunch(re, g.stream));
+    }
     RG_CUDA(cudaStreamSynchronize(g.stream));
     if ((rc = storage_error(g))) return rc;
     left = g.h_ctl[C_LEFT];
