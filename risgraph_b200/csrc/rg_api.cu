@@ -243,7 +243,7 @@ int rg_destroy(rg_graph *gh) {
   cudaFree(g.q[0]); cudaFree(g.q[1]); cudaFree(g.tree); cudaFree(g.scratch64); cudaFree(g.hubq); cudaFree(g.d.ctl);
   cudaFree(g.lb_P); cudaFree(g.lb_tile); cudaFree(g.cub_tmp); cudaFree(g.act);
   cudaFree(g.sell_ent); cudaFree(g.sell_off); cudaFree(g.sell_row); cudaFree(g.sell_hub); cudaFree(g.sell_piece);
-  cudaFree(g.sell_plan); cudaFree(g.eng_bar); cudaFree(g.sell_hub_off); cudaFree(g.sell_piece_best); cudaFree(g.lb_sums);
+  cudaFree(g.sell_plan); cudaFree(g.eng_bar); cudaFree(g.sell_hub_best); cudaFree(g.sell_piece_best); cudaFree(g.lb_sums);
   if (g.h_ctl) cudaFreeHost(g.h_ctl);
   if (g.sell_plan_host) cudaFreeHost(g.sell_plan_host);
   if (g.pev[0]) cudaEventDestroy(g.pev[0]);

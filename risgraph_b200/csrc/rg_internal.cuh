@@ -258,18 +258,22 @@ struct HistNode {
 };
 
 // Row counts and slice bounds of the sliced-ELL in-edge copy.  Rows are sorted
-// by length, longest first, so everything about the slices follows from the
-// number of rows of each length: slices [slice[L], slice[L - 1]) are L entries
-// wide and start at entry base[L] of the copy.
-constexpr uint32_t PULL_HUB = 576;  // longest row
-constexpr int SELL_BINS = (int)PULL_HUB + 1;
+// by key, largest first: hub pieces of length L have key PULL_HUB + L, the lists
+// of other vertices their length, so that the pieces come first, and in each
+// part rows of near lengths lie together.  The first vertex row starts a slice.
+// Everything about the slices follows from the number of rows of each key:
+// slices [slice[k], slice[k - 1]) hold rows whose first has key k, are as wide
+// as that row and start at entry base[k] of the copy.
+constexpr uint32_t PULL_HUB = 576;   // longer in-lists are cut into pieces
+constexpr uint32_t PULL_PIECE = 96;  // of at most this many entries
+constexpr int SELL_KEYS = (int)(PULL_HUB + PULL_PIECE) + 1;
 struct SellPlan {
   unsigned long long hubs, pieces;      // vertices cut into pieces, and their pieces
-  unsigned long long rows, slices, total;  // non-empty rows, slices, entries (padding included)
-  unsigned long long base[SELL_BINS];   // first entry of the slices of width L
-  uint32_t count[SELL_BINS];            // rows of length L
-  uint32_t cursor[SELL_BINS];           // where the next row of length L goes
-  uint32_t slice[SELL_BINS];            // first slice of width <= L
+  unsigned long long rows, slices, total;  // rows (and the gap before the vertex rows), slices, entries (padding included)
+  unsigned long long base[SELL_KEYS];
+  uint32_t count[SELL_KEYS];            // rows of the key
+  uint32_t cursor[SELL_KEYS];           // where the next row of the key goes
+  uint32_t slice[SELL_KEYS];            // first slice of key <= k
 };
 
 // A cached, instantiated level-loop graph.
@@ -320,10 +324,10 @@ struct Graph {
   uint64_t sell_off_cap = 0;
   uint32_t *sell_row = nullptr;   // row ids by length, descending: vertex id, or |V| + hub piece index
   uint64_t sell_row_cap = 0;
-  uint32_t *sell_hub = nullptr;   // hub vertices (in-list longer than a row)
+  uint32_t *sell_hub = nullptr;   // hub vertices (in-list longer than PULL_HUB)
   uint64_t sell_hub_cap = 0;
-  uint64_t *sell_hub_off = nullptr;  // first piece of each hub (prefix of piece counts)
-  uint32_t *sell_piece = nullptr;  // pieces: vertex[P+1], start[P+1], length[P+1]
+  unsigned long long *sell_hub_best = nullptr;  // best {value, piece} of each hub in a pull level
+  uint32_t *sell_piece = nullptr;  // pieces: vertex, start, length, hub (sell_piece_cap / 4 each)
   uint64_t sell_piece_cap = 0;
   ulonglong2 *sell_piece_best = nullptr;  // best {value, parent | w << 32} of each piece in a pull level
   uint64_t sell_best_cap = 0;

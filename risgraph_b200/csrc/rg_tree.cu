@@ -605,32 +605,19 @@ __global__ void __launch_bounds__(DN_TPB, 3) k_push_dense(DevGraph g, const uint
 // slice, a slice stored column-major so that lane l of a warp reads row l and
 // the 32 lanes of a warp read 32 consecutive entries.  A row is a vertex's
 // in-list, or for a hub (in-list longer than PULL_HUB) one of the equal pieces
-// its list is cut into, so every row holds at most PULL_HUB entries and the
+// its list is cut into, so every row holds at most PULL_HUB entries, a lane's
+// chain of dependent loads is short (pieces of 576 took 60 us a level on a graph
+// of 150K vertices, most of it one chain), and the
 // warps stay balanced.  A pull level is one warp per slice with no search and
 // no atomics on labels: a vertex row is written only by its own lane; a piece
 // leaves its best in a side array and k_pull_hub_fix combines the pieces of
 // each hub.
 constexpr int PS_TPB = 256;
-// Split pull levels (RG_OPT_PULL_SPLIT): a level runs in two launches, first
-// the slices of the longest in-lists (width >= PULL_SPLIT: the hubs and their
-// pieces), then k_pull_hub_fix, then every other slice.  The second launch
-// reads the hubs' values of this level (a value cached in L1 by the first
-// launch is not carried into the second), where one launch reads them stale
-// from L1 for most of the level, so values move along hub paths faster and
-// fewer levels pull.  On RMAT-22 the WCC build pulls 2 levels instead of 3
-// (1.15 ms against 1.47 unsplit), SSSP 4 instead of 5 (3.96 x E entries read
-// against 4.88; 1.70 ms against 1.73).  The first launch has few, long slices
-// and leaves part of the GPU idle at its end; SSWP, whose values settle in
-// fewer levels anyway, loses more there than it saves (2.05 ms against 1.89),
-// so by default SSSP and WCC split and SSWP does not.  Pieces of at most 576
-// entries and a split at width 288 keep the first launch within one wave of
-// resident warps (2,168 slices for 2,368 warps on RMAT-22; with 512 / 256 it
-// was 2,590 slices, and its last warp ran 42 iterations instead of 36).
-// Without the split the level is one launch over every slice, k_pull_hub_fix,
-// and an empty launch (every level runs the same three kernels).
-constexpr uint32_t PULL_SPLIT = 288;
-// every hub piece (at least PULL_HUB / 2 entries) must fall in the first launch
-static_assert(PULL_SPLIT <= PULL_HUB / 2, "hub pieces must be pulled before k_pull_hub_fix");
+// Split pull levels (RG_OPT_PULL_SPLIT): a level first pulls the hubs' pieces
+// and combines them (pull_hub_fix), then every other row, which reads the hubs'
+// values of this level, where one pass reads them stale from L1 for most of the
+// level: values move along hub paths faster and fewer levels pull.  Without the
+// split all rows go first and the pieces are combined at the end.
 // Entries of a row that a lane reads at a time.
 constexpr int PULL_DEPTH = 8;
 constexpr int PULL_CTAS = 4;  // resident CTAs per SM that the pull kernel's registers allow
@@ -654,20 +641,22 @@ struct SellE<false> {
   static __device__ __forceinline__ uint32_t wt(E) { return 0u; }
 };
 
-// Pieces of a hub of in-list length len: equal lengths of at most PULL_HUB.
-__device__ __forceinline__ uint32_t hub_pieces(uint32_t len) { return (len + PULL_HUB - 1) / PULL_HUB; }
+// Pieces of a hub of in-list length len: equal lengths of at most PULL_PIECE.
+__device__ __forceinline__ uint32_t hub_pieces(uint32_t len) { return (len + PULL_PIECE - 1) / PULL_PIECE; }
+// Entries of a row of key k.
+__host__ __device__ __forceinline__ uint32_t sell_width(uint32_t k) { return k > PULL_HUB ? k - PULL_HUB : k; }
 
 // The copy is laid out in three passes over the vertices' list lengths: count
-// the rows of each length (k_sell_count), turn the counts into row and slice
+// the rows of each key (k_sell_count), turn the counts into row and slice
 // positions (k_sell_plan, one block), and put each row in its place
-// (k_sell_rows).  Lengths are at most PULL_HUB, so a histogram in shared memory
+// (k_sell_rows).  There are few keys, so a histogram in shared memory
 // replaces a sort of all vertices, and the host waits once, for the plan, to
 // size the arrays.  (RMAT-20, 16M weighted edges: the whole preparation takes
 // 0.25 ms; 8.0 ms with a radix sort, five host synchronisations, temporary
 // allocations and one thread copying each row.)
 __global__ void __launch_bounds__(1024) k_sell_count(DevGraph g, uint32_t *hub_v, uint64_t *hub_pc, SellPlan *plan) {
-  __shared__ uint32_t s_n[SELL_BINS];
-  for (int b = threadIdx.x; b < SELL_BINS; b += blockDim.x) s_n[b] = 0;
+  __shared__ uint32_t s_n[SELL_KEYS];
+  for (int b = threadIdx.x; b < SELL_KEYS; b += blockDim.x) s_n[b] = 0;
   __syncthreads();
   const uint64_t V = g.V;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -678,40 +667,45 @@ __global__ void __launch_bounds__(1024) k_sell_count(DevGraph g, uint32_t *hub_v
       const unsigned long long h = atomicAdd(&plan->hubs, 1ull);
       hub_v[h] = (uint32_t)v;
       hub_pc[h] = atomicAdd(&plan->pieces, (unsigned long long)np) | ((uint64_t)np << 32);
-      atomicAdd(&s_n[base], np - extra);
-      if (extra) atomicAdd(&s_n[base + 1], extra);
+      atomicAdd(&s_n[PULL_HUB + base], np - extra);
+      if (extra) atomicAdd(&s_n[PULL_HUB + base + 1], extra);
     } else if (d) {
       atomicAdd(&s_n[d], 1u);
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < SELL_BINS; b += blockDim.x)
+  for (int b = threadIdx.x; b < SELL_KEYS; b += blockDim.x)
     if (s_n[b]) atomicAdd(&plan->count[b], s_n[b]);
 }
 
-// Rows of length L take the positions after all longer ones; slices are 32
-// consecutive rows, as wide as their first.
-__global__ void __launch_bounds__(1024) k_sell_plan(SellPlan *plan) {
-  using Scan = cub::BlockScan<uint64_t, 1024>;
+// Rows of key k take the positions after all larger keys, the first vertex row
+// after a gap to the next slice; slices are 32 consecutive rows, as wide as
+// their first.
+constexpr int SP_TPB = 1024;
+static_assert(SELL_KEYS <= SP_TPB + 1, "one thread per key");
+__global__ void __launch_bounds__(SP_TPB) k_sell_plan(SellPlan *plan) {
+  using Scan = cub::BlockScan<uint64_t, SP_TPB>;
   __shared__ typename Scan::TempStorage tmp;
-  const int t = threadIdx.x, L = (int)PULL_HUB - t;  // longest first
-  const uint64_t n = L >= 1 ? plan->count[L] : 0;
+  const int t = threadIdx.x, k = SELL_KEYS - 1 - t;  // largest first
+  const uint64_t n = k >= 1 ? plan->count[k] : 0;
+  const uint64_t P = plan->pieces, gap = (32 - P % 32) % 32;
   uint64_t row, rows;
   Scan(tmp).ExclusiveSum(n, row, rows);
+  if (k <= (int)PULL_HUB) row += gap;
   const uint64_t s0 = (row + 31) / 32, s1 = (row + n + 31) / 32;
   __syncthreads();
   uint64_t base, total;
-  Scan(tmp).ExclusiveSum(L >= 1 ? 32 * (uint64_t)L * (s1 - s0) : 0, base, total);
-  if (L >= 1) {
-    plan->cursor[L] = (uint32_t)row;
-    plan->slice[L] = (uint32_t)s0;
-    plan->base[L] = base;
+  Scan(tmp).ExclusiveSum(k >= 1 ? 32 * (uint64_t)sell_width(k) * (s1 - s0) : 0, base, total);
+  if (k >= 1) {
+    plan->cursor[k] = (uint32_t)row;
+    plan->slice[k] = (uint32_t)s0;
+    plan->base[k] = base;
   }
   if (t == 0) {
-    plan->rows = rows;
-    plan->slices = (rows + 31) / 32;
+    plan->rows = rows + gap;
+    plan->slices = (rows + gap + 31) / 32;
     plan->total = total;
-    plan->slice[0] = (uint32_t)((rows + 31) / 32);
+    plan->slice[0] = (uint32_t)((rows + gap + 31) / 32);
   }
 }
 
@@ -720,14 +714,15 @@ __global__ void __launch_bounds__(1024) k_sell_plan(SellPlan *plan) {
 // one length together, which keeps rows of near vertices near each other.
 constexpr int SR_TPB = 512, SR_ITEMS = 8;
 
-__global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
+__global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t *hub_v, unsigned long long *hub_pc,
                                                       SellPlan *plan, uint32_t *row_id, uint32_t *piece_v,
-                                                      uint32_t *piece_start, uint32_t *piece_len, uint64_t *off) {
-  __shared__ uint32_t s_n[SELL_BINS], s_at[SELL_BINS];
+                                                      uint32_t *piece_start, uint32_t *piece_len, uint32_t *piece_hub,
+                                                      uint64_t *off) {
+  __shared__ uint32_t s_n[PULL_HUB + 1], s_at[PULL_HUB + 1];
   const uint64_t V = g.V;
   constexpr uint64_t TILE = SR_TPB * SR_ITEMS;
   for (uint64_t b0 = blockIdx.x * TILE; b0 < V; b0 += gridDim.x * TILE) {
-    for (int b = threadIdx.x; b < SELL_BINS; b += SR_TPB) s_n[b] = 0;
+    for (int b = threadIdx.x; b <= (int)PULL_HUB; b += SR_TPB) s_n[b] = 0;
     __syncthreads();
     uint32_t d[SR_ITEMS], at[SR_ITEMS];
 #pragma unroll
@@ -739,7 +734,7 @@ __global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t
 #pragma unroll
     for (int k = 0; k < SR_ITEMS; k++) at[k] = d[k] ? atomicAdd(&s_n[d[k]], 1u) : 0u;
     __syncthreads();
-    for (int b = threadIdx.x; b < SELL_BINS; b += SR_TPB)
+    for (int b = threadIdx.x; b <= (int)PULL_HUB; b += SR_TPB)
       s_at[b] = s_n[b] ? atomicAdd(&plan->cursor[b], s_n[b]) : 0u;
     __syncthreads();
 #pragma unroll
@@ -747,7 +742,7 @@ __global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t
       if (d[k]) row_id[s_at[d[k]] + at[k]] = (uint32_t)(b0 + (uint64_t)k * SR_TPB + threadIdx.x);
     __syncthreads();
   }
-  // one warp per hub writes its pieces
+  // one warp per hub writes its pieces, and clears its best
   const int lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -759,8 +754,8 @@ __global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t
     const uint32_t p0 = (uint32_t)pc, np = (uint32_t)(pc >> 32), base = dv / np, extra = dv % np;
     uint32_t a1 = 0, a0 = 0;  // the first `extra` pieces are one longer
     if (lane == 0) {
-      if (extra) a1 = atomicAdd(&plan->cursor[base + 1], extra);
-      a0 = atomicAdd(&plan->cursor[base], np - extra);
+      if (extra) a1 = atomicAdd(&plan->cursor[PULL_HUB + base + 1], extra);
+      a0 = atomicAdd(&plan->cursor[PULL_HUB + base], np - extra);
     }
     a1 = __shfl_sync(FULL, a1, 0);
     a0 = __shfl_sync(FULL, a0, 0);
@@ -768,24 +763,31 @@ __global__ void __launch_bounds__(SR_TPB) k_sell_rows(DevGraph g, const uint32_t
       piece_v[p0 + k] = v;
       piece_start[p0 + k] = k * base + min(k, extra);
       piece_len[p0 + k] = base + (k < extra ? 1u : 0u);
+      piece_hub[p0 + k] = (uint32_t)h;
       row_id[k < extra ? a1 + k : a0 + (k - extra)] = (uint32_t)(V + p0 + k);
     }
+    __syncwarp();
+    if (lane == 0) hub_pc[h] = ~0ull;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 32) {  // the gap before the vertex rows
+    const uint64_t P = plan->pieces;
+    if (P % 32 && threadIdx.x >= P % 32) row_id[P - P % 32 + threadIdx.x] = NONE;
   }
   const uint64_t ns = plan->slices;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s <= ns; s += stride) {
-    int lo = 1, hi = (int)PULL_HUB;  // the narrowest width L with slice[L] <= s
+    int lo = 1, hi = SELL_KEYS - 1;  // the smallest key k with slice[k] <= s
     while (lo < hi) {
       const int mid = (lo + hi) / 2;
       if (plan->slice[mid] <= s) hi = mid;
       else lo = mid + 1;
     }
-    off[s] = s < ns ? plan->base[lo] + (s - plan->slice[lo]) * 32 * lo : plan->total;
+    off[s] = s < ns ? plan->base[lo] + (s - plan->slice[lo]) * 32 * sell_width(lo) : plan->total;
   }
 }
 
 // Weight classes of the entry order: 0 to 127 exactly, then sixteen to each
-// power of two (device weights are below 2^31, so there are 512).  w_floor /
+// power of two (device weights and ids are below 2^31, so there are 512).  w_floor /
 // w_ceil: the smallest / largest weight of w's class.
 constexpr int W_CLASSES = 512;
 __device__ __forceinline__ uint32_t w_class(uint32_t w) {
@@ -809,8 +811,8 @@ __device__ __forceinline__ RowSrc sell_row_src(const DevGraph &g, const uint32_t
                                                const uint32_t *piece_v, const uint32_t *piece_start,
                                                const uint32_t *piece_len) {
   RowSrc s = {0, 0};
-  if (r < rows) {
-    const uint32_t id = row_id[r];
+  const uint32_t id = r < rows ? row_id[r] : NONE;
+  if (id != NONE) {
     if (id < g.V) {
       s.from = g.in.off[id];
       s.n = seg_len(g.in, id);
@@ -825,7 +827,7 @@ __device__ __forceinline__ RowSrc sell_row_src(const DevGraph &g, const uint32_t
 
 // Copy the live in-entries of each row of slices [s_lo, s_hi) into its column;
 // pad with NONE.  One thread per row, in the order of the pool: for narrow
-// rows, and for rows without weights.
+// rows.
 template <bool W>
 __global__ void k_sell_fill(DevGraph g, const uint32_t *row_id, uint64_t rows, uint64_t s_lo, uint64_t s_hi,
                             const uint64_t *off, const uint32_t *piece_v, const uint32_t *piece_start,
@@ -854,36 +856,42 @@ __global__ void k_sell_fill(DevGraph g, const uint32_t *row_id, uint64_t rows, u
   }
 }
 
-// The same for weighted rows of more than 8 entries, each row's live entries
-// by weight class, lightest first, so that a pull can stop inside the row.
+// The same for rows of more than 8 entries, each row's live entries by class of
+// their weight, lightest first, or without weights of their source's id, lowest
+// first, so that a pull can stop inside the row.
 // One CTA per slice and one warp per row: a lane keeps its K entries in
 // registers (one round trip to the pool), the row's class counts and the
 // sorted slice are in shared memory, and the slice leaves it column-major in
 // coalesced stores.  A row of the tile is padded to an odd number of entries,
 // so that a column of 32 rows touches every bank pair once.
 constexpr int SF_TPB = 1024;
-constexpr size_t sell_fill_smem(int K) { return 32 * (32 * (size_t)K + 1) * 8 + 32 * W_CLASSES * 2; }
+constexpr size_t sell_fill_smem(int K, size_t entry) { return 32 * (32 * (size_t)K + 1) * entry + 32 * W_CLASSES * 2; }
 
-template <int K>
+template <bool W, int K>
 __global__ void __launch_bounds__(SF_TPB) k_sell_fill_sorted(DevGraph g, const uint32_t *row_id, uint64_t rows,
                                                              uint64_t s_lo, uint64_t s_hi, const uint64_t *off,
                                                              const uint32_t *piece_v, const uint32_t *piece_start,
-                                                             const uint32_t *piece_len, uint2 *ent) {
-  extern __shared__ uint2 s_tile[];  // [32 rows][32 K + 1], then [32 rows][W_CLASSES] u16 in pairs
+                                                             const uint32_t *piece_len, typename SellE<W>::E *ent) {
+  using P_ = PoolT<W>;
+  using S_ = SellE<W>;
+  using E = typename S_::E;
+  extern __shared__ __align__(16) unsigned char s_fill[];
+  E *s_tile = reinterpret_cast<E *>(s_fill);  // [32 rows][32 K + 1], then [32 rows][W_CLASSES] u16 in pairs
   constexpr int RS = 32 * K + 1;
   const int lane = lane_id(), row = threadIdx.x >> 5;
   uint32_t *cnt = reinterpret_cast<uint32_t *>(s_tile + 32 * RS) + row * (W_CLASSES / 2);  // two classes per word
   constexpr int CW = W_CLASSES / 64;  // words of classes per lane
-  const uint2 *pool = reinterpret_cast<const uint2 *>(g.in.pool);
+  const E *pool = reinterpret_cast<const E *>(g.in.pool);
+  auto key = [](const E &e) { return w_class(W ? P_::wt(e) : P_::nbr(e)); };
   for (uint64_t s = s_lo + blockIdx.x; s < s_hi; s += gridDim.x) {
     const uint64_t o0 = off[s];
     const uint32_t width = (uint32_t)((off[s + 1] - o0) >> 5);
     const RowSrc src = sell_row_src(g, row_id, s * 32 + row, rows, piece_v, piece_start, piece_len);
-    uint2 e[K];
+    E e[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
       const uint32_t i = 32 * k + lane;
-      e[k] = i < src.n ? pool[src.from + i] : make_uint2(NONE, 0u);
+      e[k] = i < src.n ? pool[src.from + i] : S_::none();
     }
 #pragma unroll
     for (int k = 0; k < CW; k++) cnt[32 * k + lane] = 0;
@@ -892,8 +900,8 @@ __global__ void __launch_bounds__(SF_TPB) k_sell_fill_sorted(DevGraph g, const u
 #pragma unroll
     for (int k = 0; k < K; k++) {
       at[k] = 0;
-      if (!(e[k].x & DEAD)) {  // (NONE has the bit too)
-        const uint32_t c = w_class(e[k].y);
+      if (!(P_::nbr(e[k]) & DEAD)) {  // (NONE has the bit too)
+        const uint32_t c = key(e[k]);
         at[k] = (atomicAdd(&cnt[c >> 1], 1u << (16 * (c & 1))) >> (16 * (c & 1))) & 0xFFFFu;
       }
     }
@@ -923,12 +931,12 @@ __global__ void __launch_bounds__(SF_TPB) k_sell_fill_sorted(DevGraph g, const u
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      if (!(e[k].x & DEAD)) {
-        const uint32_t c = w_class(e[k].y);
+      if (!(P_::nbr(e[k]) & DEAD)) {
+        const uint32_t c = key(e[k]);
         s_tile[row * RS + ((cnt[c >> 1] >> (16 * (c & 1))) & 0xFFFFu) + at[k]] = e[k];
       }
     }
-    for (uint32_t j = live + lane; j < width; j += 32) s_tile[row * RS + j] = make_uint2(NONE, 0u);
+    for (uint32_t j = live + lane; j < width; j += 32) s_tile[row * RS + j] = S_::none();
     __syncthreads();
     for (uint32_t j = row; j < width; j += 32) ent[o0 + (uint64_t)j * 32 + lane] = s_tile[lane * RS + j];
     __syncthreads();
@@ -986,9 +994,11 @@ __device__ __forceinline__ void pull_take(const typename SellE<W>::E &e, uint32_
   }
 }
 
-// A warp's new frontier entries, collected in shared memory and written to the
-// queue PQ_CAP at a time: one atomic on the queue's counter and one round trip
-// for a buffer instead of for every slice.
+// A warp's new frontier entries, collected in shared memory: a full buffer goes
+// to the queue with one atomic on its counter, and at the end the CTA's buffers
+// go together.  (One atomic for every slice with a change, and one for every
+// warp on each of the counts, took most of a level on graphs of 10^5 vertices:
+// same-address atomics are served one after the other.)
 constexpr uint32_t PQ_CAP = 128;
 struct PullQueue {
   uint32_t *buf;  // this warp's PQ_CAP entries
@@ -998,7 +1008,7 @@ struct PullQueue {
 __device__ __forceinline__ void pull_flush(PullQueue &q, uint32_t *fout, unsigned long long *fout_n) {
   const uint32_t lane = (uint32_t)lane_id();
   unsigned long long base = 0;
-  if (lane == 0 && q.n) base = atomicAdd(fout_n, (unsigned long long)q.n);
+  if (lane == 0) base = atomicAdd(fout_n, (unsigned long long)q.n);
   base = __shfl_sync(FULL, base, 0);
   __syncwarp();
   for (uint32_t i = lane; i < q.n; i += 32) fout[base + i] = q.buf[i];
@@ -1006,39 +1016,111 @@ __device__ __forceinline__ void pull_flush(PullQueue &q, uint32_t *fout, unsigne
   q.n = 0;
 }
 
+// Append by every lane with pred set.
+__device__ __forceinline__ void pull_append(PullQueue &q, bool pred, uint32_t v, uint32_t *fout,
+                                            unsigned long long *fout_n) {
+  const unsigned b = __ballot_sync(FULL, pred);
+  if (b) {
+    if (pred) q.buf[q.n + __popc(b & ((1u << lane_id()) - 1))] = v;
+    q.n += __popc(b);
+    if (q.n > PQ_CAP - 32) pull_flush(q, fout, fout_n);
+  }
+}
+
+// Work counts of a CTA, summed in shared memory.
+struct BlockCounts {
+  unsigned long long updates, scanned;
+};
+__device__ __forceinline__ void block_count(BlockCounts *bc, unsigned long long updates, unsigned long long scanned) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    updates += __shfl_down_sync(FULL, updates, o);
+    scanned += __shfl_down_sync(FULL, scanned, o);
+  }
+  if (lane_id() == 0) {
+    if (updates) atomicAdd(&bc->updates, updates);
+    if (scanned) atomicAdd(&bc->scanned, scanned);
+  }
+}
+
+// End of a pass (all threads of the CTA): what the warps' buffers still hold
+// goes to the queue with one atomic per CTA.
+__device__ __forceinline__ void pull_drain(PullQueue &q, uint32_t *fout, unsigned long long *fout_n) {
+  __shared__ unsigned long long s_at[32];
+  const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (lane == 0) s_at[w] = q.n;
+  __syncthreads();
+  if (w == 0) {
+    const uint32_t n = lane < nw ? (uint32_t)s_at[lane] : 0u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= (unsigned)o) incl += y;
+    }
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(fout_n, (unsigned long long)incl);
+    base = __shfl_sync(FULL, base, 31);
+    if (lane < nw) s_at[lane] = base + incl - n;
+  }
+  __syncthreads();
+  for (uint32_t i = lane; i < q.n; i += 32) fout[s_at[w] + i] = q.buf[i];
+  __syncthreads();
+  q.n = 0;
+}
+
 // Commit of one pulled row (all lanes of the warp call it): a vertex has a
-// single writer, so its label needs no atomic; a piece leaves its best for
-// k_pull_hub_fix.  fb: the best value committed by this thread.
+// single writer, so its label needs no atomic; a piece that improves its hub
+// leaves its best for pull_hub_fix, and its number with its hub if no other
+// piece has a better value.  fb: the best value committed by this thread.
+struct PullHubs {
+  const uint32_t *piece_v, *piece_hub, *hub_v;
+  ulonglong2 *piece_best;        // {value, parent | w << 32}
+  unsigned long long *hub_best;  // {order of the value, piece}; all ones: none
+};
+// Values as words that a minimum orders best first.
+template <int A>
+__device__ __forceinline__ uint64_t hub_order(uint32_t v) {
+  return (uint64_t)(A == RG_SSWP ? ~v : v) << 32;
+}
+
 template <int A>
 __device__ __forceinline__ void pull_row_done(const DevGraph &g, bool active, uint32_t id, const PullRow &p,
-                                              ulonglong2 *piece_best, PullQueue &q, uint32_t *fout,
+                                              const PullHubs &hubs, PullQueue &q, uint32_t *fout,
                                               unsigned long long *fout_n, uint32_t mst, uint32_t &local, uint32_t &fb) {
   const bool upd = active && id < g.V && p.has;
   if (upd) {
     g.lab[id] = make_ulonglong2(p.best, pack_parent(p.bsrc, p.bw));
     g.val32[id] = p.best;
     if (better32<A>(p.best, fb)) fb = p.best;
-  } else if (active && id >= g.V) {
-    piece_best[id - g.V] = make_ulonglong2(p.best, p.has ? pack_parent(p.bsrc, p.bw) : ~0ull);
+  } else if (active && p.has) {
+    const uint32_t pi = id - g.V;
+    hubs.piece_best[pi] = make_ulonglong2(p.best, pack_parent(p.bsrc, p.bw));
+    atomicMin(&hubs.hub_best[hubs.piece_hub[pi]], (unsigned long long)(hub_order<A>(p.best) | pi));
   }
   local += upd;
-  const unsigned b = __ballot_sync(FULL, upd);
-  if (b) {
-    if (upd) q.buf[q.n + __popc(b & ((1u << lane_id()) - 1))] = id;
-    q.n += __popc(b);
-    if (q.n > PQ_CAP - 32) pull_flush(q, fout, fout_n);
-  }
+  pull_append(q, upd, id, fout, fout_n);
   if (mst) mark_modified(g, upd, id, mst);
 }
 
-// The best value committed by the warp, into the bound of the next frontier.
+// The best value committed by the CTA, into the bound of the next frontier (all
+// threads of the CTA).
 template <int A>
 __device__ __forceinline__ void pull_bound_out(uint32_t fb, unsigned long long *bout) {
+  __shared__ uint32_t s_b[32];
+  const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const uint32_t b = A == RG_SSWP ? __reduce_max_sync(FULL, fb) : __reduce_min_sync(FULL, fb);
-  if (lane_id() == 0 && better32<A>(b, (uint32_t)__ldcg(bout))) {
-    if (A == RG_SSWP) atomicMax(bout, (unsigned long long)b);
-    else atomicMin(bout, (unsigned long long)b);
+  if (lane == 0) s_b[w] = b;
+  __syncthreads();
+  if (w == 0) {
+    const uint32_t x = s_b[lane < nw ? lane : 0];
+    const uint32_t y = A == RG_SSWP ? __reduce_max_sync(FULL, x) : __reduce_min_sync(FULL, x);
+    if (lane == 0) {
+      if (A == RG_SSWP) atomicMax(bout, (unsigned long long)y);
+      else atomicMin(bout, (unsigned long long)y);
+    }
   }
+  __syncthreads();
 }
 template <int A>
 __device__ __forceinline__ uint32_t pull_worst() {
@@ -1057,42 +1139,40 @@ __device__ __forceinline__ uint32_t pull_src_val(const DevGraph &g, uint32_t u) 
 // registers a thread and left a quarter of the warps resident.)
 template <int A, bool W, int G>
 __device__ __forceinline__ void pull_narrow(const DevGraph &g, const typename SellE<W>::E *ent, const uint64_t *off,
-                                            const uint32_t *row_id, uint32_t rows, uint32_t lo, uint32_t hi, uint32_t m,
+                                            const uint32_t *row_id, uint32_t rows, uint32_t s0, uint32_t hi, uint32_t m,
                                             PullQueue &q, uint32_t *fout, unsigned long long *fout_n, uint32_t mst,
-                                            uint32_t &local, uint32_t &fb, uint32_t warp, uint32_t nwarps) {
+                                            uint32_t &local, uint32_t &fb) {
   using S_ = SellE<W>;
   constexpr int NP = PULL_DEPTH / G;
   const int lane = lane_id();
-  for (uint32_t s0 = lo + warp * G; s0 < hi; s0 += nwarps * G) {
-    typename S_::E e[PULL_DEPTH];
-    uint32_t id[G];
+  typename S_::E e[PULL_DEPTH];
+  uint32_t id[G];
 #pragma unroll
-    for (int gi = 0; gi < G; gi++) {
-      const uint32_t s = s0 + gi;
-      const uint64_t o = s < hi ? off[s] : 0;
-      const uint32_t w = s < hi ? (uint32_t)((off[s + 1] - o) >> 5) : 0u;
-      id[gi] = s < hi && s * 32 + lane < rows ? row_id[s * 32 + lane] : NONE;
+  for (int gi = 0; gi < G; gi++) {
+    const uint32_t s = s0 + gi;
+    const uint64_t o = s < hi ? off[s] : 0;
+    const uint32_t w = s < hi ? (uint32_t)((off[s + 1] - o) >> 5) : 0u;
+    id[gi] = s < hi && s * 32 + lane < rows ? row_id[s * 32 + lane] : NONE;
 #pragma unroll
-      for (int k = 0; k < NP; k++) e[gi * NP + k] = k < w ? __ldcs(&ent[o + (uint64_t)k * 32 + lane]) : S_::none();
-    }
-    uint32_t cur[G];
+    for (int k = 0; k < NP; k++) e[gi * NP + k] = k < w ? __ldcs(&ent[o + (uint64_t)k * 32 + lane]) : S_::none();
+  }
+  uint32_t cur[G];
 #pragma unroll
-    for (int gi = 0; gi < G; gi++) cur[gi] = id[gi] != NONE ? __ldcg(&g.val32[id[gi]]) : 0u;
-    uint32_t sv[PULL_DEPTH];
-    bool on[PULL_DEPTH];
+  for (int gi = 0; gi < G; gi++) cur[gi] = id[gi] != NONE ? __ldcg(&g.val32[id[gi]]) : 0u;
+  uint32_t sv[PULL_DEPTH];
+  bool on[PULL_DEPTH];
 #pragma unroll
-    for (int k = 0; k < PULL_DEPTH; k++) {
-      on[k] = S_::nbr(e[k]) != NONE && pull_open<A>(m, S_::wt(e[k]), cur[k / NP]);
-      sv[k] = on[k] ? pull_src_val(g, S_::nbr(e[k])) : 0u;
-    }
+  for (int k = 0; k < PULL_DEPTH; k++) {
+    on[k] = S_::nbr(e[k]) != NONE && pull_open<A>(m, S_::wt(e[k]), cur[k / NP]);
+    sv[k] = on[k] ? pull_src_val(g, S_::nbr(e[k])) : 0u;
+  }
 #pragma unroll
-    for (int gi = 0; gi < G; gi++) {
-      PullRow p = {cur[gi], 0u, 0u, false};
+  for (int gi = 0; gi < G; gi++) {
+    PullRow p = {cur[gi], 0u, 0u, false};
 #pragma unroll
-      for (int k = 0; k < NP; k++) pull_take<A, W>(e[gi * NP + k], sv[gi * NP + k], on[gi * NP + k], p);
-      // (a row this narrow is a vertex)
-      pull_row_done<A>(g, id[gi] != NONE, id[gi], p, nullptr, q, fout, fout_n, mst, local, fb);
-    }
+    for (int k = 0; k < NP; k++) pull_take<A, W>(e[gi * NP + k], sv[gi * NP + k], on[gi * NP + k], p);
+    // (a row this narrow is a vertex)
+    pull_row_done<A>(g, id[gi] != NONE, id[gi], p, PullHubs{}, q, fout, fout_n, mst, local, fb);
   }
 }
 
@@ -1107,42 +1187,64 @@ enum PullPart : int { PART_HUBS, PART_REST, PART_ALL, PART_NONE, PART_RANGE };
 // (q_buf: this warp's PQ_CAP words of shared memory)
 template <int A, bool W>
 __device__ __forceinline__ void pull_part(const DevGraph &g, const typename SellE<W>::E *ent, const uint64_t *off,
-                                          const uint32_t *row_id, const uint32_t *piece_v, const SellPlan *plan,
+                                          const uint32_t *row_id, const PullHubs &hubs, const SellPlan *plan,
                                           int part, uint32_t s_lo, uint32_t s_hi, int rest, uint32_t m,
-                                          unsigned long long *bout, ulonglong2 *piece_best, uint32_t *q_buf,
-                                          uint32_t *fout, unsigned long long *fout_n, uint32_t mst,
-                                          unsigned long long &updates, unsigned long long &scanned, uint32_t warp,
-                                          uint32_t nwarps) {
+                                          unsigned long long *bout, uint32_t *q_buf, uint32_t *fout,
+                                          unsigned long long *fout_n, uint32_t mst, BlockCounts *bc, bool first,
+                                          uint32_t warp, uint32_t nwarps) {
   using S_ = SellE<W>;
   constexpr bool rev = A == RG_SSWP;  // heaviest entries first
   constexpr bool by_w = W && (A == RG_SSSP || A == RG_SSWP);
+  constexpr bool by_id = !W && A == RG_WCC;
   constexpr int N = PULL_DEPTH;
   const uint32_t rows = (uint32_t)plan->rows, c4 = plan->slice[4];
   if (part != PART_RANGE) {
-    const uint32_t mid = plan->slice[PULL_SPLIT - 1];
+    const uint32_t mid = plan->slice[PULL_HUB];
     s_lo = part == PART_REST ? mid : 0;
     s_hi = part == PART_HUBS ? mid : c4;
     rest = part != PART_HUBS;
   }
+  // the warps' work items: the wide slices one by one, then the narrow ones
+  // in groups of 2, 4 and 8, so that on a small graph, where each warp has one
+  // item, the classes run side by side
+  const uint32_t c2 = plan->slice[2], c1 = plan->slice[1], slices = (uint32_t)plan->slices;
+  const uint32_t n1 = s_hi - s_lo, n2 = rest ? (c2 - c4 + 1) / 2 : 0, n4 = rest ? (c1 - c2 + 3) / 4 : 0,
+                 n8 = rest ? (slices - c1 + 7) / 8 : 0;
   const int lane = lane_id();
   PullQueue q = {q_buf, 0u};
   uint32_t fb = pull_worst<A>();
   uint32_t local = 0, chunks = 0;
-  for (uint32_t s = s_lo + warp; s < s_hi; s += nwarps) {
-    const uint32_t r = s * 32 + lane;
-    const bool active = r < rows;
-    const uint32_t id = active ? row_id[r] : 0u;
+  unsigned long long scanned = 0;
+  for (uint32_t i = warp; i < n1 + n2 + n4 + n8; i += nwarps) {
+    if (i >= n1) {
+      const uint32_t x = i - n1;
+      if (x < n2)
+        pull_narrow<A, W, 2>(g, ent, off, row_id, rows, c4 + 2 * x, c2, m, q, fout, fout_n, mst, local, fb);
+      else if (x < n2 + n4)
+        pull_narrow<A, W, 4>(g, ent, off, row_id, rows, c2 + 4 * (x - n2), c1, m, q, fout, fout_n, mst, local, fb);
+      else
+        pull_narrow<A, W, 8>(g, ent, off, row_id, rows, c1 + 8 * (x - n2 - n4), slices, m, q, fout, fout_n, mst, local,
+                             fb);
+      continue;
+    }
+    const uint32_t s = s_lo + i, r = s * 32 + lane;
+    const uint32_t id = r < rows ? row_id[r] : NONE;
+    const bool active = id != NONE;
     const uint64_t o0 = off[s];
     const uint32_t width = (uint32_t)((off[s + 1] - o0) >> 5);
     const typename S_::E *col = ent + o0 + lane;
-    typename S_::E e[N];
+    auto load = [&](typename S_::E(&x)[N], uint32_t j, bool on) {
 #pragma unroll
-    for (int k = 0; k < N; k++)  // (the first entries travel with the row's value)
-      e[k] = active && k < width ? __ldcs(&col[(rev ? width - 1 - k : k) * 32]) : S_::none();
+      for (int k = 0; k < N; k++)
+        x[k] = on && j + k < width ? __ldcs(&col[(rev ? width - 1 - (j + k) : j + k) * 32]) : S_::none();
+    };
+    typename S_::E e[N];
+    load(e, 0, true);  // (the first entries travel with the row's value)
     PullRow p = {0u, 0u, 0u, false};
-    if (active) p.best = __ldcg(&g.val32[id < g.V ? id : piece_v[id - g.V]]);
+    if (active) p.best = __ldcg(&g.val32[id < g.V ? id : hubs.piece_v[id - g.V]]);
     bool live = active && pull_open<A>(m, A == RG_SSWP ? 0xFFFFFFFFu : 0u, p.best);
-    for (uint32_t j = N;; j += N) {
+    // takes the entries held and says whether the row goes on
+    auto take = [&](uint32_t next) -> bool {
       uint32_t sv[N];
       bool on[N];
 #pragma unroll
@@ -1153,79 +1255,88 @@ __device__ __forceinline__ void pull_part(const DevGraph &g, const typename Sell
 #pragma unroll
       for (int k = 0; k < N; k++) pull_take<A, W>(e[k], sv[k], on[k], p);
       chunks += live;
-      if (j >= width) break;
+      if (next >= width) return false;
       if constexpr (by_w) {
         // padding ends a row read forwards and comes first in one read backwards
         if (S_::nbr(e[N - 1]) == NONE) live = live && rev;
         else live = live && pull_more<A>(m, S_::wt(e[N - 1]), p.best);
       } else {
         live = live && pull_open<A>(m, 0u, p.best);
+        // WCC's first level starts with every label its vertex's id, and the
+        // rows are in order of ids: the sources still to come start above the
+        // best (those that changed in this level are in the next frontier)
+        if (by_id && first)
+          live = live && S_::nbr(e[N - 1]) != NONE && better32<A>(w_floor(S_::nbr(e[N - 1])), p.best);
       }
-      if (!__any_sync(FULL, live)) break;
+      return __any_sync(FULL, live);
+    };
+    if (take(N)) {
+      // past its first entries a row is likely to go on: the next ones are on
+      // their way while these are taken
+      load(e, N, live);
+      for (uint32_t j = 2 * N;; j += N) {
+        typename S_::E ne[N];
+        load(ne, j, live);
+        if (!take(j)) break;
 #pragma unroll
-      for (int k = 0; k < N; k++)
-        e[k] = live && j + k < width ? __ldcs(&col[(rev ? width - 1 - (j + k) : j + k) * 32]) : S_::none();
+        for (int k = 0; k < N; k++) e[k] = ne[k];
+      }
     }
-    pull_row_done<A>(g, active, id, p, piece_best, q, fout, fout_n, mst, local, fb);
+    pull_row_done<A>(g, active, id, p, hubs, q, fout, fout_n, mst, local, fb);
   }
   scanned += (unsigned long long)chunks * N;
-  if (rest) {
-    const uint32_t c2 = plan->slice[2], c1 = plan->slice[1], slices = (uint32_t)plan->slices;
-    pull_narrow<A, W, 2>(g, ent, off, row_id, rows, c4, c2, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
-    pull_narrow<A, W, 4>(g, ent, off, row_id, rows, c2, c1, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
-    pull_narrow<A, W, 8>(g, ent, off, row_id, rows, c1, slices, m, q, fout, fout_n, mst, local, fb, warp, nwarps);
-    if (blockIdx.x == 0 && threadIdx.x == 0) scanned += off[slices] - off[c4];
-  }
-  pull_flush(q, fout, fout_n);
+  if (rest && blockIdx.x == 0 && threadIdx.x == 0) scanned += off[slices] - off[c4];
+  pull_drain(q, fout, fout_n);
   pull_bound_out<A>(fb, bout);
-  updates += local;
+  block_count(bc, local, scanned);
+}
+
+// A CTA's counts into the control block (all threads of the CTA).
+__device__ __forceinline__ void counts_out(const DevGraph &g, BlockCounts *bc) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (bc->updates) atomicAdd(&g.ctl[C_RESULT], bc->updates);
+    if (bc->scanned) atomicAdd(&g.ctl[C_EDGES], bc->scanned);
+  }
 }
 
 template <int A, bool W>
 __global__ void __launch_bounds__(PS_TPB, PULL_CTAS)
-    k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off, const uint32_t *row_id,
-                const uint32_t *piece_v, const SellPlan *plan, int part, uint32_t s_lo, uint32_t s_hi, int rest,
-                const unsigned long long *bin, unsigned long long *bout, ulonglong2 *piece_best, uint32_t *fout,
-                unsigned long long *fout_n, uint32_t mst) {
+    k_pull_sell(DevGraph g, const typename SellE<W>::E *ent, const uint64_t *off, const uint32_t *row_id, PullHubs hubs,
+                const SellPlan *plan, int part, uint32_t s_lo, uint32_t s_hi, int rest, const unsigned long long *bin,
+                unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n, uint32_t mst) {
   if (g.ctl[C_MODE] != M_PULL || part == PART_NONE) return;
   __shared__ uint32_t s_q[PS_TPB / 32][PQ_CAP];
-  unsigned long long local = 0, scanned = 0;
-  pull_part<A, W>(g, ent, off, row_id, piece_v, plan, part, s_lo, s_hi, rest, (uint32_t)*bin, bout, piece_best,
-                  s_q[threadIdx.x >> 5], fout, fout_n, mst, local, scanned,
-                  (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
-  warp_add_result(local, &g.ctl[C_RESULT]);
-  warp_add_result(scanned, &g.ctl[C_EDGES]);
+  __shared__ BlockCounts s_bc;
+  if (threadIdx.x == 0) s_bc = BlockCounts{0, 0};
+  __syncthreads();
+  pull_part<A, W>(g, ent, off, row_id, hubs, plan, part, s_lo, s_hi, rest, (uint32_t)*bin, bout, s_q[threadIdx.x >> 5],
+                  fout, fout_n, mst, &s_bc, g.ctl[C_DEPTH] == 0, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                  (gridDim.x * blockDim.x) >> 5);
+  counts_out(g, &s_bc);
 }
 
-// One warp per hub: best of its pieces, one write.
+// The best piece of each hub, one lane per hub, one write (pieces only compete
+// when they improve their hub).
 template <int A>
-__device__ __forceinline__ void pull_hub_fix(const DevGraph &g, const uint32_t *hub_v, const uint64_t *hub_pc,
-                                             const SellPlan *plan, const ulonglong2 *piece_best,
+__device__ __forceinline__ void pull_hub_fix(const DevGraph &g, const PullHubs &hubs, const SellPlan *plan,
                                              unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n,
-                                             uint32_t mst, unsigned long long &local, uint32_t warp, uint32_t nwarps) {
-  const int lane = lane_id();
+                                             uint32_t mst, unsigned long long &local, uint64_t gtid,
+                                             uint64_t gthreads) {
   const uint64_t nh = plan->hubs;
   uint32_t fb = pull_worst<A>();
-  for (uint64_t h = warp; h < nh; h += nwarps) {
-    const uint32_t v = hub_v[h];
-    const uint64_t pc = hub_pc[h];
-    const uint32_t p0 = (uint32_t)pc, np = (uint32_t)(pc >> 32);
-    uint32_t best = pull_worst<A>();
-    uint64_t meta = ~0ull;
-    for (uint32_t k = lane; k < np; k += 32) {
-      const ulonglong2 b = __ldcg(&piece_best[p0 + k]);
-      if (b.y != ~0ull && (meta == ~0ull || better32<A>((uint32_t)b.x, best))) {
-        best = (uint32_t)b.x;
-        meta = b.y;
-      }
-    }
-    const uint32_t top = A == RG_SSWP ? __reduce_max_sync(FULL, best) : __reduce_min_sync(FULL, best);
-    const unsigned won = __ballot_sync(FULL, meta != ~0ull && best == top);
-    const bool upd = won && lane == __ffs(won) - 1;
+  for (uint64_t h0 = gtid - lane_id(); h0 < nh; h0 += gthreads) {
+    const uint64_t h = h0 + lane_id();
+    const unsigned long long b = h < nh ? __ldcg(&hubs.hub_best[h]) : ~0ull;
+    const bool upd = b != ~0ull;
+    uint32_t v = 0;
     if (upd) {
-      g.lab[v] = make_ulonglong2(best, meta);
-      g.val32[v] = best;
-      if (better32<A>(best, fb)) fb = best;
+      v = hubs.hub_v[h];
+      const ulonglong2 lab = __ldcg(&hubs.piece_best[(uint32_t)b]);
+      hubs.hub_best[h] = ~0ull;
+      g.lab[v] = lab;
+      g.val32[v] = (uint32_t)lab.x;
+      if (better32<A>((uint32_t)lab.x, fb)) fb = (uint32_t)lab.x;
     }
     local += upd;
     warp_append(upd, v, fout, fout_n, FULL);
@@ -1235,14 +1346,13 @@ __device__ __forceinline__ void pull_hub_fix(const DevGraph &g, const uint32_t *
 }
 
 template <int A>
-__global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t *hub_v, const uint64_t *hub_pc,
-                                                      const SellPlan *plan, const ulonglong2 *piece_best,
+__global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, PullHubs hubs, const SellPlan *plan,
                                                       unsigned long long *bout, uint32_t *fout,
                                                       unsigned long long *fout_n, uint32_t mst) {
   if (g.ctl[C_MODE] != M_PULL) return;
   unsigned long long local = 0;
-  pull_hub_fix<A>(g, hub_v, hub_pc, plan, piece_best, bout, fout, fout_n, mst, local,
-                  (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
+  pull_hub_fix<A>(g, hubs, plan, bout, fout, fout_n, mst, local, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+                  (uint64_t)gridDim.x * blockDim.x);
   warp_add_result(local, &g.ctl[C_RESULT]);
 }
 
@@ -1251,55 +1361,94 @@ __global__ void __launch_bounds__(256) k_pull_hub_fix(DevGraph g, const uint32_t
 // its in-edges and takes the first in-neighbour at depth d as its parent,
 // stopping there.  Used when the frontier is large; each vertex is written
 // only by its own thread, so no atomics on labels.
-// The in-list is read four entries at a time: the search is a chain of dependent
-// loads, and most vertices find a parent in the first few entries.
+// Most vertices find a parent in the first few entries: each thread reads up to
+// BU_ALONE of its own list, four at a time (the search is a chain of dependent
+// loads), and the warp then searches what is left of each longer list together.
+constexpr uint32_t BU_ALONE = 8;
 template <bool W>
 __device__ __forceinline__ void bottom_up(const DevGraph &g, uint64_t d, uint32_t *fout, unsigned long long *fout_n,
-                                          uint64_t gtid, uint64_t gthreads, unsigned long long &local,
-                                          unsigned long long &scanned) {
+                                          uint64_t gtid, uint64_t gthreads, uint32_t *q_buf, BlockCounts *bc) {
+  PullQueue q = {q_buf, 0u};
+  unsigned long long local = 0, scanned = 0;
   using P_ = PoolT<W>;
   const typename P_::E *pool = reinterpret_cast<const typename P_::E *>(g.in.pool);
   const uint64_t V = g.V;
   const int lane = lane_id();
+  // (a stale value only hides a parent found this level)
+  auto is_parent = [&](uint32_t u) { return !(u & DEAD) && __ldca(&g.val32[u]) == (uint32_t)d; };
   for (uint64_t v0 = gtid - lane; v0 < V; v0 += gthreads) {
     const uint64_t v = v0 + lane;
-    bool found = false;
+    uint32_t parent = NONE, pw = 0, len = 0;
+    uint64_t off = 0;
     if (v < V && ld_v32(g.val32, (uint32_t)v) == BFS_MAXL) {
-      const uint32_t len = seg_len(g.in, (uint32_t)v);
-      const uint64_t off = g.in.off[v];
-      for (uint32_t k = 0; k < len && !found; k += 4) {
+      len = seg_len(g.in, (uint32_t)v);
+      off = g.in.off[v];
+      for (uint32_t k = 0; k < len && k < BU_ALONE && parent == NONE; k += 4) {
         typename P_::E e[4];
-        uint32_t sv[4];
+        bool ok[4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
           if (k + i < len) e[i] = pool[off + k + i];
 #pragma unroll
-        for (int i = 0; i < 4; i++)  // a stale value only hides a parent found this level
-          sv[i] = k + i < len && !(P_::nbr(e[i]) & DEAD) ? __ldca(&g.val32[P_::nbr(e[i])]) : NONE;
+        for (int i = 0; i < 4; i++) ok[i] = k + i < len && is_parent(P_::nbr(e[i]));
         scanned += min(4u, len - k);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          if (!found && sv[i] == d) {
-            g.lab[v] = make_ulonglong2(d + 1, pack_parent(P_::nbr(e[i]), P_::wt(e[i])));
-            g.val32[v] = (uint32_t)(d + 1);
-            found = true;
+          if (parent == NONE && ok[i]) {
+            parent = P_::nbr(e[i]);
+            pw = P_::wt(e[i]);
           }
         }
       }
     }
+    for (unsigned rest = __ballot_sync(FULL, parent == NONE && len > BU_ALONE); rest; rest &= rest - 1) {
+      const int l = __ffs(rest) - 1;
+      const uint32_t n = __shfl_sync(FULL, len, l);
+      const uint64_t o = __shfl_sync(FULL, off, l);
+      for (uint32_t k = BU_ALONE; k < n; k += 64) {
+        typename P_::E e[2];
+        bool ok[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+          if (k + 32 * i + lane < n) e[i] = pool[o + k + 32 * i + lane];
+#pragma unroll
+        for (int i = 0; i < 2; i++) ok[i] = k + 32 * i + lane < n && is_parent(P_::nbr(e[i]));
+        if (lane == l) scanned += min(64u, n - k);
+        const unsigned hit = __ballot_sync(FULL, ok[0] || ok[1]);
+        if (hit) {
+          const int h = __ffs(hit) - 1;
+          const uint32_t hp = __shfl_sync(FULL, ok[0] ? P_::nbr(e[0]) : P_::nbr(e[1]), h);
+          const uint32_t hw = __shfl_sync(FULL, ok[0] ? P_::wt(e[0]) : P_::wt(e[1]), h);
+          if (lane == l) {
+            parent = hp;
+            pw = hw;
+          }
+          break;
+        }
+      }
+    }
+    const bool found = parent != NONE;
+    if (found) {
+      g.lab[v] = make_ulonglong2(d + 1, pack_parent(parent, pw));
+      g.val32[v] = (uint32_t)(d + 1);
+    }
     local += found;
-    warp_append(found, (uint32_t)v, fout, fout_n, FULL);
+    pull_append(q, found, (uint32_t)v, fout, fout_n);
   }
+  pull_drain(q, fout, fout_n);
+  block_count(bc, local, scanned);
 }
 
 template <bool W>
-__global__ void k_bfs_bottom_up(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
+__global__ void __launch_bounds__(TPB) k_bfs_bottom_up(DevGraph g, uint32_t *fout, unsigned long long *fout_n) {
   if (g.ctl[C_MODE] != M_BOTTOM_UP) return;
-  unsigned long long local = 0, scanned = 0;
+  __shared__ uint32_t s_q[TPB / 32][PQ_CAP];
+  __shared__ BlockCounts s_bc;
+  if (threadIdx.x == 0) s_bc = BlockCounts{0, 0};
+  __syncthreads();
   bottom_up<W>(g, g.ctl[C_DEPTH], fout, fout_n, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
-               (uint64_t)gridDim.x * blockDim.x, local, scanned);
-  warp_add_result(local, &g.ctl[C_RESULT]);
-  warp_add_result(scanned, &g.ctl[C_EDGES]);
+               (uint64_t)gridDim.x * blockDim.x, s_q[threadIdx.x >> 5], &s_bc);
+  counts_out(g, &s_bc);
 }
 
 // ---- small frontiers: several levels in one CTA -----------------------------
@@ -2706,9 +2855,12 @@ __global__ void __launch_bounds__(FS_TPB)
 // graph-driven loop: the engine waits until every SM has room, which other
 // instances' epochs delay.
 constexpr int ENG_TPB = 1024;
-constexpr uint32_t ENG_STAGE = 1024;
+constexpr uint32_t ENG_STAGE = 2048;
 constexpr int ENG_MAX_CTAS = 256;
-constexpr uint32_t ENG_TINY = 4096;          // out-slots that CTA 0 relaxes alone
+constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alone (4096 took 20 us a level, the grid 9)
+// a build's push level pulls instead when its out-slots are at least 1 / 12 of the copy's
+// entries (RMAT-22 SSWP: the push of 97K vertices took 241 us, a pull level 75)
+constexpr uint64_t ENG_PULL_DIV = 12;
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
 constexpr uint32_t ENG_SPINS = 1u << 26;     // polls before a barrier gives up (tens of seconds)
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
@@ -2718,10 +2870,9 @@ struct EngineArgs {
   // sliced in-edge copy (pull levels)
   const void *ent;
   const uint64_t *off;
-  const uint32_t *row_id, *piece_v, *hub_v;
-  const uint64_t *hub_pc;
+  const uint32_t *row_id;
+  PullHubs hubs;
   const SellPlan *plan;
-  ulonglong2 *piece_best;
   // queues and scratch
   uint32_t *q[2], *tree;
   uint64_t *P;                  // frontier degree prefix, per CTA piece
@@ -2775,20 +2926,27 @@ __device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b) {
   return s_ok != 0;
 }
 
-union EngShared {
-  struct {
-    uint64_t pref[ENG_STAGE + 1];  // first slot of each staged vertex, relative to the CTA's share
-    uint64_t base[ENG_STAGE];      // pool slot minus level slot
-    uint32_t u[ENG_STAGE], su[ENG_STAGE];
-    uint64_t tot[ENG_MAX_CTAS + 1];
-  } p;
+struct EngStage {
+  uint64_t pref[ENG_STAGE + 1];  // first level slot of each staged vertex
+  uint64_t base[ENG_STAGE];      // pool slot minus level slot
+  uint32_t u[ENG_STAGE], su[ENG_STAGE];
+  uint64_t tot[ENG_MAX_CTAS + 1];
+};
+struct EngShared {
+  EngStage p;
   uint32_t q[ENG_TPB / 32][PQ_CAP];
+  BlockCounts bc;
+  // the kernel's parameters: the level kinds are calls and take them by
+  // reference, and a reference into parameter space is read through L1, which
+  // every barrier empties
+  DevGraph g;
+  EngineArgs a;
 };
 
 // Relax level slots [e0, e1) over the staged vertices (pref ascending; the
 // slots of vertex j start at pref[j]).  All threads of the CTA.
 template <int A, bool W>
-__device__ __noinline__ void eng_relax(const DevGraph &g, const EngShared &sh, uint32_t m, uint64_t e0, uint64_t e1,
+__device__ __noinline__ void eng_relax(const DevGraph &g, EngShared &sh, uint32_t m, uint64_t e0, uint64_t e1,
                                        uint32_t st, uint32_t *fout, unsigned long long *fout_n, uint32_t mst) {
   unsigned long long local = 0;
   using P_ = PoolT<W>;
@@ -2820,7 +2978,7 @@ __device__ __noinline__ void eng_relax(const DevGraph &g, const EngShared &sh, u
     }
     relax_batch<A, ENG_ITEMS>(g, on, uu, vv, ww, su, st, fout, fout_n, local, mst);
   }
-  warp_add_result(local, &g.ctl[C_RESULT]);
+  block_count(&sh.bc, local, 0);
 }
 
 // CTA r's share of S level slots.
@@ -2908,31 +3066,26 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
 // (inlined into one function they spilled over a kilobyte per thread).
 template <int A, bool W>
 __device__ __noinline__ void eng_pull(const DevGraph &g, const EngineArgs &a, EngShared &sh, int what, uint32_t m,
-                                      unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n) {
-  unsigned long long local = 0, scanned = 0;
-  pull_part<A, W>(g, reinterpret_cast<const typename SellE<W>::E *>(a.ent), a.off, a.row_id, a.piece_v, a.plan, what, 0,
-                  0, 0, m, bout, a.piece_best, sh.q[threadIdx.x >> 5], fout, fout_n, a.mst, local, scanned,
+                                      bool first, unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n) {
+  pull_part<A, W>(g, reinterpret_cast<const typename SellE<W>::E *>(a.ent), a.off, a.row_id, a.hubs, a.plan, what, 0,
+                  0, 0, m, bout, sh.q[threadIdx.x >> 5], fout, fout_n, a.mst, &sh.bc, first,
                   (blockIdx.x * ENG_TPB + threadIdx.x) >> 5, (gridDim.x * ENG_TPB) >> 5);
-  warp_add_result(local, &g.ctl[C_RESULT]);
-  warp_add_result(scanned, &g.ctl[C_EDGES]);
 }
 
 template <int A>
-__device__ __noinline__ void eng_hub_fix(const DevGraph &g, const EngineArgs &a, unsigned long long *bout,
-                                         uint32_t *fout, unsigned long long *fout_n) {
+__device__ __noinline__ void eng_hub_fix(const DevGraph &g, const EngineArgs &a, EngShared &sh,
+                                         unsigned long long *bout, uint32_t *fout, unsigned long long *fout_n) {
   unsigned long long local = 0;
-  pull_hub_fix<A>(g, a.hub_v, a.hub_pc, a.plan, a.piece_best, bout, fout, fout_n, a.mst, local,
-                  (blockIdx.x * ENG_TPB + threadIdx.x) >> 5, (gridDim.x * ENG_TPB) >> 5);
-  warp_add_result(local, &g.ctl[C_RESULT]);
+  pull_hub_fix<A>(g, a.hubs, a.plan, bout, fout, fout_n, a.mst, local, blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x,
+                  (uint64_t)gridDim.x * ENG_TPB);
+  block_count(&sh.bc, local, 0);
 }
 
 template <bool W>
-__device__ __noinline__ void eng_bottom_up(const DevGraph &g, uint64_t d, uint32_t *fout, unsigned long long *fout_n) {
-  unsigned long long local = 0, scanned = 0;
-  bottom_up<W>(g, d, fout, fout_n, blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB, local,
-               scanned);
-  warp_add_result(local, &g.ctl[C_RESULT]);
-  warp_add_result(scanned, &g.ctl[C_EDGES]);
+__device__ __noinline__ void eng_bottom_up(const DevGraph &g, EngShared &sh, uint64_t d, uint32_t *fout,
+                                           unsigned long long *fout_n) {
+  bottom_up<W>(g, d, fout, fout_n, blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB,
+               sh.q[threadIdx.x >> 5], &sh.bc);
 }
 
 template <int A, bool W>
@@ -2944,22 +3097,34 @@ __device__ __noinline__ void eng_tiny(const DevGraph &g, const EngineArgs &a, ui
 
 using EngScan = cub::BlockScan<uint64_t, ENG_TPB>;
 
-// Stages a frontier of at most ENG_STAGE vertices and returns its out-slots.
+// Stages a frontier of at most ENG_STAGE vertices (two a thread) and returns its
+// out-slots.
 __device__ __noinline__ uint64_t eng_stage(const DevGraph &g, EngShared &sh, EngScan::TempStorage &tmp,
                                            const uint32_t *fin, uint32_t n) {
-  const unsigned tid = threadIdx.x;
-  uint64_t d = 0, excl, S;
-  if (tid < n) {
-    const uint32_t u = fin[tid];
-    d = seg_len(g.out, u);
-    sh.p.u[tid] = u;
-    sh.p.base[tid] = g.out.off[u];
-    sh.p.su[tid] = (uint32_t)ld_v32(g.val32, u);
+  static_assert(ENG_STAGE == 2 * ENG_TPB, "two vertices per thread");
+  const unsigned i = 2 * threadIdx.x;
+  uint64_t d[2] = {0, 0}, excl, S;
+  uint32_t u[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    if (i + k < n) u[k] = fin[i + k];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (i + k < n) {
+      d[k] = seg_len(g.out, u[k]);
+      sh.p.u[i + k] = u[k];
+      sh.p.base[i + k] = g.out.off[u[k]];
+      sh.p.su[i + k] = (uint32_t)ld_v32(g.val32, u[k]);
+    }
   }
-  EngScan(tmp).ExclusiveSum(d, excl, S);
-  if (tid < n) {
-    sh.p.pref[tid] = excl;
-    sh.p.base[tid] -= excl;
+  EngScan(tmp).ExclusiveSum(d[0] + d[1], excl, S);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (i + k < n) {
+      sh.p.pref[i + k] = excl;
+      sh.p.base[i + k] -= excl;
+    }
+    excl += d[k];
   }
   __syncthreads();
   return S;
@@ -3035,11 +3200,19 @@ __device__ __noinline__ uint32_t eng_stage_from(const DevGraph &g, const EngineA
 }
 
 template <int A, bool W>
-__global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ DevGraph g,
-                                                       const __grid_constant__ EngineArgs a) {
+__global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ DevGraph g_arg,
+                                                       const __grid_constant__ EngineArgs a_arg) {
   __shared__ EngScan::TempStorage scan_tmp;
   extern __shared__ __align__(16) unsigned char eng_smem[];
   EngShared &sh = *reinterpret_cast<EngShared *>(eng_smem);
+  if (threadIdx.x == 0) {
+    sh.g = g_arg;
+    sh.a = a_arg;
+    sh.bc = BlockCounts{0, 0};
+  }
+  __syncthreads();
+  const DevGraph &g = sh.g;
+  const EngineArgs &a = sh.a;
   unsigned long long *c = g.ctl;
   unsigned long long *bnd = a.bar + EB_BND;
   auto cnt = [&](uint32_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
@@ -3084,24 +3257,15 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       }
       c[C_LEVEL] = lvl + 1;
     }
-    // the mode rules of k_level_begin
+    // the mode rules of k_level_begin, and a pull in place of a push that
+    // would relax a large part of the graph
     const bool bu = a.cfg.bottom_up && n * a.cfg.bu_div >= g.V;
-    const bool pull = !bu && a.cfg.allow_pull && n * (pulled ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
+    bool pull = !bu && a.cfg.allow_pull && n * (pulled ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
     if (bu) {
-      eng_bottom_up<W>(g, lvl, fout, fout_n);
-    } else if (pull) {
-      const uint32_t m = pulled ? (uint32_t)__ldcg(&bnd[k % 3]) : a.cfg.bnd_best;
-      unsigned long long *bout = &bnd[(k + 1) % 3];
-      eng_pull<A, W>(g, a, sh, a.cfg.pull_split ? PART_HUBS : PART_ALL, m, bout, fout, fout_n);
-      if (!grid_sync(g, bar)) return;
-      eng_hub_fix<A>(g, a, bout, fout, fout_n);
-      if (a.cfg.pull_split) {
-        if (!grid_sync(g, bar)) return;
-        eng_pull<A, W>(g, a, sh, PART_REST, m, bout, fout, fout_n);
-      }
-    } else if (n <= ENG_STAGE) {
+      eng_bottom_up<W>(g, sh, lvl, fout, fout_n);
+    } else if (!pull && n <= ENG_STAGE) {
       const uint64_t S = eng_stage(g, sh, scan_tmp, fin, (uint32_t)n);
-      if (S <= a.cfg.tiny_edges && S <= ENG_TINY) {
+      if (n <= TINY_N && S <= a.cfg.tiny_edges && S <= ENG_TINY) {
         if (!grid_sync(g, bar)) return;  // (every CTA has read the counts that CTA 0 now uses by turns)
         unsigned long long *at = a.bar + EB_LVL + 2 * (k & 1);  // where CTA 0 got to
         if (blockIdx.x == 0) {
@@ -3121,15 +3285,16 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       uint64_t e0, e1;
       eng_share(S, e0, e1);
       eng_relax<A, W>(g, sh, (uint32_t)n, e0, e1, st, fout, fout_n, a.mst);
-      if (lead) atomicAdd(&c[C_EDGES], (unsigned long long)S);
-    } else {
+      if (lead) atomicAdd(&sh.bc.scanned, (unsigned long long)S);
+    } else if (!pull) {
       const uint32_t per = (uint32_t)((n + gridDim.x - 1) / gridDim.x);
       eng_prefix(g, a, scan_tmp, fin, (uint32_t)n, per);
       if (!grid_sync(g, bar)) return;
       uint64_t e0, e1;
       uint32_t i;
       const uint64_t S = eng_first(a, sh, scan_tmp, (uint32_t)n, per, e0, e1, i);
-      for (uint64_t e = e0; e < e1;) {
+      pull = a.cfg.allow_pull && S * ENG_PULL_DIV >= a.plan->total;
+      for (uint64_t e = e0; e < e1 && !pull;) {
         const uint32_t m = eng_stage_from(g, a, sh, fin, (uint32_t)n, per, i, S);
         const uint64_t end = min(e1, sh.p.pref[m]);
         eng_relax<A, W>(g, sh, m, e, end, st, fout, fout_n, a.mst);
@@ -3137,13 +3302,25 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
         e = end;
         i += m;
       }
-      if (lead) atomicAdd(&c[C_EDGES], (unsigned long long)S);
+      if (lead && !pull) atomicAdd(&sh.bc.scanned, (unsigned long long)S);
+    }
+    if (pull) {
+      const uint32_t m = pulled ? (uint32_t)__ldcg(&bnd[k % 3]) : a.cfg.bnd_best;
+      unsigned long long *bout = &bnd[(k + 1) % 3];
+      eng_pull<A, W>(g, a, sh, a.cfg.pull_split ? PART_HUBS : PART_ALL, m, lvl == 0, bout, fout, fout_n);
+      if (!grid_sync(g, bar)) return;
+      eng_hub_fix<A>(g, a, sh, bout, fout, fout_n);
+      if (a.cfg.pull_split) {
+        if (!grid_sync(g, bar)) return;
+        eng_pull<A, W>(g, a, sh, PART_REST, m, lvl == 0, bout, fout, fout_n);
+      }
     }
     pulled = pull;
     lvl++;
     if (!grid_sync(g, bar)) return;
   }
-  if (!grid_sync(g, bar)) return;  // (every CTA has read the last counts)
+  counts_out(g, &sh.bc);
+  if (!grid_sync(g, bar)) return;  // (every CTA has read the last queue counts)
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
       c[C_QN0] = 0;
@@ -3231,17 +3408,18 @@ int guard_counters(Graph &g) {
   return RG_OK;
 }
 
-template <int K>
+template <bool W, int K>
 int sell_fill_sorted(Graph &g, uint64_t s_lo, uint64_t s_hi, const uint32_t *pv, const uint32_t *pst,
                      const uint32_t *pln) {
   if (s_lo >= s_hi) return RG_OK;
-  const size_t smem = sell_fill_smem(K);
-  RG_CUDA(cudaFuncSetAttribute(k_sell_fill_sorted<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  using E = typename SellE<W>::E;
+  const size_t smem = sell_fill_smem(K, sizeof(E));
+  RG_CUDA(cudaFuncSetAttribute(k_sell_fill_sorted<W, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   count_launch(g);
   const uint64_t blocks = std::min<uint64_t>(s_hi - s_lo, (uint64_t)g.num_sms * 8);
-  k_sell_fill_sorted<K><<<(unsigned)blocks, SF_TPB, smem, g.stream>>>(g.d, g.sell_row, g.sell_plan_host->rows, s_lo, s_hi,
+  k_sell_fill_sorted<W, K><<<(unsigned)blocks, SF_TPB, smem, g.stream>>>(g.d, g.sell_row, g.sell_plan_host->rows, s_lo, s_hi,
                                                                       g.sell_off, pv, pst, pln,
-                                                                      reinterpret_cast<uint2 *>(g.sell_ent));
+                                                                      reinterpret_cast<E *>(g.sell_ent));
   RG_CUDA(cudaGetLastError());
   return RG_OK;
 }
@@ -3275,8 +3453,8 @@ int prepare_pull_w(Graph &g) {
   // the hub arrays are sized for every vertex once, so their addresses stay
   // fixed for the cached level-loop graph
   if ((rc = grow((void **)&g.sell_hub, g.sell_hub_cap, V + 1, 4))) return rc;
-  if (!g.sell_hub_off) {
-    if (cudaMalloc(&g.sell_hub_off, g.sell_hub_cap * 8) != cudaSuccess) {
+  if (!g.sell_hub_best) {
+    if (cudaMalloc(&g.sell_hub_best, g.sell_hub_cap * 8) != cudaSuccess) {
       cudaGetLastError();
       set_error("device allocation failed: pull preparation");
       return RG_ENOMEM_HBM;
@@ -3285,33 +3463,36 @@ int prepare_pull_w(Graph &g) {
   }
   RG_CUDA(cudaMemsetAsync(g.sell_plan, 0, sizeof(SellPlan), g.stream));
   count_launch(g, 2);
-  k_sell_count<<<g.num_sms * 2, 1024, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan);
-  k_sell_plan<<<1, 1024, 0, g.stream>>>(g.sell_plan);
+  k_sell_count<<<g.num_sms * 2, 1024, 0, g.stream>>>(g.d, g.sell_hub, reinterpret_cast<uint64_t *>(g.sell_hub_best),
+                                                      g.sell_plan);
+  k_sell_plan<<<1, SP_TPB, 0, g.stream>>>(g.sell_plan);
   RG_CUDA(cudaMemcpyAsync(g.sell_plan_host, g.sell_plan, sizeof(SellPlan), cudaMemcpyDeviceToHost, g.stream));
   RG_CUDA(cudaStreamSynchronize(g.stream));
   const SellPlan &plan = *g.sell_plan_host;
   const uint64_t P = plan.pieces;
-  if ((rc = grow((void **)&g.sell_piece, g.sell_piece_cap, 3 * (P + 1), 4))) return rc;
+  if ((rc = grow((void **)&g.sell_piece, g.sell_piece_cap, 4 * (P + 1), 4))) return rc;
   if ((rc = grow((void **)&g.sell_piece_best, g.sell_best_cap, P + 1, 16))) return rc;
-  if ((rc = grow((void **)&g.sell_row, g.sell_row_cap, V + P, 4))) return rc;
+  if ((rc = grow((void **)&g.sell_row, g.sell_row_cap, V + P + 32, 4))) return rc;
   if ((rc = grow((void **)&g.sell_off, g.sell_off_cap, plan.slices + 1, 8))) return rc;
   if ((rc = grow(&g.sell_ent, g.sell_cap, plan.total, W ? 8 : 4))) return rc;
-  uint32_t *pv = g.sell_piece, *pst = pv + (P + 1), *pln = pst + (P + 1);
+  // (the parts of the piece table lie by its capacity: the cached loop graphs hold their addresses)
+  const uint64_t pcap = g.sell_piece_cap / 4;
+  uint32_t *pv = g.sell_piece, *pst = pv + pcap, *pln = pst + pcap;
   count_launch(g);
-  k_sell_rows<<<g.num_sms * 4, SR_TPB, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan, g.sell_row, pv, pst,
-                                                      pln, g.sell_off);
+  k_sell_rows<<<g.num_sms * 4, SR_TPB, 0, g.stream>>>(g.d, g.sell_hub, g.sell_hub_best, g.sell_plan, g.sell_row, pv, pst,
+                                                      pln, pln + pcap, g.sell_off);
   RG_CUDA(cudaGetLastError());
-  uint64_t plain_lo = 0;
-  if constexpr (W) {
-    // the rows that a pull reads in pieces, by weight; K = ceil(width / 32)
-    const uint32_t *sl = plan.slice;
-    if ((rc = sell_fill_sorted<18>(g, 0, sl[256], pv, pst, pln))) return rc;
-    if ((rc = sell_fill_sorted<8>(g, sl[256], sl[128], pv, pst, pln))) return rc;
-    if ((rc = sell_fill_sorted<4>(g, sl[128], sl[64], pv, pst, pln))) return rc;
-    if ((rc = sell_fill_sorted<2>(g, sl[64], sl[32], pv, pst, pln))) return rc;
-    if ((rc = sell_fill_sorted<1>(g, sl[32], sl[8], pv, pst, pln))) return rc;
-    plain_lo = sl[8];
-  }
+  // the rows that a pull reads in parts, in order; K = ceil(width / 32)
+  constexpr int KP = ((int)PULL_PIECE + 31) / 32, KV = ((int)PULL_HUB + 31) / 32;
+  static_assert(KV > 8 && PULL_HUB > 256, "K of the fills below");
+  const uint32_t *sl = plan.slice;
+  if ((rc = sell_fill_sorted<W, KP>(g, 0, sl[PULL_HUB], pv, pst, pln))) return rc;
+  if ((rc = sell_fill_sorted<W, KV>(g, sl[PULL_HUB], sl[256], pv, pst, pln))) return rc;
+  if ((rc = sell_fill_sorted<W, 8>(g, sl[256], sl[128], pv, pst, pln))) return rc;
+  if ((rc = sell_fill_sorted<W, 4>(g, sl[128], sl[64], pv, pst, pln))) return rc;
+  if ((rc = sell_fill_sorted<W, 2>(g, sl[64], sl[32], pv, pst, pln))) return rc;
+  if ((rc = sell_fill_sorted<W, 1>(g, sl[32], sl[8], pv, pst, pln))) return rc;
+  const uint64_t plain_lo = sl[8];
   if (plain_lo < plan.slices) {
     count_launch(g);
     k_sell_fill<W><<<g.num_sms * 16, TPB, 0, g.stream>>>(g.d, g.sell_row, plan.rows, plain_lo, plan.slices,
@@ -3337,17 +3518,21 @@ int prepare_pull(Graph &g) {
   return g.weighted ? prepare_pull_w<true>(g) : prepare_pull_w<false>(g);
 }
 
+PullHubs pull_hubs(const Graph &g) {
+  return PullHubs{g.sell_piece, g.sell_piece + 3 * (g.sell_piece_cap / 4), g.sell_hub, g.sell_piece_best, g.sell_hub_best};
+}
+
 // First entry of slice s (or the entries in all).
 uint64_t sell_offset(const Graph &g, uint64_t s) {
   const SellPlan &p = *g.sell_plan_host;
   if (s >= p.slices) return p.total;
-  int lo = 1, hi = (int)PULL_HUB;  // the narrowest width L with slice[L] <= s
+  int lo = 1, hi = SELL_KEYS - 1;  // the smallest key k with slice[k] <= s
   while (lo < hi) {
     const int mid = (lo + hi) / 2;
     if (p.slice[mid] <= s) hi = mid;
     else lo = mid + 1;
   }
-  return p.base[lo] + (s - p.slice[lo]) * 32 * lo;
+  return p.base[lo] + (s - p.slice[lo]) * 32 * sell_width(lo);
 }
 
 // Slice bounds of the launches that follow the hub launch of a split pull
@@ -3397,19 +3582,17 @@ int enqueue_mode(Graph &g, cudaStream_t s, int half, unsigned long long mode) {
       const unsigned long long *bin = &g.d.ctl[C_BND0 + half];
       unsigned long long *bout = &g.d.ctl[C_BND0 + (half ^ 1)];
       auto pull = [&](int part, uint32_t lo, uint32_t hi, int rest) {
-        k_pull_sell<A, W><<<g.num_sms * 8, PS_TPB, 0, s>>>(g.d, ent, g.sell_off, g.sell_row, g.sell_piece, g.sell_plan,
-                                                           part, lo, hi, rest, bin, bout, g.sell_piece_best, fout,
-                                                           fout_n, mst);
+        k_pull_sell<A, W><<<g.num_sms * 8, PS_TPB, 0, s>>>(g.d, ent, g.sell_off, g.sell_row, pull_hubs(g), g.sell_plan,
+                                                           part, lo, hi, rest, bin, bout, fout, fout_n, mst);
       };
       pull(split ? PART_HUBS : PART_ALL, 0, 0, 0);
-      k_pull_hub_fix<A><<<g.num_sms * 2, 256, 0, s>>>(g.d, g.sell_hub, g.sell_hub_off, g.sell_plan, g.sell_piece_best,
-                                                      bout, fout, fout_n, mst);
+      k_pull_hub_fix<A><<<g.num_sms * 2, 256, 0, s>>>(g.d, pull_hubs(g), g.sell_plan, bout, fout, fout_n, mst);
       if (!split || g.pull_groups <= 2) {
         pull(split ? PART_REST : PART_NONE, 0, 0, 0);
       } else {
         // the other rows, in widest-first groups of equal entries: each group
         // reads the values the groups before it set in this level
-        const std::vector<uint64_t> b = pull_group_bounds(g, g.sell_plan_host->slice[PULL_SPLIT - 1],
+        const std::vector<uint64_t> b = pull_group_bounds(g, g.sell_plan_host->slice[PULL_HUB],
                                                           g.sell_plan_host->slice[4], g.pull_groups);
         for (size_t i = 0; i + 1 < b.size(); i++) pull(PART_RANGE, (uint32_t)b[i], (uint32_t)b[i + 1], i + 2 == b.size() ? 1 : 0);
       }
@@ -3846,11 +4029,8 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
     a.ent = g.sell_ent;
     a.off = g.sell_off;
     a.row_id = g.sell_row;
-    a.piece_v = g.sell_piece;
-    a.hub_v = g.sell_hub;
-    a.hub_pc = g.sell_hub_off;
+    a.hubs = pull_hubs(g);
     a.plan = g.sell_plan;
-    a.piece_best = g.sell_piece_best;
   }
   a.q[0] = g.q[0];
   a.q[1] = g.q[1];
