@@ -1490,7 +1490,7 @@ __device__ __forceinline__ void tiny_levels(const DevGraph &g, uint32_t *q_in, u
   unsigned long long *cur_n = n_in, *nxt_n = n_out;
   unsigned long long local = 0, scanned = 0;
   for (bool first = true;; first = false) {
-    const uint64_t n = *cur_n;
+    const uint64_t n = __ldcg(cur_n);
     // stage the frontier and its degree prefix
     uint32_t d = 0;
     if (n <= TINY_N && tid < n) {
@@ -1556,7 +1556,7 @@ __device__ __forceinline__ void tiny_levels(const DevGraph &g, uint32_t *q_in, u
     nxt_n = tn;
   }
   if (cur != q_final) {
-    const uint64_t n = *cur_n;
+    const uint64_t n = __ldcg(cur_n);
     for (uint64_t i = tid; i < n; i += TINY_TPB) q_final[i] = cur[i];
     __syncthreads();
     if (tid == 0) *n_final = n;
@@ -2066,6 +2066,61 @@ __device__ __forceinline__ bool queue_heavy(uint32_t *hv, unsigned long long *hv
   return false;
 }
 
+// Rescue of one invalidated vertex d (value sd, in-list [off, off + len)) by a
+// warp.
+template <int A, bool W>
+__device__ __forceinline__ void rescue_one(const DevGraph &g, uint32_t d, uint64_t sd, uint32_t len, uint64_t off,
+                                           uint32_t tag_inv, uint64_t limit) {
+  using P = PoolT<W>;
+  const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
+  const int lane = lane_id();
+  for (uint32_t kb = 0; kb < len; kb += 32) {
+    const uint32_t k = kb + lane;
+    bool ok = false;
+    uint32_t src = 0, w = 0;
+    if (k < len) {
+      typename P::E e = pool[off + k];
+      src = P::nbr(e);
+      w = P::wt(e);
+      if (!(src & DEAD) && Hook<A>::combine(ld_v32(g.val32, src), w) == sd) ok = !has_parents(g, src, tag_inv, limit);
+    }
+    unsigned b = __ballot_sync(FULL, ok);
+    bool done = false;
+    while (b) {
+      int l = __ffs(b) - 1;
+      b &= b - 1;
+      bool won = false;
+      if (lane == l) {
+        won = atomicCAS(&g.inv[d], tag_inv, tag_inv + 1) == tag_inv;
+        if (won) reinterpret_cast<unsigned long long *>(&g.lab[d])[1] = pack_parent(src, w);
+      }
+      won = __shfl_sync(FULL, won, l);
+      if (won) { done = true; break; }
+    }
+    if (done || __shfl_sync(FULL, ld_u32(&g.inv[d]), 0) != tag_inv) break;
+  }
+}
+
+// The passes of the deletion repair over more vertices than there are warps
+// take four vertices to a warp, eight lanes each: most lists are a few entries,
+// and a pass is chains of dependent loads, not bandwidth.  (One vertex to a
+// warp, the rescue of 517 vertices in the one-CTA repair took 16 rounds, 125 us; a
+// batch of 1,000 undirected updates with it 310 us, now 205.)
+// Lists longer than REP_LONG get the whole warp, one after the other.
+constexpr uint32_t REP_GS = 8, REP_NG = 32 / REP_GS, REP_LONG = 64;
+
+// Whether this group's vertex went to the heavy queue.
+__device__ __forceinline__ bool queue_heavy_group(bool want, uint32_t *hv, unsigned long long *hv_n, uint64_t hv_cap,
+                                                  uint32_t v) {
+  bool in = false;
+  if (want && lane_id() % REP_GS == 0) {
+    const unsigned long long k = atomicAdd(hv_n, 1ull);
+    in = k < hv_cap;
+    if (in) hv[k] = v;
+  }
+  return __shfl_sync(FULL, in, lane_id() & ~(REP_GS - 1));
+}
+
 template <int A, bool W>
 __device__ __forceinline__ void rescue_warps(const DevGraph &g, const uint32_t *fin, uint64_t n, uint64_t limit,
                                              uint64_t warp, uint64_t nwarps, uint32_t *hv = nullptr,
@@ -2074,39 +2129,63 @@ __device__ __forceinline__ void rescue_warps(const DevGraph &g, const uint32_t *
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
-  for (uint64_t idx = warp; idx < n; idx += nwarps) {
-    const uint32_t d = fin[idx];
-    // (the vertex's words in one round trip)
-    const uint32_t td = ld_u32(&g.inv[d]);
-    const uint64_t sd = ld_v32(g.val32, d);
-    const uint32_t len = seg_len(g.in, d);
-    const uint64_t off = g.in.off[d];
-    if (td != tag_inv) continue;
-    if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
-    for (uint32_t kb = 0; kb < len; kb += 32) {
-      const uint32_t k = kb + lane;
+  if (n <= nwarps) {
+    for (uint64_t idx = warp; idx < n; idx += nwarps) {
+      const uint32_t d = fin[idx];
+      // (the vertex's words in one round trip)
+      const uint32_t td = ld_u32(&g.inv[d]);
+      const uint64_t sd = ld_v32(g.val32, d);
+      const uint32_t len = seg_len(g.in, d);
+      const uint64_t off = g.in.off[d];
+      if (td != tag_inv) continue;
+      if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
+      rescue_one<A, W>(g, d, sd, len, off, tag_inv, limit);
+    }
+    return;
+  }
+  const uint32_t sub = lane % REP_GS, gsh = lane & ~(REP_GS - 1);
+  for (uint64_t base = warp * REP_NG; base < n; base += nwarps * REP_NG) {
+    const uint64_t idx = base + lane / REP_GS;
+    uint32_t d = 0, len = 0;
+    uint64_t sd = 0, off = 0;
+    bool act = false;
+    if (idx < n) {
+      d = fin[idx];
+      const uint32_t td = ld_u32(&g.inv[d]);
+      sd = ld_v32(g.val32, d);
+      len = seg_len(g.in, d);
+      off = g.in.off[d];
+      act = td == tag_inv;
+    }
+    if (hv) {
+      const bool queued = queue_heavy_group(act && len > HEAVY_DEG, hv, hv_n, hv_cap, d);
+      act = act && !queued;
+    }
+    const unsigned lng = __ballot_sync(FULL, act && len > REP_LONG && sub == 0);
+    bool open = act && len <= REP_LONG;
+    for (uint32_t kb = 0; __any_sync(FULL, open && kb < len); kb += REP_GS) {
+      const uint32_t k = kb + sub;
       bool ok = false;
       uint32_t src = 0, w = 0;
-      if (k < len) {
+      if (open && k < len) {
         typename P::E e = pool[off + k];
         src = P::nbr(e);
         w = P::wt(e);
-        if (!(src & DEAD) && Hook<A>::combine(ld_v32(g.val32, src), w) == sd) ok = !has_parents(g, src, tag_inv, limit);
+        if (!(src & DEAD) && Hook<A>::combine(ld_v32(g.val32, src), w) == sd)
+          ok = !has_parents(g, src, tag_inv, limit);
       }
-      unsigned b = __ballot_sync(FULL, ok);
-      bool done = false;
-      while (b) {
-        int l = __ffs(b) - 1;
-        b &= b - 1;
-        bool won = false;
-        if (lane == l) {
-          won = atomicCAS(&g.inv[d], tag_inv, tag_inv + 1) == tag_inv;
-          if (won) reinterpret_cast<unsigned long long *>(&g.lab[d])[1] = pack_parent(src, w);
-        }
-        won = __shfl_sync(FULL, won, l);
-        if (won) { done = true; break; }
+      const unsigned gb = (__ballot_sync(FULL, ok) >> gsh) & ((1u << REP_GS) - 1);
+      if (gb) {  // the group's first candidate
+        if (sub == (uint32_t)__ffs(gb) - 1 && atomicCAS(&g.inv[d], tag_inv, tag_inv + 1) == tag_inv)
+          reinterpret_cast<unsigned long long *>(&g.lab[d])[1] = pack_parent(src, w);
+        open = false;
       }
-      if (done || __shfl_sync(FULL, ld_u32(&g.inv[d]), 0) != tag_inv) break;
+    }
+    for (unsigned m = lng; m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const uint32_t d1 = __shfl_sync(FULL, d, l), len1 = __shfl_sync(FULL, len, l);
+      const uint64_t sd1 = __shfl_sync(FULL, sd, l), off1 = __shfl_sync(FULL, off, l);
+      rescue_one<A, W>(g, d1, sd1, len1, off1, tag_inv, limit);
     }
   }
 }
@@ -2166,44 +2245,95 @@ __global__ void __launch_bounds__(TPB) k_rescue_heavy(DevGraph g, uint64_t limit
 
 // Collect and expand (core/graph.hpp:1363-1417): a still-invalid vertex joins
 // the reset set; its tree children (parent == (u,w)) are invalidated next.
+// The tree children of u among N slots a lane holds, invalidated and appended
+// (all lanes of the warp).
+template <bool W, int N>
+__device__ __forceinline__ void expand_slots(const DevGraph &g, uint32_t u, uint64_t off, uint32_t k0, uint32_t step,
+                                             uint32_t len, uint32_t tag_inv, uint32_t *fout,
+                                             unsigned long long *fout_n) {
+  using P = PoolT<W>;
+  const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.out.pool);
+  typename P::E e[N];
+  uint64_t meta[N];
+  uint32_t t[N];
+#pragma unroll
+  for (int i = 0; i < N; i++)
+    if (k0 + i * step < len) e[i] = pool[off + k0 + i * step];
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const bool on = k0 + i * step < len && !(P::nbr(e[i]) & DEAD);
+    meta[i] = on ? ld_meta(&g.lab[P::nbr(e[i])]) : ~0ull;
+    t[i] = on ? ld_u32(&g.inv[P::nbr(e[i])]) : tag_inv;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    bool app = false;
+    uint32_t v = 0;
+    if (t[i] != tag_inv && t[i] != tag_inv + 1 && meta[i] == pack_parent(u, P::wt(e[i]))) {
+      v = P::nbr(e[i]);
+      app = atomicCAS(&g.inv[v], t[i], tag_inv) == t[i];
+    }
+    warp_append(app, v, fout, fout_n, FULL);
+  }
+}
+
 template <int A, bool W>
 __device__ __forceinline__ void expand_warps(const DevGraph &g, const uint32_t *fin, uint64_t n, uint32_t *tree,
                                              uint32_t *fout, unsigned long long *fout_n, uint64_t warp,
                                              uint64_t nwarps, uint32_t *hv = nullptr,
                                              unsigned long long *hv_n = nullptr, uint64_t hv_cap = 0) {
   const uint32_t tag_inv = (uint32_t)g.ctl[C_INVTAG];
-  using P = PoolT<W>;
-  const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.out.pool);
   const int lane = lane_id();
-  for (uint64_t idx = warp; idx < n; idx += nwarps) {
-    const uint32_t u = fin[idx];
-    // (the vertex's words in one round trip; its slot in the reset set is
-    // taken here and written after the scan, off the critical path)
-    const uint32_t tu = ld_u32(&g.inv[u]);
-    const uint32_t len = seg_len(g.out, u);
-    const uint64_t off = g.out.off[u];
-    if (tu != tag_inv) continue;
-    unsigned long long slot = 0;
-    if (lane == 0) slot = atomicAdd(&g.ctl[C_TREEN], 1ull);
-    if (!(hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, u, lane))) {
-      for (uint32_t kb = 0; kb < len; kb += 32) {
-        const uint32_t k = kb + lane;
-        bool app = false;
-        uint32_t v = 0;
-        if (k < len) {
-          typename P::E e = pool[off + k];
-          v = P::nbr(e);
-          if (!(v & DEAD)) {
-            const uint64_t meta = ld_meta(&g.lab[v]);
-            const uint32_t t = ld_u32(&g.inv[v]);
-            if (meta == pack_parent(u, P::wt(e)) && t != tag_inv && t != tag_inv + 1)
-              app = atomicCAS(&g.inv[v], t, tag_inv) == t;
-          }
-        }
-        warp_append(app, v, fout, fout_n, FULL);
+  if (n <= nwarps) {
+    for (uint64_t idx = warp; idx < n; idx += nwarps) {
+      const uint32_t u = fin[idx];
+      // (the vertex's words in one round trip; its slot in the reset set is
+      // taken here and written after the scan, off the critical path)
+      const uint32_t tu = ld_u32(&g.inv[u]);
+      const uint32_t len = seg_len(g.out, u);
+      const uint64_t off = g.out.off[u];
+      if (tu != tag_inv) continue;
+      unsigned long long slot = 0;
+      if (lane == 0) slot = atomicAdd(&g.ctl[C_TREEN], 1ull);
+      if (!(hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, u, lane))) {
+        uint32_t kb = 0;
+        for (; kb + 32 < len; kb += 128) expand_slots<W, 4>(g, u, off, kb + lane, 32, len, tag_inv, fout, fout_n);
+        if (kb < len) expand_slots<W, 1>(g, u, off, kb + lane, 32, len, tag_inv, fout, fout_n);
       }
+      if (lane == 0) tree[slot] = u;
     }
-    if (lane == 0) tree[slot] = u;
+    return;
+  }
+  const uint32_t sub = lane % REP_GS;
+  for (uint64_t base = warp * REP_NG; base < n; base += nwarps * REP_NG) {
+    const uint64_t idx = base + lane / REP_GS;
+    uint32_t u = 0, len = 0;
+    uint64_t off = 0;
+    bool act = false;
+    if (idx < n) {
+      u = fin[idx];
+      const uint32_t tu = ld_u32(&g.inv[u]);
+      len = seg_len(g.out, u);
+      off = g.out.off[u];
+      act = tu == tag_inv;
+    }
+    if (!__any_sync(FULL, act)) continue;
+    warp_append(act && sub == 0, u, tree, &g.ctl[C_TREEN], FULL);
+    if (hv) {
+      const bool queued = queue_heavy_group(act && len > HEAVY_DEG, hv, hv_n, hv_cap, u);
+      act = act && !queued;
+    }
+    const unsigned lng = __ballot_sync(FULL, act && len > REP_LONG && sub == 0);
+    const uint32_t end = act && len <= REP_LONG ? len : 0u;
+    for (uint32_t kb = 0; __any_sync(FULL, kb < end); kb += 2 * REP_GS)
+      expand_slots<W, 2>(g, u, off, kb + sub, REP_GS, end, tag_inv, fout, fout_n);
+    for (unsigned m = lng; m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const uint32_t u1 = __shfl_sync(FULL, u, l), len1 = __shfl_sync(FULL, len, l);
+      const uint64_t off1 = __shfl_sync(FULL, off, l);
+      for (uint32_t kb = 0; kb < len1; kb += 128)
+        expand_slots<W, 4>(g, u1, off1, kb + lane, 32, len1, tag_inv, fout, fout_n);
+    }
   }
 }
 
@@ -2282,43 +2412,103 @@ __global__ void k_reset(DevGraph g, const uint32_t *tree, const unsigned long lo
 }
 
 // One transposed pull over the reset set (core/graph.hpp:1433-1511): each
-// vertex takes its best in-neighbour by update_func.  One warp per vertex.
+// vertex takes its best in-neighbour by update_func.
+struct PullBest {
+  uint64_t best, su;
+  uint32_t src, w;
+};
+
+// The best of the N slots a lane holds and of p.
+template <int A, bool W, int N>
+__device__ __forceinline__ void pull_slots(const DevGraph &g, uint64_t off, uint32_t k0, uint32_t step, uint32_t len,
+                                           PullBest &p) {
+  using P = PoolT<W>;
+  const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
+  typename P::E e[N];
+  uint64_t su[N];
+#pragma unroll
+  for (int i = 0; i < N; i++)
+    if (k0 + i * step < len) e[i] = pool[off + k0 + i * step];
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const bool on = k0 + i * step < len && !(P::nbr(e[i]) & DEAD);
+    su[i] = on ? ld_v32(g.val32, P::nbr(e[i])) : ~0ull;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    if (su[i] == ~0ull) continue;
+    const uint64_t nv = Hook<A>::combine(su[i], P::wt(e[i]));
+    if (Hook<A>::better(nv, p.best)) p = PullBest{nv, su[i], P::nbr(e[i]), P::wt(e[i])};
+  }
+}
+
+// The best over the `width` lanes of each group, in its first lane; relaxes the
+// vertex with it there (all lanes of the warp).
+template <int A>
+__device__ __forceinline__ bool pull_reduce(const DevGraph &g, PullBest p, uint32_t d, bool act, int width,
+                                            uint32_t mst) {
+  for (int o = width / 2; o; o >>= 1) {
+    const uint64_t ob = __shfl_down_sync(FULL, p.best, o), osu = __shfl_down_sync(FULL, p.su, o);
+    const uint32_t os = __shfl_down_sync(FULL, p.src, o), ow = __shfl_down_sync(FULL, p.w, o);
+    if (os != NONE && (p.src == NONE || Hook<A>::better(ob, p.best))) p = PullBest{ob, osu, os, ow};
+  }
+  const bool upd = act && lane_id() % width == 0 && p.src != NONE && relax<A>(g, p.src, p.su, d, p.w);
+  __syncwarp();
+  if (mst) mark_modified(g, upd, d, mst);
+  return upd;
+}
+
 template <int A, bool W>
 __device__ __forceinline__ unsigned long long pull_warps(const DevGraph &g, const uint32_t *fin, uint64_t n,
                                                          uint32_t mst, uint64_t warp, uint64_t nwarps,
                                                          uint32_t *hv = nullptr, unsigned long long *hv_n = nullptr,
                                                          uint64_t hv_cap = 0) {
-  using P = PoolT<W>;
-  const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
   unsigned long long local = 0;
-  for (uint64_t idx = warp; idx < n; idx += nwarps) {
-    const uint32_t d = fin[idx];
-    const uint32_t len = seg_len(g.in, d);
-    const uint64_t off = g.in.off[d];
-    if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
-    uint64_t best = ld_v32(g.val32, d), bsu = 0;
-    uint32_t bsrc = NONE, bw = 0;
-    for (uint32_t k = lane; k < len; k += 32) {
-      typename P::E e = pool[off + k];
-      uint32_t s = P::nbr(e);
-      if (s & DEAD) continue;
-      uint64_t su = ld_v32(g.val32, s);
-      uint64_t nv = Hook<A>::combine(su, P::wt(e));
-      if (Hook<A>::better(nv, best)) { best = nv; bsrc = s; bw = P::wt(e); bsu = su; }
+  if (n <= nwarps) {
+    for (uint64_t idx = warp; idx < n; idx += nwarps) {
+      const uint32_t d = fin[idx];
+      const uint32_t len = seg_len(g.in, d);
+      const uint64_t off = g.in.off[d];
+      if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
+      PullBest p = {ld_v32(g.val32, d), 0, NONE, 0};
+      uint32_t kb = 0;
+      for (; kb + 32 < len; kb += 128) pull_slots<A, W, 4>(g, off, kb + lane, 32, len, p);
+      if (kb < len) pull_slots<A, W, 1>(g, off, kb + lane, 32, len, p);
+      local += pull_reduce<A>(g, p, d, true, 32, mst);
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      uint64_t ob = __shfl_down_sync(FULL, best, o);
-      uint64_t osu = __shfl_down_sync(FULL, bsu, o);
-      uint32_t os = __shfl_down_sync(FULL, bsrc, o);
-      uint32_t ow = __shfl_down_sync(FULL, bw, o);
-      if (os != NONE && (bsrc == NONE || Hook<A>::better(ob, best))) { best = ob; bsu = osu; bsrc = os; bw = ow; }
+    return local;
+  }
+  const uint32_t sub = lane % REP_GS;
+  for (uint64_t base = warp * REP_NG; base < n; base += nwarps * REP_NG) {
+    const uint64_t idx = base + lane / REP_GS;
+    uint32_t d = 0, len = 0;
+    uint64_t off = 0;
+    bool act = idx < n;
+    PullBest p = {0, 0, NONE, 0};
+    if (act) {
+      d = fin[idx];
+      len = seg_len(g.in, d);
+      off = g.in.off[d];
+      p.best = ld_v32(g.val32, d);
     }
-    bool upd = false;
-    if (lane == 0 && bsrc != NONE) upd = relax<A>(g,bsrc, bsu, d, bw);
-    local += upd;
-    if (mst) mark_modified(g, __shfl_sync(FULL, upd, 0) && lane == 0, d, mst);
+    if (hv) {
+      const bool queued = queue_heavy_group(act && len > HEAVY_DEG, hv, hv_n, hv_cap, d);
+      act = act && !queued;
+    }
+    const unsigned lng = __ballot_sync(FULL, act && len > REP_LONG && sub == 0);
+    const uint32_t end = act && len <= REP_LONG ? len : 0u;
+    for (uint32_t kb = 0; __any_sync(FULL, kb < end); kb += 2 * REP_GS)
+      pull_slots<A, W, 2>(g, off, kb + sub, REP_GS, end, p);
+    local += pull_reduce<A>(g, p, d, act && end, REP_GS, mst);
+    for (unsigned m = lng; m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const uint32_t d1 = __shfl_sync(FULL, d, l), len1 = __shfl_sync(FULL, len, l);
+      const uint64_t off1 = __shfl_sync(FULL, off, l);
+      PullBest p1 = {ld_v32(g.val32, d1), 0, NONE, 0};
+      for (uint32_t kb = 0; kb < len1; kb += 128) pull_slots<A, W, 4>(g, off1, kb + lane, 32, len1, p1);
+      local += pull_reduce<A>(g, p1, d1, true, 32, mst);
+    }
   }
   return local;
 }
@@ -2399,7 +2589,7 @@ constexpr uint64_t DEL_TINY_N = 1024, DEL_TINY_TREE = 8192;
 template <int A, bool W>
 __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0, uint32_t *q1, uint32_t *tree,
                                                 uint64_t limit, uint64_t big, uint64_t max_iter, uint32_t mst) {
-  __shared__ int s_go;
+  __shared__ int s_go, s_rec;  // decisions by thread 0: every thread takes the same branch
   unsigned long long *c = g.ctl;
   const unsigned tid = threadIdx.x;
   const uint64_t warp = tid >> 5, nwarps = DT_TPB / 32;
@@ -2410,21 +2600,22 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
     // or in the reset set once the levels are done, goes to the grid-wide repair
     int heavy = 0;
     {
-      const uint64_t n0 = *cur_n;
+      const uint64_t n0 = __ldcg(cur_n);
       if (n0 && n0 <= DEL_TINY_N) {
         for (uint64_t i = tid; i < n0; i += DT_TPB)
           heavy |= seg_len(g.in, cur[i]) > HEAVY_DEG || seg_len(g.out, cur[i]) > HEAVY_DEG;
       } else if (n0 == 0) {
-        const uint64_t tn = c[C_TREEN];
+        const uint64_t tn = __ldcg(&c[C_TREEN]);
         if (tn <= DEL_TINY_TREE)
           for (uint64_t i = tid; i < tn; i += DT_TPB) heavy |= seg_len(g.in, tree[i]) > HEAVY_DEG;
       }
     }
     heavy = __syncthreads_or(heavy);
     if (tid == 0) {
-      const uint64_t n = *cur_n;
+      const uint64_t n = __ldcg(cur_n), tree_n = __ldcg(&c[C_TREEN]);
+      bool rec = __ldcg(&c[C_RECOMPUTE]) != 0;
       int go = 1;  // 1: run this level; 0: invalidation done; 2: hand over
-      if (n == 0 || c[C_RECOMPUTE]) {
+      if (n == 0 || rec) {
         go = 0;
       } else if (n > DEL_TINY_N || heavy) {
         go = 2;
@@ -2432,20 +2623,22 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
         const uint64_t it = c[C_INVITER];
         if (it >= max_iter) {
           go = 0;
-        } else if (it <= 10 && c[C_TREEN] + n > big) {  // core/graph.hpp:1252
+        } else if (it <= 10 && tree_n + n > big) {  // core/graph.hpp:1252
           c[C_RECOMPUTE] = 1;
+          rec = true;
           go = 0;
         } else {
           c[C_INVITER] = it + 1;
           *nxt_n = 0;
         }
       }
-      if (go == 0 && (c[C_TREEN] > DEL_TINY_TREE || heavy) && !c[C_RECOMPUTE]) go = 2;
+      if (go == 0 && (tree_n > DEL_TINY_TREE || heavy) && !rec) go = 2;
       s_go = go;
+      s_rec = rec;
     }
     __syncthreads();
     if (s_go != 1) break;
-    const uint64_t n = *cur_n;
+    const uint64_t n = __ldcg(cur_n);
     rescue_warps<A, W>(g, cur, n, limit, warp, nwarps);
     __syncthreads();
     expand_warps<A, W>(g, cur, n, tree, nxt, nxt_n, warp, nwarps);
@@ -2460,7 +2653,7 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
   if (s_go == 2) {
     // the multi-CTA repair continues from queue 0
     if (cur != q0) {
-      const uint64_t n = *cur_n;
+      const uint64_t n = __ldcg(cur_n);
       for (uint64_t i = tid; i < n; i += DT_TPB) q0[i] = cur[i];
       __syncthreads();
       if (tid == 0) c[C_QN0] = n;
@@ -2469,9 +2662,9 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
     return true;
   }
   unsigned long long local = 0;
-  const bool recompute = c[C_RECOMPUTE] != 0;
+  const bool recompute = s_rec != 0;
   if (!recompute) {
-    const uint64_t tn = c[C_TREEN];
+    const uint64_t tn = __ldcg(&c[C_TREEN]);
     reset_warps<A>(g, tree, tn, mst, warp, nwarps);
     __syncthreads();
     local = pull_warps<A, W>(g, tree, tn, mst, warp, nwarps);
@@ -2538,11 +2731,11 @@ struct FusedRepair {
 };
 
 // The control block to the host's mapped copy, by the whole CTA after its
-// last update (the host reads it once the stream has synchronised).
+// last update (the host reads it once the stream has synchronised, and the
+// kernel's end makes its writes visible).
 __device__ __forceinline__ void ctl_to_host(const DevGraph &g, unsigned long long *ctl_host) {
   __syncthreads();
   if (threadIdx.x < C_COUNT) ctl_host[threadIdx.x] = g.ctl[threadIdx.x];
-  __threadfence_system();
 }
 
 // A batch's header as the fused kernels read it.
@@ -2584,6 +2777,30 @@ __device__ __forceinline__ void stage_batch(const DevGraph &g, const ApplyHdr *h
   }
 }
 
+// The in-place repair of a batch whose seeds are in queue 0, by all threads of
+// the CTA after a barrier: returns 1 when work is left for the launches after
+// the kernel (C_OVER set when the deletion repair handed over), else 0.
+template <int A, bool W>
+__device__ __forceinline__ int batch_repair(const DevGraph &g, const FusedRepair &fr, int add, uint32_t *q0,
+                                            uint32_t mst, unsigned long long *tr) {
+  unsigned long long *c = g.ctl;
+  // (every thread takes the same branch: thread 0 looks)
+  auto open = [&]() { return __syncthreads_or(threadIdx.x == 0 && __ldcg(&c[C_QN0]) && !__ldcg(&c[C_ERR])) != 0; };
+  bool over = false, left = open();
+  if (left) {
+    if (!add) over = del_tiny_levels<A, W>(g, q0, fr.q1, fr.tree, fr.limit, fr.big, fr.max_iter, mst);
+    if (tr && threadIdx.x == 0) tr[RG_PH_DELREPAIR] = global_ns();
+    if (!over && fr.tiny_edges && open())
+      tiny_levels<A, W>(g, q0, &c[C_QN0], fr.q1, &c[C_QN1], q0, &c[C_QN0], fr.max_levels, fr.tiny_edges, mst, false);
+    left = open() || over;
+  }
+  if (threadIdx.x == 0) {
+    c[C_OVER] = over ? 1 : 0;
+    c[C_QN1] = 0;  // (the engine's first output count)
+  }
+  return left ? 1 : 0;
+}
+
 // One staged batch through the storage steps, the seeding and the in-place
 // repair, by all threads of the CTA after a barrier.  Returns 0 when nothing
 // is left, 1 when the repair left work for the graph nodes after the kernel
@@ -2591,7 +2808,7 @@ __device__ __forceinline__ void stage_batch(const DevGraph &g, const ApplyHdr *h
 // or when it skipped the batch.  inl: the batch's words in the kernel's
 // parameters (an inline batch), or null when they were staged into scratch.
 template <int A, bool W>
-__device__ __forceinline__ int apply_batch(const DevGraph &g, sdev::OpView ops, const StagedBatch &sb,
+__device__ __forceinline__ int apply_batch(const DevGraph &g, const sdev::OpView &ops, const StagedBatch &sb,
                                            const char *data, uint64_t *old_host, uint32_t *cand, int add, int directed,
                                            uint32_t *q0, uint32_t mst, int second, const FusedRepair &fr,
                                            uint4 *scratch, const uint64_t *inl = nullptr) {
@@ -2714,28 +2931,233 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, sdev::OpView ops, 
   }
   __syncthreads();
   stamp(RG_PH_SEED);
-  bool over = false;
-  if (c[C_QN0] && !c[C_ERR]) {
-    if (!add) over = del_tiny_levels<A, W>(g, q0, fr.q1, fr.tree, fr.limit, fr.big, fr.max_iter, mst);
-    stamp(RG_PH_DELREPAIR);
-    if (!over && fr.tiny_edges && c[C_QN0])
-      tiny_levels<A, W>(g, q0, &c[C_QN0], fr.q1, &c[C_QN1], q0, &c[C_QN0], fr.max_levels, fr.tiny_edges, mst, false);
-  }
-  const bool left = over || (c[C_QN0] && !c[C_ERR]);
-  __syncthreads();  // every thread has read the counts before the next batch resets them
+  const int left = batch_repair<A, W>(g, fr, add, q0, mst, tr);
   stamp(RG_PH_END);
-  if (tid == 0) {
-    c[C_OVER] = over ? 1 : 0;
-    c[C_QN1] = 0;  // (the engine's first output count)
+  return left;
+}
+
+// ---- inline batches without a complication -----------------------------------
+// An inline batch (at most INLINE_EDGES edges) usually meets none of the cases
+// that the phases of apply_batch exist for: no list has to grow, no two edges of
+// the submission are the same, each key is found or its slot is free within the
+// first FAST_PROBES index slots (at the index's usual load of 0.45 two leave a
+// quarter of the keys open, six 2 in a hundred).  fast_inline then has one lane per directed op (warp 0
+// the inserts, warp 1 the deletes) load everything the op can need in one round
+// trip: the index slots, the ends and offsets of both lists, the value of the
+// source and the label of the destination; a second trip loads the records of
+// edges that exist.  The rest is stores and atomics that nothing waits for.
+// apply_batch takes the same update through eight phases with barriers and one
+// or two dependent trips each, 5 to 8 us a batch (RMAT-20 SSSP, an insert and a
+// delete per call: 33 us a call through the phases, 22 with this).  Anything
+// else is decided before the first store, and the submission goes to apply_batch
+// untouched.
+constexpr int FAST_PROBES = 6;
+struct FastShared {
+  uint32_t s[32], d[32], w[32];  // the inserts' ops
+  uint32_t n_ins;
+  unsigned fall[2], improve, seeds;
+};
+enum FastResult : int { FAST_NO = -1, FAST_INS_SEEDS = 1, FAST_DEL_DONE = 2, FAST_DEL_SEEDS = 4 };
+
+// old_host: where the per-edge old counts of a single batch go, or null.
+// Returns FAST_NO (nothing done), or what was done: the insert batch's storage
+// and seeds (FAST_INS_SEEDS when queue 0 holds some; the delete batch is then
+// still to do), the delete batch's (FAST_DEL_DONE, FAST_DEL_SEEDS).
+template <int A, bool W>
+__device__ __forceinline__ int fast_inline(const DevGraph &g, const InlineBatch *ins, const InlineBatch *del,
+                                           int directed, uint64_t *old_host, uint32_t *q0, uint32_t mst) {
+  using E = typename std::conditional<W, uint2, uint32_t>::type;
+  __shared__ FastShared fs;
+  unsigned long long *c = g.ctl;
+  const unsigned tid = threadIdx.x, lane = tid & 31, lt = (1u << lane) - 1;
+  const bool is_ins = tid < 32 && ins, is_del = tid >= 32 && tid < 64 && del;
+  const InlineBatch *ib = is_ins ? ins : del;
+  bool on = false, fall = false, better_now = false;
+  uint32_t s = 0, d = 0, w = 0;
+  uint64_t n = 0;
+  if (is_ins || is_del) {
+    n = ib->n < INLINE_EDGES ? ib->n : INLINE_EDGES;
+    const uint64_t nops = directed ? n : 2 * n;
+    on = lane < nops;
+    if (is_ins && lane == 0) fs.n_ins = (uint32_t)nops;
+    if (on) {
+      const uint64_t i = directed ? lane : lane >> 1;
+      const uint64_t a = ib->words[(ib->pairs ? 2 : 3) * i], b = ib->words[(ib->pairs ? 2 : 3) * i + 1];
+      if (W) w = ib->pairs ? (uint32_t)(splitmix64((a << 32) | b) % 255 + 1) : (uint32_t)ib->words[3 * i + 2];
+      const bool flip = !directed && (lane & 1);
+      s = (uint32_t)(flip ? b : a);
+      d = (uint32_t)(flip ? a : b);
+      fall = !directed && s == d;  // (a self-loop is one op of multiplicity 2)
+    }
+    if (is_ins) {
+      fs.s[lane] = s;
+      fs.d[lane] = d;
+      fs.w[lane] = w;
+    }
   }
-  return left ? 1 : 0;
+  // 1. everything the ops can need, in one round trip
+  const ulonglong2 none = make_ulonglong2(~0ull, ~0ull);
+  const ulonglong2 key = make_ulonglong2((uint64_t)s | ((uint64_t)d << 32), (uint64_t)w);
+  const uint64_t h0 = on ? sdev::ht_hash(s, d, w) & g.ht_mask : 0;
+  ulonglong2 e[FAST_PROBES], lab = none;
+  uint32_t len_o = 0, cap_o = 0, len_i = 0, cap_i = 0, val = 0;
+  uint64_t off_o = 0, off_i = 0;
+  unsigned long long top = 0;
+  if (on) {
+#pragma unroll
+    for (int k = 0; k < FAST_PROBES; k++) e[k] = __ldcg(&g.ht[(h0 + k) & g.ht_mask]);
+    off_o = g.out.off[s];
+    cap_o = g.out.cap[s];
+    if (!g.symmetric) {
+      off_i = g.in.off[d];
+      cap_i = g.in.cap[d];
+    }
+    lab = ld_lab(&g.lab[d]);
+    if (is_ins) {
+      len_o = __ldcg(&g.out.len[s]);
+      if (!g.symmetric) len_i = __ldcg(&g.in.len[d]);
+      val = (uint32_t)ld_v32(g.val32, s);
+      top = __ldcg(g.rec_top);
+    }
+  }
+  // 2. found, free, or past the last probe
+  uint32_t rid = UNSET;
+  bool create = false, open = on;
+  uint64_t slot = h0;
+#pragma unroll
+  for (int k = 0; k < FAST_PROBES; k++) {
+    if (open && e[k].x == key.x && (uint32_t)e[k].y == w) {
+      rid = (uint32_t)(e[k].y >> 32);
+      open = false;
+    } else if (open && (uint32_t)e[k].x == NONE) {
+      slot = (h0 + k) & g.ht_mask;
+      create = is_ins;
+      open = false;
+    }
+  }
+  fall = fall || open;
+  uint32_t pos_o = 0, pos_i = 0, made = 0;
+  if (is_ins || is_del) {
+    // two ops on one record, or claiming one slot
+    const unsigned long long id = rid != UNSET ? rid : create ? (1ull << 40) | slot : (1ull << 50) | lane;
+    const bool twice = __popc(__match_any_sync(FULL, id)) > 1;  // (by every lane, whatever it has found)
+    fall = fall || twice;
+  }
+  if (is_ins) {
+    const unsigned cm = __ballot_sync(FULL, create);
+    made = __popc(cm);
+    const unsigned ms = __match_any_sync(FULL, create ? (unsigned long long)s : (1ull << 40) | lane);
+    const unsigned md = __match_any_sync(FULL, create ? (unsigned long long)d : (1ull << 40) | lane);
+    if (create) {
+      rid = (uint32_t)top + __popc(cm & lt);
+      pos_o = len_o + __popc(ms & lt);
+      pos_i = len_i + __popc(md & lt);
+      fall = fall || top + made > g.rec_cap || pos_o >= cap_o || (!g.symmetric && pos_i >= cap_i);
+    }
+    better_now = on && Hook<A>::better(Hook<A>::combine(val, w), lab.x);
+    const unsigned f = __ballot_sync(FULL, fall), im = __ballot_sync(FULL, better_now);
+    if (lane == 0) {
+      fs.fall[0] = f;
+      fs.improve = im;
+    }
+  }
+  __syncthreads();
+  if (is_del) {
+    for (uint32_t k = 0; ins && k < fs.n_ins; k++)  // an edge that this submission also inserts
+      fall = fall || (on && fs.s[k] == s && fs.d[k] == d && fs.w[k] == w);
+    const unsigned f = __ballot_sync(FULL, fall);
+    if (lane == 0) fs.fall[1] = f;
+  }
+  if (tid == 64) {  // (a warp of its own)
+    fs.seeds = 0;
+    prologue_ctl(c, del ? del->inv_tag : 0ull);
+    c[C_STAMP] += ins && del ? 1 : 0;  // as two batches count
+    c[C_CANDN] = 0;
+  }
+  __syncthreads();
+  if ((ins && fs.fall[0]) || (del && fs.fall[1])) return FAST_NO;
+  const bool seeds_ins = ins && fs.improve != 0;
+  // 3. storage; the delete batch waits for an insert that changes labels
+  const bool go = is_ins || (is_del && !seeds_ins);
+  uint32_t old = 0, ro = pos_o, ri = pos_i;
+  if (go && on && rid != UNSET && !create) {
+    old = __ldcg(&g.rec_num[rid]);
+    ro = __ldcg(&g.rec_out[rid]);
+    ri = __ldcg(&g.rec_in[rid]);
+  }
+  bool seed = false;
+  if (go && on && rid != UNSET && (is_ins || old)) {
+    E *po = reinterpret_cast<E *>(g.out.pool) + off_o, *pi = reinterpret_cast<E *>(g.in.pool) + off_i;
+    auto put = [](E *p, uint32_t x, uint32_t wt) {
+      if constexpr (W) *p = make_uint2(x, wt);
+      else *p = x;
+    };
+    const unsigned long long delta = is_ins ? 1ull : ~0ull;
+    if (create) {
+      g.ht[slot] = make_ulonglong2(key.x, key.y | ((uint64_t)rid << 32));
+      g.rec_out[rid] = ro;
+      g.rec_in[rid] = g.symmetric ? UNSET : ri;
+      g.out.owner[off_o + ro] = s;
+      atomicAdd(&g.out.len[s], 1u);
+      if (!g.symmetric) {
+        g.in.owner[off_i + ri] = d;
+        atomicAdd(&g.in.len[d], 1u);
+      }
+    }
+    g.rec_num[rid] = old + (uint32_t)delta;
+    atomicAdd(&g.out.deg[s], delta);
+    if (!g.symmetric) atomicAdd(&g.in.deg[d], delta);
+    if (old == (is_ins ? 0u : 1u)) {  // 0 -> 1 or 1 -> 0
+      const uint32_t dead = is_ins ? 0u : DEAD;
+      if (ro < cap_o) put(po + ro, d | dead, w);
+      if (!g.symmetric && ri < cap_i) put(pi + ri, s | dead, w);
+      seed = is_ins ? better_now : lab.y == pack_parent(s, w);
+    }
+  }
+  if (is_ins && made && lane == 0) *g.rec_top = top + made;
+  if (go && on && old_host) {
+    // both orientations of an undirected edge count alike
+    if (directed) old_host[lane] = old;
+    else if (!(lane & 1)) old_host[lane >> 1] = old;
+  }
+  // 4. seeds
+  if (is_ins && seeds_ins) {
+    const uint32_t st = (uint32_t)c[C_STAMP];
+    const bool upd = seed && relax<A>(g, s, ld_v32(g.val32, s), d, w);
+    const bool app = upd && atomicExch(&g.stamp[d], st) != st;
+    warp_append(app, d, q0, &c[C_QN0], FULL);
+    if (mst) mark_modified(g, upd, d, mst);
+    warp_add_result(upd, &c[C_RESULT]);
+    if (__any_sync(FULL, app) && lane == 0) fs.seeds = 1;
+  } else if (is_del && !seeds_ins) {
+    const uint32_t tag = (uint32_t)del->inv_tag;
+    const bool app = seed && atomicExch(&g.inv[d], tag) != tag;
+    warp_append(app, d, q0, &c[C_QN0], FULL);
+    if (__any_sync(FULL, app) && lane == 0) fs.seeds = 1;
+  }
+  __syncthreads();
+  if (seeds_ins) return FAST_INS_SEEDS;
+  return (del ? FAST_DEL_DONE : 0) | (fs.seeds ? FAST_DEL_SEEDS : 0);
+}
+
+// The repair after fast_inline, as a call (its code is in the kernel once more
+// in apply_batch), with the kernel's parameters in shared memory: a reference
+// into parameter space would be read through L1.
+struct FusedShared {
+  DevGraph g;
+  FusedRepair fr;
+};
+template <int A, bool W>
+__device__ __noinline__ int fast_repair(const FusedShared &f, int add, uint32_t *q0, uint32_t mst) {
+  return batch_repair<A, W>(f.g, f.fr, add, q0, mst, nullptr);
 }
 
 template <int A, bool W>
 __global__ void __launch_bounds__(FS_TPB)
-    k_apply_small(DevGraph g, sdev::OpView ops, const ApplyHdr *hdr, const char *data, uint64_t *old_host,
-                  uint32_t *cand, int add, int directed, uint32_t *q0, uint32_t mst, int second, FusedRepair fr,
-                  uint4 *scratch, unsigned long long *ctl_host) {
+    k_apply_small(const __grid_constant__ DevGraph g, const __grid_constant__ sdev::OpView ops, const ApplyHdr *hdr,
+                  const char *data, uint64_t *old_host, uint32_t *cand, int add, int directed, uint32_t *q0,
+                  uint32_t mst, int second, const __grid_constant__ FusedRepair fr, uint4 *scratch,
+                  unsigned long long *ctl_host) {
   __shared__ StagedBatch sb;
   if (g.ptrace && threadIdx.x == 0) {
     g.ptrace[32 + 2 * second] = global_ns();
@@ -2757,9 +3179,10 @@ __global__ void __launch_bounds__(FS_TPB)
 // repair.
 template <int A, bool W>
 __global__ void __launch_bounds__(FS_TPB)
-    k_apply_mixed(DevGraph g, sdev::OpView ops, const ApplyHdr *hdr1, const char *data1, const ApplyHdr *hdr2,
-                  const char *data2, uint32_t *cand, int directed, uint32_t *q0, uint32_t mst, FusedRepair fr,
-                  uint4 *scratch1, uint4 *scratch2, unsigned long long *ctl_host) {
+    k_apply_mixed(const __grid_constant__ DevGraph g, const __grid_constant__ sdev::OpView ops, const ApplyHdr *hdr1,
+                  const char *data1, const ApplyHdr *hdr2, const char *data2, uint32_t *cand, int directed,
+                  uint32_t *q0, uint32_t mst, const __grid_constant__ FusedRepair fr, uint4 *scratch1, uint4 *scratch2,
+                  unsigned long long *ctl_host) {
   __shared__ StagedBatch sb1, sb2;
   if (g.ptrace && threadIdx.x == 0) {
     g.ptrace[32] = g.ptrace[34] = global_ns();
@@ -2772,6 +3195,7 @@ __global__ void __launch_bounds__(FS_TPB)
   int r = apply_batch<A, W>(g, ops, sb1, data1, nullptr, cand, 1, directed, q0, mst, 0, fr, scratch1);
   unsigned long long lf = r == 1 ? 1 : 0;
   if (r == 0) {
+    __syncthreads();
     r = apply_batch<A, W>(g, ops, sb2, data2, nullptr, cand, 0, directed, q0, mst, 1, fr, scratch2);
     lf = r == 1 ? 2 : 0;
   }
@@ -2791,20 +3215,34 @@ __device__ __forceinline__ void inline_header(const DevGraph &g, const InlineBat
 }
 
 // k_apply_small for an inline batch (launched directly, not from a graph).
+// (With the phase trace on, batches take the phases that it stamps.)
 template <int A, bool W>
 __global__ void __launch_bounds__(FS_TPB)
-    k_apply_small_inl(DevGraph g, sdev::OpView ops, const __grid_constant__ InlineBatch ib, uint64_t *old_host,
-                      uint32_t *cand, int add, int directed, uint32_t *q0, uint32_t mst, FusedRepair fr,
+    k_apply_small_inl(const __grid_constant__ DevGraph g, const __grid_constant__ sdev::OpView ops,
+                      const __grid_constant__ InlineBatch ib, uint64_t *old_host, uint32_t *cand, int add, int directed,
+                      uint32_t *q0, uint32_t mst, const __grid_constant__ FusedRepair fr,
                       unsigned long long *ctl_host) {
   __shared__ StagedBatch sb;
-  if (g.ptrace && threadIdx.x == 0) {
-    g.ptrace[32] = g.ptrace[33] = global_ns();
-    g.ptrace[15] = 0;
-    g.ptrace[31] = 0;
+  __shared__ FusedShared f;
+  if (threadIdx.x == 96) {  // (a thread off the critical path)
+    f.g = g;
+    f.fr = fr;
   }
   inline_header(g, ib, sb);
   __syncthreads();
-  const int r = apply_batch<A, W>(g, ops, sb, nullptr, old_host, cand, add, directed, q0, mst, 0, fr, nullptr, ib.words);
+  int r = g.ptrace ? FAST_NO
+                   : fast_inline<A, W>(g, add ? &ib : nullptr, add ? nullptr : &ib, directed,
+                                       ib.want ? old_host : nullptr, q0, mst);
+  if (r == FAST_NO) {
+    if (g.ptrace && threadIdx.x == 0) {
+      g.ptrace[32] = g.ptrace[33] = global_ns();
+      g.ptrace[15] = 0;
+      g.ptrace[31] = 0;
+    }
+    r = apply_batch<A, W>(g, ops, sb, nullptr, old_host, cand, add, directed, q0, mst, 0, fr, nullptr, ib.words);
+  } else {
+    r = r & (FAST_INS_SEEDS | FAST_DEL_SEEDS) ? fast_repair<A, W>(f, add, q0, mst) : 0;
+  }
   if (threadIdx.x == 0) g.ctl[C_LEFT] = r == 1 ? (add ? 1 : 2) : 0;
   ctl_to_host(g, ctl_host);
 }
@@ -2814,21 +3252,37 @@ __global__ void __launch_bounds__(FS_TPB)
 // the staging buffer too (the host wrote it there before the launch).
 template <int A, bool W>
 __global__ void __launch_bounds__(FS_TPB)
-    k_apply_mixed_inl(DevGraph g, sdev::OpView ops, const __grid_constant__ InlineBatch ib1,
-                      const __grid_constant__ InlineBatch ib2, uint32_t *cand, int directed, uint32_t *q0,
-                      uint32_t mst, FusedRepair fr, unsigned long long *ctl_host) {
+    k_apply_mixed_inl(const __grid_constant__ DevGraph g, const __grid_constant__ sdev::OpView ops,
+                      const __grid_constant__ InlineBatch ib1, const __grid_constant__ InlineBatch ib2, uint32_t *cand,
+                      int directed, uint32_t *q0, uint32_t mst, const __grid_constant__ FusedRepair fr,
+                      unsigned long long *ctl_host) {
   __shared__ StagedBatch sb1, sb2;
-  if (g.ptrace && threadIdx.x == 0) {
-    g.ptrace[32] = g.ptrace[33] = g.ptrace[34] = g.ptrace[35] = global_ns();
-    g.ptrace[15] = g.ptrace[31] = 0;
+  __shared__ FusedShared f;
+  if (threadIdx.x == 96) {  // (a thread off the critical path)
+    f.g = g;
+    f.fr = fr;
   }
   inline_header(g, ib1, sb1);
   inline_header(g, ib2, sb2);
   __syncthreads();
-  int r = apply_batch<A, W>(g, ops, sb1, nullptr, nullptr, cand, 1, directed, q0, mst, 0, fr, nullptr, ib1.words);
+  const int fast = g.ptrace ? FAST_NO : fast_inline<A, W>(g, &ib1, &ib2, directed, nullptr, q0, mst);
+  int r = 0;  // the insert batch
+  if (fast == FAST_NO) {
+    if (g.ptrace && threadIdx.x == 0) {
+      g.ptrace[32] = g.ptrace[33] = g.ptrace[34] = g.ptrace[35] = global_ns();
+      g.ptrace[15] = g.ptrace[31] = 0;
+    }
+    r = apply_batch<A, W>(g, ops, sb1, nullptr, nullptr, cand, 1, directed, q0, mst, 0, fr, nullptr, ib1.words);
+  } else if (fast & FAST_INS_SEEDS) {
+    r = fast_repair<A, W>(f, 1, q0, mst);
+  }
   unsigned long long lf = r == 1 ? 1 : 0;
   if (r == 0) {
-    r = apply_batch<A, W>(g, ops, sb2, nullptr, nullptr, cand, 0, directed, q0, mst, 1, fr, nullptr, ib2.words);
+    __syncthreads();
+    if (fast == FAST_NO || !(fast & FAST_DEL_DONE))
+      r = apply_batch<A, W>(g, ops, sb2, nullptr, nullptr, cand, 0, directed, q0, mst, 1, fr, nullptr, ib2.words);
+    else if (fast & FAST_DEL_SEEDS)
+      r = fast_repair<A, W>(f, 0, q0, mst);
     lf = r == 1 ? 2 : 0;
   }
   if (threadIdx.x == 0) g.ctl[C_LEFT] = lf;
@@ -2862,7 +3316,7 @@ constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alo
 // entries (RMAT-22 SSWP: the push of 97K vertices took 241 us, a pull level 75)
 constexpr uint64_t ENG_PULL_DIV = 12;
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
-constexpr uint32_t ENG_SPINS = 1u << 26;     // polls before a barrier gives up (tens of seconds)
+constexpr uint32_t ENG_SPINS = 1u << 24;     // polls before a barrier gives up (ten seconds or more)
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
 
