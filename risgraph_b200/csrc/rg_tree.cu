@@ -2066,15 +2066,15 @@ __device__ __forceinline__ bool queue_heavy(uint32_t *hv, unsigned long long *hv
   return false;
 }
 
-// Rescue of one invalidated vertex d (value sd, in-list [off, off + len)) by a
-// warp.
+// Rescue of one invalidated vertex d (value sd) by a warp, over slots [lo, len)
+// of its in-list at off; returns whether d is rescued.
 template <int A, bool W>
-__device__ __forceinline__ void rescue_one(const DevGraph &g, uint32_t d, uint64_t sd, uint32_t len, uint64_t off,
-                                           uint32_t tag_inv, uint64_t limit) {
+__device__ __forceinline__ bool rescue_one(const DevGraph &g, uint32_t d, uint64_t sd, uint32_t lo, uint32_t len,
+                                           uint64_t off, uint32_t tag_inv, uint64_t limit) {
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
-  for (uint32_t kb = 0; kb < len; kb += 32) {
+  for (uint32_t kb = lo; kb < len; kb += 32) {
     const uint32_t k = kb + lane;
     bool ok = false;
     uint32_t src = 0, w = 0;
@@ -2084,21 +2084,35 @@ __device__ __forceinline__ void rescue_one(const DevGraph &g, uint32_t d, uint64
       w = P::wt(e);
       if (!(src & DEAD) && Hook<A>::combine(ld_v32(g.val32, src), w) == sd) ok = !has_parents(g, src, tag_inv, limit);
     }
-    unsigned b = __ballot_sync(FULL, ok);
-    bool done = false;
-    while (b) {
-      int l = __ffs(b) - 1;
-      b &= b - 1;
-      bool won = false;
-      if (lane == l) {
-        won = atomicCAS(&g.inv[d], tag_inv, tag_inv + 1) == tag_inv;
-        if (won) reinterpret_cast<unsigned long long *>(&g.lab[d])[1] = pack_parent(src, w);
-      }
-      won = __shfl_sync(FULL, won, l);
-      if (won) { done = true; break; }
+    const unsigned b = __ballot_sync(FULL, ok);
+    if (b) {  // the first candidate, unless another warp was first
+      if (lane == __ffs(b) - 1 && atomicCAS(&g.inv[d], tag_inv, tag_inv + 1) == tag_inv)
+        reinterpret_cast<unsigned long long *>(&g.lab[d])[1] = pack_parent(src, w);
+      return true;
     }
-    if (done || __shfl_sync(FULL, ld_u32(&g.inv[d]), 0) != tag_inv) break;
+    if (__shfl_sync(FULL, ld_u32(&g.inv[d]), 0) != tag_inv) return true;
   }
+  return false;
+}
+
+// Long lists in the grid engine: a warp scans the first TASK_SLOTS slots of a
+// list of more than TASK_DEG and queues the rest as tasks of TASK_SLOTS, which
+// every warp of the grid takes after the next barrier.  (With whole lists of up
+// to HEAVY_DEG to a warp, each pass of a batch of 100,000 deletions waited 70 us
+// for its longest list.)
+constexpr uint32_t TASK_DEG = 256, TASK_SLOTS = 128;
+struct RepQueue {
+  uint32_t *hv = nullptr;  // vertices left for a pass of their own ...
+  unsigned long long *n = nullptr;
+  uint64_t cap = 0;
+  uint64_t *task = nullptr;  // ... or tasks (vertex | chunk << 32), with n their count
+};
+__device__ __forceinline__ void queue_tasks(const RepQueue &q, uint32_t v, uint32_t len, int lane) {
+  const uint32_t nt = (len - 1) / TASK_SLOTS;  // chunks 1 .. nt
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(q.n, (unsigned long long)nt);
+  at = __shfl_sync(FULL, at, 0);
+  for (uint32_t c = lane; c < nt; c += 32) q.task[at + c] = (uint64_t)v | ((uint64_t)(c + 1) << 32);
 }
 
 // The passes of the deletion repair over more vertices than there are warps
@@ -2123,12 +2137,19 @@ __device__ __forceinline__ bool queue_heavy_group(bool want, uint32_t *hv, unsig
 
 template <int A, bool W>
 __device__ __forceinline__ void rescue_warps(const DevGraph &g, const uint32_t *fin, uint64_t n, uint64_t limit,
-                                             uint64_t warp, uint64_t nwarps, uint32_t *hv = nullptr,
-                                             unsigned long long *hv_n = nullptr, uint64_t hv_cap = 0) {
+                                             uint64_t warp, uint64_t nwarps, const RepQueue &rq = RepQueue{}) {
   const uint32_t tag_inv = (uint32_t)g.ctl[C_INVTAG];
   using P = PoolT<W>;
   const typename P::E *pool = reinterpret_cast<const typename P::E *>(g.in.pool);
   const int lane = lane_id();
+  uint32_t *const hv = rq.hv;
+  unsigned long long *const hv_n = rq.n;
+  const uint64_t hv_cap = rq.cap;
+  auto one = [&](uint32_t d, uint64_t sd, uint32_t len, uint64_t off) {
+    const bool cut = rq.task && len > TASK_DEG;
+    const bool done = rescue_one<A, W>(g, d, sd, 0, cut ? TASK_SLOTS : len, off, tag_inv, limit);
+    if (cut && !done) queue_tasks(rq, d, len, lane);
+  };
   if (n <= nwarps) {
     for (uint64_t idx = warp; idx < n; idx += nwarps) {
       const uint32_t d = fin[idx];
@@ -2139,7 +2160,7 @@ __device__ __forceinline__ void rescue_warps(const DevGraph &g, const uint32_t *
       const uint64_t off = g.in.off[d];
       if (td != tag_inv) continue;
       if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
-      rescue_one<A, W>(g, d, sd, len, off, tag_inv, limit);
+      one(d, sd, len, off);
     }
     return;
   }
@@ -2185,7 +2206,7 @@ __device__ __forceinline__ void rescue_warps(const DevGraph &g, const uint32_t *
       const int l = __ffs(m) - 1;
       const uint32_t d1 = __shfl_sync(FULL, d, l), len1 = __shfl_sync(FULL, len, l);
       const uint64_t sd1 = __shfl_sync(FULL, sd, l), off1 = __shfl_sync(FULL, off, l);
-      rescue_one<A, W>(g, d1, sd1, len1, off1, tag_inv, limit);
+      one(d1, sd1, len1, off1);
     }
   }
 }
@@ -2196,7 +2217,7 @@ __global__ void __launch_bounds__(TPB) k_rescue(DevGraph g, const uint32_t *fin,
   if (g.ctl[C_RECOMPUTE]) return;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  rescue_warps<A, W>(g, fin, *fin_n, limit, warp, nwarps, g.heavy, &g.ctl[C_HVR], g.heavy_cap);
+  rescue_warps<A, W>(g, fin, *fin_n, limit, warp, nwarps, RepQueue{g.heavy, &g.ctl[C_HVR], g.heavy_cap});
 }
 
 // Rescue of the queued heavy vertices: for each in turn, every warp scans a
@@ -2280,10 +2301,20 @@ __device__ __forceinline__ void expand_slots(const DevGraph &g, uint32_t u, uint
 template <int A, bool W>
 __device__ __forceinline__ void expand_warps(const DevGraph &g, const uint32_t *fin, uint64_t n, uint32_t *tree,
                                              uint32_t *fout, unsigned long long *fout_n, uint64_t warp,
-                                             uint64_t nwarps, uint32_t *hv = nullptr,
-                                             unsigned long long *hv_n = nullptr, uint64_t hv_cap = 0) {
+                                             uint64_t nwarps, const RepQueue &rq = RepQueue{}) {
   const uint32_t tag_inv = (uint32_t)g.ctl[C_INVTAG];
   const int lane = lane_id();
+  uint32_t *const hv = rq.hv;
+  unsigned long long *const hv_n = rq.n;
+  const uint64_t hv_cap = rq.cap;
+  auto one = [&](uint32_t u, uint32_t len, uint64_t off) {
+    const bool cut = rq.task && len > TASK_DEG;
+    if (cut) queue_tasks(rq, u, len, lane);
+    const uint32_t end = cut ? TASK_SLOTS : len;
+    uint32_t kb = 0;
+    for (; kb + 32 < end; kb += 128) expand_slots<W, 4>(g, u, off, kb + lane, 32, end, tag_inv, fout, fout_n);
+    if (kb < end) expand_slots<W, 1>(g, u, off, kb + lane, 32, end, tag_inv, fout, fout_n);
+  };
   if (n <= nwarps) {
     for (uint64_t idx = warp; idx < n; idx += nwarps) {
       const uint32_t u = fin[idx];
@@ -2295,11 +2326,7 @@ __device__ __forceinline__ void expand_warps(const DevGraph &g, const uint32_t *
       if (tu != tag_inv) continue;
       unsigned long long slot = 0;
       if (lane == 0) slot = atomicAdd(&g.ctl[C_TREEN], 1ull);
-      if (!(hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, u, lane))) {
-        uint32_t kb = 0;
-        for (; kb + 32 < len; kb += 128) expand_slots<W, 4>(g, u, off, kb + lane, 32, len, tag_inv, fout, fout_n);
-        if (kb < len) expand_slots<W, 1>(g, u, off, kb + lane, 32, len, tag_inv, fout, fout_n);
-      }
+      if (!(hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, u, lane))) one(u, len, off);
       if (lane == 0) tree[slot] = u;
     }
     return;
@@ -2331,8 +2358,7 @@ __device__ __forceinline__ void expand_warps(const DevGraph &g, const uint32_t *
       const int l = __ffs(m) - 1;
       const uint32_t u1 = __shfl_sync(FULL, u, l), len1 = __shfl_sync(FULL, len, l);
       const uint64_t off1 = __shfl_sync(FULL, off, l);
-      for (uint32_t kb = 0; kb < len1; kb += 128)
-        expand_slots<W, 4>(g, u1, off1, kb + lane, 32, len1, tag_inv, fout, fout_n);
+      one(u1, len1, off1);
     }
   }
 }
@@ -2382,8 +2408,8 @@ __global__ void __launch_bounds__(TPB) k_expand(DevGraph g, const uint32_t *fin,
   if (g.ctl[C_RECOMPUTE]) return;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  expand_warps<A, W>(g, fin, *fin_n, tree, fout, fout_n, warp, nwarps, g.heavy + g.heavy_cap, &g.ctl[C_HVE],
-                     g.heavy_cap);
+  expand_warps<A, W>(g, fin, *fin_n, tree, fout, fout_n, warp, nwarps,
+                     RepQueue{g.heavy + g.heavy_cap, &g.ctl[C_HVE], g.heavy_cap});
 }
 
 // Reset the invalid set to init (core/graph.hpp:1420-1430).
@@ -2461,21 +2487,29 @@ __device__ __forceinline__ bool pull_reduce(const DevGraph &g, PullBest p, uint3
 template <int A, bool W>
 __device__ __forceinline__ unsigned long long pull_warps(const DevGraph &g, const uint32_t *fin, uint64_t n,
                                                          uint32_t mst, uint64_t warp, uint64_t nwarps,
-                                                         uint32_t *hv = nullptr, unsigned long long *hv_n = nullptr,
-                                                         uint64_t hv_cap = 0) {
+                                                         const RepQueue &rq = RepQueue{}) {
   const int lane = lane_id();
   unsigned long long local = 0;
+  uint32_t *const hv = rq.hv;
+  unsigned long long *const hv_n = rq.n;
+  const uint64_t hv_cap = rq.cap;
+  auto one = [&](uint32_t d, uint32_t len, uint64_t off) {
+    const bool cut = rq.task && len > TASK_DEG;
+    if (cut) queue_tasks(rq, d, len, lane);
+    const uint32_t end = cut ? TASK_SLOTS : len;
+    PullBest p = {ld_v32(g.val32, d), 0, NONE, 0};
+    uint32_t kb = 0;
+    for (; kb + 32 < end; kb += 128) pull_slots<A, W, 4>(g, off, kb + lane, 32, end, p);
+    if (kb < end) pull_slots<A, W, 1>(g, off, kb + lane, 32, end, p);
+    local += pull_reduce<A>(g, p, d, true, 32, mst);
+  };
   if (n <= nwarps) {
     for (uint64_t idx = warp; idx < n; idx += nwarps) {
       const uint32_t d = fin[idx];
       const uint32_t len = seg_len(g.in, d);
       const uint64_t off = g.in.off[d];
       if (hv && len > HEAVY_DEG && queue_heavy(hv, hv_n, hv_cap, d, lane)) continue;
-      PullBest p = {ld_v32(g.val32, d), 0, NONE, 0};
-      uint32_t kb = 0;
-      for (; kb + 32 < len; kb += 128) pull_slots<A, W, 4>(g, off, kb + lane, 32, len, p);
-      if (kb < len) pull_slots<A, W, 1>(g, off, kb + lane, 32, len, p);
-      local += pull_reduce<A>(g, p, d, true, 32, mst);
+      one(d, len, off);
     }
     return local;
   }
@@ -2505,9 +2539,7 @@ __device__ __forceinline__ unsigned long long pull_warps(const DevGraph &g, cons
       const int l = __ffs(m) - 1;
       const uint32_t d1 = __shfl_sync(FULL, d, l), len1 = __shfl_sync(FULL, len, l);
       const uint64_t off1 = __shfl_sync(FULL, off, l);
-      PullBest p1 = {ld_v32(g.val32, d1), 0, NONE, 0};
-      for (uint32_t kb = 0; kb < len1; kb += 128) pull_slots<A, W, 4>(g, off1, kb + lane, 32, len1, p1);
-      local += pull_reduce<A>(g, p1, d1, true, 32, mst);
+      one(d1, len1, off1);
     }
   }
   return local;
@@ -2520,7 +2552,8 @@ __global__ void __launch_bounds__(TPB) k_pull(DevGraph g, const uint32_t *fin, c
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long local =
-      pull_warps<A, W>(g, fin, *fin_n, mst, warp, nwarps, g.heavy + 2 * g.heavy_cap, &g.ctl[C_HVP], g.heavy_cap);
+      pull_warps<A, W>(g, fin, *fin_n, mst, warp, nwarps,
+                       RepQueue{g.heavy + 2 * g.heavy_cap, &g.ctl[C_HVP], g.heavy_cap});
   warp_add_result(local, &g.ctl[C_RESULT]);
 }
 
@@ -3319,6 +3352,7 @@ constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others
 constexpr uint32_t ENG_SPINS = 1u << 24;     // polls before a barrier gives up (ten seconds or more)
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
+static_assert(TASK_SLOTS >= CHUNK && TASK_DEG >= 2 * TASK_SLOTS, "the hub task queue holds the tasks");
 
 struct EngineArgs {
   // sliced in-edge copy (pull levels)
@@ -3329,6 +3363,7 @@ struct EngineArgs {
   const SellPlan *plan;
   // queues and scratch
   uint32_t *q[2], *tree;
+  uint64_t *task;               // tasks of long lists (deletion repairs)
   uint64_t *P;                  // frontier degree prefix, per CTA piece
   unsigned long long *tot;      // slots of each CTA's piece
   unsigned long long *bar;      // barrier words, third queue counter, bounds
@@ -3446,7 +3481,7 @@ __device__ __forceinline__ void eng_share(uint64_t S, uint64_t &e0, uint64_t &e1
 
 // Deletion repair over the whole grid (do_update_tree_del,
 // core/graph.hpp:1250-1511): the phases of k_rescue, k_expand, k_reset and
-// k_pull, and of their heavy-vertex passes when a vertex was queued for one.
+// k_pull, each followed by the tasks of the long lists it met.
 // Leaves the reset set in queue 0 with its count in ctl[C_QN0].
 template <int A, bool W>
 __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar) {
@@ -3470,11 +3505,24 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
       *cnt(it + 2) = 0;
       c[C_INVITER] = it + 1;
     }
-    rescue_warps<A, W>(g, fin, n, a.limit, warp, nwarps, g.heavy, &hvr[it & 1], g.heavy_cap);
+    RepQueue rq;
+    rq.task = a.task;
+    rq.n = &hvr[it & 1];
+    rescue_warps<A, W>(g, fin, n, a.limit, warp, nwarps, rq);
     if (!grid_sync(g, bar)) return false;
-    const uint64_t nr = __ldcg(&hvr[it & 1]);
+    const uint64_t nr = __ldcg(rq.n);
     if (nr) {
-      rescue_heavy_warps<A, W>(g, nr, a.limit, warp, nwarps);
+      const uint32_t tag_inv = (uint32_t)c[C_INVTAG];
+      for (uint64_t t = warp; t < nr; t += nwarps) {
+        const uint64_t x = a.task[t];
+        const uint32_t d = (uint32_t)x, k0 = (uint32_t)(x >> 32) * TASK_SLOTS;
+        const uint32_t td = ld_u32(&g.inv[d]);
+        const uint64_t sd = ld_v32(g.val32, d);
+        const uint32_t len = seg_len(g.in, d);
+        const uint64_t off = g.in.off[d];
+        if (__shfl_sync(FULL, td, 0) != tag_inv) continue;  // rescued by another task
+        rescue_one<A, W>(g, d, sd, k0, min(len, k0 + TASK_SLOTS), off, tag_inv, a.limit);
+      }
       if (!grid_sync(g, bar)) return false;
     }
     if (__ldcg(&c[C_RECOMPUTE])) {  // a chain ran past the guard (nothing sets it before the next level's rescue)
@@ -3482,12 +3530,19 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
       break;
     }
     if (lead) hvr[(it + 1) & 1] = hve[(it + 1) & 1] = 0;
-    expand_warps<A, W>(g, fin, n, a.tree, fout, cnt(it + 1), warp, nwarps, g.heavy + g.heavy_cap, &hve[it & 1],
-                       g.heavy_cap);
+    rq.n = &hve[it & 1];
+    expand_warps<A, W>(g, fin, n, a.tree, fout, cnt(it + 1), warp, nwarps, rq);
     if (!grid_sync(g, bar)) return false;
-    const uint64_t ne = __ldcg(&hve[it & 1]);
+    const uint64_t ne = __ldcg(rq.n);
     if (ne) {
-      expand_heavy_warps<A, W>(g, ne, fout, cnt(it + 1), warp, nwarps);
+      const uint32_t tag_inv = (uint32_t)c[C_INVTAG];
+      for (uint64_t t = warp; t < ne; t += nwarps) {
+        const uint64_t x = a.task[t];
+        const uint32_t u = (uint32_t)x, k0 = (uint32_t)(x >> 32) * TASK_SLOTS;
+        const uint32_t len = seg_len(g.out, u);
+        expand_slots<W, 4>(g, u, g.out.off[u], k0 + lane_id(), 32, min(len, k0 + TASK_SLOTS), tag_inv, fout,
+                           cnt(it + 1));
+      }
       if (!grid_sync(g, bar)) return false;
     }
   }
@@ -3504,15 +3559,24 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
   for (uint64_t i = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; i < tn; i += (uint64_t)gridDim.x * ENG_TPB)
     a.q[0][i] = a.tree[i];
   if (!grid_sync(g, bar)) return false;
-  unsigned long long local = pull_warps<A, W>(g, a.tree, tn, a.mst, warp, nwarps, g.heavy + 2 * g.heavy_cap, &c[C_HVP],
-                                              g.heavy_cap);
-  warp_add_result(local, &c[C_RESULT]);
+  RepQueue rq;
+  rq.task = a.task;
+  rq.n = &c[C_HVP];
+  unsigned long long local = pull_warps<A, W>(g, a.tree, tn, a.mst, warp, nwarps, rq);
   if (!grid_sync(g, bar)) return false;
-  if (__ldcg(&c[C_HVP])) {
-    local = pull_heavy_warps<A, W>(g, a.mst, warp, nwarps);
-    warp_add_result(local, &c[C_RESULT]);
+  const uint64_t np = __ldcg(rq.n);
+  if (np) {
+    for (uint64_t t = warp; t < np; t += nwarps) {
+      const uint64_t x = a.task[t];
+      const uint32_t d = (uint32_t)x, k0 = (uint32_t)(x >> 32) * TASK_SLOTS;
+      const uint32_t len = seg_len(g.in, d);
+      PullBest p = {ld_v32(g.val32, d), 0, NONE, 0};
+      pull_slots<A, W, 4>(g, g.in.off[d], k0 + lane_id(), 32, min(len, k0 + TASK_SLOTS), p);
+      local += pull_reduce<A>(g, p, d, true, 32, a.mst);
+    }
     if (!grid_sync(g, bar)) return false;
   }
+  warp_add_result(local, &c[C_RESULT]);
   return true;
 }
 
@@ -4489,6 +4553,7 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
   a.q[0] = g.q[0];
   a.q[1] = g.q[1];
   a.tree = g.tree;
+  a.task = g.hubq;  // (at least a task for every CHUNK slots of a pool)
   a.P = g.lb_P;
   a.tot = reinterpret_cast<unsigned long long *>(g.lb_sums);
   a.bar = g.eng_bar;
