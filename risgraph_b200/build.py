@@ -32,9 +32,9 @@ NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-ccbin", HOST_CXX, "-Xcompi
                   "-I" + INCLUDE, "-I" + CSRC, "--expt-relaxed-constexpr"]
 
 CU_SOURCES = ["rg_api.cu", "rg_storage.cu", "rg_tree.cu", "rg_static.cu", "rg_serve.cu", "rg_history.cu", "rg_autotune.cu"]
-C_SOURCES = ["rg_gen.c"]
+C_SOURCES = ["rg_gen.c", "rg_stage.c"]
 CXX_SOURCES = ["rg_front.cpp"]
-HEADERS = ["rg_internal.cuh", "rg_storage_dev.cuh"]
+HEADERS = ["rg_internal.cuh", "rg_storage_dev.cuh", "rg_stage.h"]
 
 
 def _newer(target, deps):
@@ -76,7 +76,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src.replace(".c", ".o"))
         if force or _newer(o, [s] + hdrs):
-            _run([HOST_CC, "-O3", "-fPIC", "-fopenmp", "-std=c11", "-I" + INCLUDE, "-c", s, "-o", o], verbose)
+            _run([HOST_CC, "-O3", "-fPIC", "-fopenmp", "-std=c11", "-I" + INCLUDE, "-I" + CSRC, "-c", s, "-o", o], verbose)
         objs.append(o)
     if force or _newer(LIB, objs):
         _run([NVCC] + ARCH + ["-ccbin", HOST_CXX, "-shared", "-o", LIB] + objs +

@@ -9,6 +9,7 @@
 #include <string>
 
 #include "rg_internal.cuh"
+#include "rg_stage.h"
 
 namespace rg {
 
@@ -107,40 +108,72 @@ int check_algo(const Graph &g, int algo) {
   return RG_OK;
 }
 
+// One staged batch of at most CHUNK_EDGES edges whose ops are unpacked: storage
+// update, candidate list and, when `apply`, tree repair in one submission.
+int batch_update(Graph &g, uint64_t m, uint64_t nops, int directed, uint64_t *old_num, bool add, bool apply) {
+  const int what = add ? 1 : 2;
+  int rc = rg::storage_enqueue(g, add, m, nops, directed, apply);
+  if (!rc && apply) rc = rg::tree_enqueue(g, what, m, directed, true);
+  if (!rc && old_num) rc = rg::storage_copy_old(g, m);
+  if (!rc) rc = rg::sync_ctl(g);
+  if (rc) return rc;
+  if (add && g.h_ctl[rg::C_ERR] == RG_ENOSPACE && g.h_ctl[rg::C_AUX] == 1) {
+    // growth ran out of pool: compact, then replay from the growth step
+    rc = rg::storage_recover(g);
+    if (!rc) rc = rg::storage_replay(g, m, nops, directed, apply);
+    if (!rc && apply) rc = rg::tree_enqueue(g, what, m, directed, true);
+    if (!rc && old_num) rc = rg::storage_copy_old(g, m);
+    if (!rc) rc = rg::sync_ctl(g);
+    if (rc) return rc;
+  }
+  if ((rc = rg::storage_error(g))) return rc;
+  if (apply && (rc = rg::tree_after_sync(g, what, nullptr))) return rc;
+  if (old_num) std::memcpy(old_num, rg::storage_old_host(g), m * 8);
+  return RG_OK;
+}
+
+// Stage a batch that nothing has checked yet, in one pass over it: an error
+// status names the first bad edge's fault; weights that need codes take the
+// slow way.
+int stage_unchecked(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, uint64_t after) {
+  int flags = 0;
+  int rc = rg::stage_copy(g, edges, pairs, n, after, &flags);
+  if (rc || !flags) return rc;
+  if ((rc = check_edges(g, edges, pairs, n))) {
+    // (an earlier step of the batch may still be on its way from the buffer)
+    cudaStreamSynchronize(g.stream);
+    return rc;
+  }
+  RG_CUDA(cudaStreamSynchronize(g.stream));
+  std::vector<rg_edge> buf;
+  if ((rc = device_edges(g, edges, n, buf, &edges))) return rc;
+  return rg::stage_coded(g, edges, n, after);
+}
+
 // add/del over edges or pairs, chunked; tree repair of each chunk's candidates
 // when `apply` (the final values are the unique fixpoint either way).
 int edge_updates(rg_graph *gh, const rg_edge *edges, const uint64_t *pairs, uint64_t n, int directed,
                  uint64_t *old_num, bool add, bool apply) {
   Graph &g = gh->g;
-  int rc = check_edges(g, edges, pairs, n);
-  if (rc) return rc;
+  int rc = RG_OK;
+  // small batches (single updates, served epochs): one fused launch
+  const bool small = apply && n && n <= g.fused_max && !g.profiling;
+  if (!small && n && n <= CHUNK_EDGES && (edges || pairs)) {
+    uint64_t nops = 0;
+    rc = rg::stage_reserve(g, pairs != nullptr, n, 0);
+    if (!rc) rc = stage_unchecked(g, edges, pairs, n, 0);
+    if (!rc) rc = rg::stage_unpack(g, pairs != nullptr, n, 0, directed, &nops);
+    return rc ? rc : batch_update(g, n, nops, directed, old_num, add, apply);
+  }
+  if ((rc = check_edges(g, edges, pairs, n))) return rc;
   std::vector<rg_edge> wbuf;
   if ((rc = device_edges(g, edges, n, wbuf, &edges))) return rc;
-  // small batches (single updates, served epochs): one fused graph launch
-  if (apply && n && n <= g.fused_max && !g.profiling) return rg::apply_small(g, edges, pairs, n, directed, add, old_num);
-  const int what = add ? 1 : 2;
+  if (small) return rg::apply_small(g, edges, pairs, n, directed, add, old_num);
   for (uint64_t b = 0; b < n; b += CHUNK_EDGES) {
     uint64_t m = std::min(CHUNK_EDGES, n - b), nops = 0;
     rc = rg::stage_edges(g, edges ? edges + b : nullptr, pairs ? pairs + 2 * b : nullptr, m, directed, &nops);
     if (rc) return rc;
-    // storage update, candidate list and tree repair in one submission
-    rc = rg::storage_enqueue(g, add, m, nops, directed, apply);
-    if (!rc && apply) rc = rg::tree_enqueue(g, what, m, directed, true);
-    if (!rc && old_num) rc = rg::storage_copy_old(g, m);
-    if (!rc) rc = rg::sync_ctl(g);
-    if (rc) return rc;
-    if (add && g.h_ctl[rg::C_ERR] == RG_ENOSPACE && g.h_ctl[rg::C_AUX] == 1) {
-      // growth ran out of pool: compact, then replay from the growth step
-      rc = rg::storage_recover(g);
-      if (!rc) rc = rg::storage_replay(g, m, nops, directed, apply);
-      if (!rc && apply) rc = rg::tree_enqueue(g, what, m, directed, true);
-      if (!rc && old_num) rc = rg::storage_copy_old(g, m);
-      if (!rc) rc = rg::sync_ctl(g);
-      if (rc) return rc;
-    }
-    if ((rc = rg::storage_error(g))) return rc;
-    if (apply && (rc = rg::tree_after_sync(g, what, nullptr))) return rc;
-    if (old_num) std::memcpy(old_num + b, rg::storage_old_host(g), m * 8);
+    if ((rc = batch_update(g, m, nops, directed, old_num ? old_num + b : nullptr, add, apply))) return rc;
   }
   return RG_OK;
 }
@@ -302,6 +335,20 @@ int rg_apply_add_del(rg_graph *g, int algo, const rg_edge *adds, uint64_t n_add,
                      int directed) {
   int rc = check_graph(g);
   if (!rc) rc = check_algo(g->g, algo);
+  if (rc) return rc;
+  const uint64_t most = std::max(n_add, n_del);
+  if (adds && dels && n_add && n_del && most > g->g.fused_max && most <= CHUNK_EDGES && !g->g.profiling) {
+    // both batches are checked, packed and on their way before the first one runs
+    Graph &gr = g->g;
+    uint64_t nops = 0;
+    rc = rg::stage_reserve(gr, false, n_add, n_del);
+    if (!rc) rc = stage_unchecked(gr, adds, nullptr, n_add, 0);
+    if (!rc) rc = stage_unchecked(gr, dels, nullptr, n_del, n_add);
+    if (!rc) rc = rg::stage_unpack(gr, false, n_add, 0, directed, &nops);
+    if (!rc) rc = batch_update(gr, n_add, nops, directed, nullptr, true, true);
+    if (!rc) rc = rg::stage_unpack(gr, false, n_del, n_add, directed, &nops);
+    return rc ? rc : batch_update(gr, n_del, nops, directed, nullptr, false, true);
+  }
   if (!rc) rc = check_edges(g->g, adds, nullptr, n_add);
   if (!rc) rc = check_edges(g->g, dels, nullptr, n_del);
   if (rc) return rc;

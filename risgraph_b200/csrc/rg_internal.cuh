@@ -432,6 +432,14 @@ void storage_free(Graph &g);
 // Stage n edges (rg_edge or reference pairs) into the device op arrays as
 // directed ops (2 per edge when undirected).  Returns number of ops.
 int stage_edges(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, int directed, uint64_t *nops);
+// The same in steps, for one or two batches of a submission: reserve the
+// buffers for n1 and n2 edges; check a batch, pack it and copy it to the device
+// (`after`: the edges of the batch staged before it; flags: RG_STAGE_BAD /
+// RG_STAGE_HEAVY, and the batch is not staged); make its ops.
+int stage_reserve(Graph &g, bool pairs, uint64_t n1, uint64_t n2);
+int stage_copy(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, uint64_t after, int *flags);
+int stage_coded(Graph &g, const rg_edge *edges, uint64_t n, uint64_t after);  // a checked batch with coded weights
+int stage_unpack(Graph &g, bool pairs, uint64_t n, uint64_t after, int directed, uint64_t *nops);
 // One staged batch: storage_enqueue launches the multiplicity update (and, when
 // collect, the tree-repair candidate list) without waiting; after sync_ctl,
 // storage_error reports a device error.  A pool exhausted by growth is

@@ -21,6 +21,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "rg_internal.cuh"
+#include "rg_stage.h"
 #include "rg_storage_dev.cuh"
 
 namespace rg {
@@ -34,12 +35,16 @@ using namespace sdev;
 #define GRID_STRIDE(j, n) \
   for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, _st = (uint64_t)gridDim.x * blockDim.x; j < (n); j += _st)
 
-__global__ void k_unpack_edges(const rg_edge *e, uint64_t n, int directed, int weighted, OpView ops) {
-  GRID_STRIDE(i, n) unpack_edge(e, i, directed, weighted, ops);
-}
-
-__global__ void k_unpack_pairs(const uint64_t *p, uint64_t n, int directed, int weighted, OpView ops) {
-  GRID_STRIDE(i, n) unpack_pair(p, i, directed, weighted, ops);
+// The staged records ({src, dst} or {src, dst, weight} words).  pairs: the
+// reference's file format, whose weights are a function of the endpoints.
+__global__ void k_unpack(const uint32_t *r, uint64_t n, int directed, int weighted, int pairs, OpView ops) {
+  const int words = weighted && !pairs ? 3 : 2;
+  GRID_STRIDE(i, n) {
+    const uint32_t s = r[words * i], d = r[words * i + 1];
+    uint32_t w = 0;
+    if (weighted) w = pairs ? (uint32_t)(splitmix64(((uint64_t)s << 32) | d) % 255 + 1) : r[3 * i + 2];
+    put_ops(ops, i, s, d, w, directed);
+  }
 }
 
 __global__ void k_lookup(DevGraph g, OpView ops, uint64_t nops, int create) {
@@ -262,24 +267,66 @@ void storage_free(Graph &g) {
   g.ops = nullptr; g.stage_dev = nullptr; g.stage_host = nullptr;
 }
 
-int stage_edges(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, int directed, uint64_t *nops) {
-  uint64_t k = directed ? n : 2 * n;
-  *nops = k;
-  int rc = ensure_ops(g, k, n);
-  if (rc) return rc;
-  size_t bytes = pairs ? n * 16 : n * sizeof(rg_edge);
-  if ((rc = ensure_stage(g, bytes))) return rc;
-  if (n == 0) return RG_OK;
-  std::memcpy(g.stage_host, pairs ? (const void *)pairs : (const void *)edges, bytes);
-  RG_CUDA(cudaMemcpyAsync(g.stage_dev, g.stage_host, bytes, cudaMemcpyHostToDevice, g.stream));
-  OpView ops = op_view(g);
+// Staging buffers hold a batch as 32-bit records (rg_stage.c).  A submission of
+// two batches keeps the second one after the first.
+static uint64_t stage_bytes(const Graph &g, bool pairs, uint64_t n) {
+  return (n * (g.weighted && !pairs ? 12 : 8) + 255) & ~255ull;
+}
+constexpr uint64_t STAGE_STEP = 1ull << 18;  // edges packed between two copies
+
+int stage_reserve(Graph &g, bool pairs, uint64_t n1, uint64_t n2) {
+  return ensure_stage(g, stage_bytes(g, pairs, n1) + stage_bytes(g, pairs, n2));
+}
+
+int stage_copy(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, uint64_t after, int *flags) {
+  const uint64_t words = g.weighted && !pairs ? 3 : 2, at = stage_bytes(g, pairs != nullptr, after);
+  uint32_t *host = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_host) + at);
+  uint32_t *dev = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_dev) + at);
+  *flags = 0;
+  for (uint64_t b = 0; b < n; b += STAGE_STEP) {
+    const uint64_t m = std::min(STAGE_STEP, n - b);
+    *flags |= pairs ? rg_stage_pairs(pairs + 2 * b, m, g.V, host + words * b)
+                    : rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, host + words * b);
+    if (*flags) return RG_OK;
+    RG_CUDA(cudaMemcpyAsync(dev + words * b, host + words * b, m * words * 4, cudaMemcpyHostToDevice, g.stream));
+  }
+  return RG_OK;
+}
+
+int stage_unpack(Graph &g, bool pairs, uint64_t n, uint64_t after, int directed, uint64_t *nops) {
+  *nops = directed ? n : 2 * n;
+  int rc = ensure_ops(g, *nops, n);
+  if (rc || n == 0) return rc;
+  const char *dev = static_cast<const char *>(g.stage_dev) + stage_bytes(g, pairs, after);
   count_launch(g);
-  if (pairs)
-    k_unpack_pairs<<<grid_for(g, n), TPB, 0, g.stream>>>((const uint64_t *)g.stage_dev, n, directed, g.weighted, ops);
-  else
-    k_unpack_edges<<<grid_for(g, n), TPB, 0, g.stream>>>((const rg_edge *)g.stage_dev, n, directed, g.weighted, ops);
+  k_unpack<<<grid_for(g, n), TPB, 0, g.stream>>>(reinterpret_cast<const uint32_t *>(dev), n, directed, g.weighted,
+                                                 pairs ? 1 : 0, op_view(g));
   RG_CUDA(cudaGetLastError());
   return RG_OK;
+}
+
+// A checked batch, or its weights' codes (device_edges), packed and copied.
+static int stage_trusted(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, uint64_t after) {
+  const uint64_t words = g.weighted && !pairs ? 3 : 2, at = stage_bytes(g, pairs != nullptr, after);
+  uint32_t *host = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_host) + at);
+  uint32_t *dev = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_dev) + at);
+  for (uint64_t b = 0; b < n; b += STAGE_STEP) {
+    const uint64_t m = std::min(STAGE_STEP, n - b);
+    if (pairs) rg_stage_pairs(pairs + 2 * b, m, g.V, host + words * b);
+    else rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, host + words * b);
+    RG_CUDA(cudaMemcpyAsync(dev + words * b, host + words * b, m * words * 4, cudaMemcpyHostToDevice, g.stream));
+  }
+  return RG_OK;
+}
+
+int stage_coded(Graph &g, const rg_edge *edges, uint64_t n, uint64_t after) {
+  return stage_trusted(g, edges, nullptr, n, after);
+}
+
+int stage_edges(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n, int directed, uint64_t *nops) {
+  int rc = stage_reserve(g, pairs != nullptr, n, 0);
+  if (!rc) rc = stage_trusted(g, edges, pairs, n, 0);
+  return rc ? rc : stage_unpack(g, pairs != nullptr, n, 0, directed, nops);
 }
 
 static int grow_dir(Graph &g, DevDir &dir, int which) {

@@ -48,20 +48,6 @@ __device__ __forceinline__ void put_ops(OpView ops, uint64_t i, uint32_t s, uint
   }
 }
 
-__device__ __forceinline__ void unpack_edge(const rg_edge *e, uint64_t i, int directed, int weighted, OpView ops) {
-  uint32_t s = (uint32_t)e[i].src, d = (uint32_t)e[i].dst, w = weighted ? (uint32_t)e[i].data : 0u;
-  put_ops(ops, i, s, d, w, directed);
-}
-
-// Reference file format pairs; weights are the pure function of the endpoints
-// used by every implementation here (splitmix64(src<<32|dst) % 255 + 1).
-__device__ __forceinline__ void unpack_pair(const uint64_t *p, uint64_t i, int directed, int weighted, OpView ops) {
-  uint64_t s64 = p[2 * i], d64 = p[2 * i + 1];
-  uint32_t s = (uint32_t)s64, d = (uint32_t)d64;
-  uint32_t w = weighted ? (uint32_t)(splitmix64((s64 << 32) | d64) % 255 + 1) : 0u;
-  put_ops(ops, i, s, d, w, directed);
-}
-
 // Find the record of op j's (s,d,w); create it (and reserve its slots at the
 // end of the src / dst segments) when `create`.  Vertices whose segment just
 // ran out of capacity go to the direction's grow list.  Lanes of a warp that

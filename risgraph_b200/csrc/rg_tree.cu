@@ -1490,7 +1490,7 @@ __device__ __forceinline__ void tiny_levels(const DevGraph &g, uint32_t *q_in, u
   unsigned long long *cur_n = n_in, *nxt_n = n_out;
   unsigned long long local = 0, scanned = 0;
   for (bool first = true;; first = false) {
-    const uint64_t n = __ldcg(cur_n);
+    const uint64_t n = *cur_n;
     // stage the frontier and its degree prefix
     uint32_t d = 0;
     if (n <= TINY_N && tid < n) {
@@ -1556,7 +1556,7 @@ __device__ __forceinline__ void tiny_levels(const DevGraph &g, uint32_t *q_in, u
     nxt_n = tn;
   }
   if (cur != q_final) {
-    const uint64_t n = __ldcg(cur_n);
+    const uint64_t n = *cur_n;
     for (uint64_t i = tid; i < n; i += TINY_TPB) q_final[i] = cur[i];
     __syncthreads();
     if (tid == 0) *n_final = n;
@@ -2633,20 +2633,20 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
     // or in the reset set once the levels are done, goes to the grid-wide repair
     int heavy = 0;
     {
-      const uint64_t n0 = __ldcg(cur_n);
+      const uint64_t n0 = *cur_n;
       if (n0 && n0 <= DEL_TINY_N) {
         for (uint64_t i = tid; i < n0; i += DT_TPB)
           heavy |= seg_len(g.in, cur[i]) > HEAVY_DEG || seg_len(g.out, cur[i]) > HEAVY_DEG;
       } else if (n0 == 0) {
-        const uint64_t tn = __ldcg(&c[C_TREEN]);
+        const uint64_t tn = c[C_TREEN];
         if (tn <= DEL_TINY_TREE)
           for (uint64_t i = tid; i < tn; i += DT_TPB) heavy |= seg_len(g.in, tree[i]) > HEAVY_DEG;
       }
     }
     heavy = __syncthreads_or(heavy);
     if (tid == 0) {
-      const uint64_t n = __ldcg(cur_n), tree_n = __ldcg(&c[C_TREEN]);
-      bool rec = __ldcg(&c[C_RECOMPUTE]) != 0;
+      const uint64_t n = *cur_n, tree_n = c[C_TREEN];
+      bool rec = c[C_RECOMPUTE] != 0;
       int go = 1;  // 1: run this level; 0: invalidation done; 2: hand over
       if (n == 0 || rec) {
         go = 0;
@@ -2671,7 +2671,7 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
     }
     __syncthreads();
     if (s_go != 1) break;
-    const uint64_t n = __ldcg(cur_n);
+    const uint64_t n = *cur_n;
     rescue_warps<A, W>(g, cur, n, limit, warp, nwarps);
     __syncthreads();
     expand_warps<A, W>(g, cur, n, tree, nxt, nxt_n, warp, nwarps);
@@ -2686,7 +2686,7 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
   if (s_go == 2) {
     // the multi-CTA repair continues from queue 0
     if (cur != q0) {
-      const uint64_t n = __ldcg(cur_n);
+      const uint64_t n = *cur_n;
       for (uint64_t i = tid; i < n; i += DT_TPB) q0[i] = cur[i];
       __syncthreads();
       if (tid == 0) c[C_QN0] = n;
@@ -2697,7 +2697,7 @@ __device__ __forceinline__ bool del_tiny_levels(const DevGraph &g, uint32_t *q0,
   unsigned long long local = 0;
   const bool recompute = s_rec != 0;
   if (!recompute) {
-    const uint64_t tn = __ldcg(&c[C_TREEN]);
+    const uint64_t tn = c[C_TREEN];
     reset_warps<A>(g, tree, tn, mst, warp, nwarps);
     __syncthreads();
     local = pull_warps<A, W>(g, tree, tn, mst, warp, nwarps);
@@ -2817,16 +2817,15 @@ template <int A, bool W>
 __device__ __forceinline__ int batch_repair(const DevGraph &g, const FusedRepair &fr, int add, uint32_t *q0,
                                             uint32_t mst, unsigned long long *tr) {
   unsigned long long *c = g.ctl;
-  // (every thread takes the same branch: thread 0 looks)
-  auto open = [&]() { return __syncthreads_or(threadIdx.x == 0 && __ldcg(&c[C_QN0]) && !__ldcg(&c[C_ERR])) != 0; };
-  bool over = false, left = open();
-  if (left) {
+  bool over = false;
+  if (c[C_QN0] && !c[C_ERR]) {
     if (!add) over = del_tiny_levels<A, W>(g, q0, fr.q1, fr.tree, fr.limit, fr.big, fr.max_iter, mst);
     if (tr && threadIdx.x == 0) tr[RG_PH_DELREPAIR] = global_ns();
-    if (!over && fr.tiny_edges && open())
+    if (!over && fr.tiny_edges && c[C_QN0])
       tiny_levels<A, W>(g, q0, &c[C_QN0], fr.q1, &c[C_QN1], q0, &c[C_QN0], fr.max_levels, fr.tiny_edges, mst, false);
-    left = open() || over;
   }
+  const bool left = over || (c[C_QN0] && !c[C_ERR]);
+  __syncthreads();  // every thread has read the counts before the next batch resets them
   if (threadIdx.x == 0) {
     c[C_OVER] = over ? 1 : 0;
     c[C_QN1] = 0;  // (the engine's first output count)
