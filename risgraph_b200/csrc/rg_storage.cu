@@ -48,7 +48,7 @@ __global__ void k_unpack(const uint32_t *r, uint64_t n, int directed, int weight
 }
 
 __global__ void k_lookup(DevGraph g, OpView ops, uint64_t nops, int create) {
-  GRID_STRIDE(j, nops) lookup_op(g, ops, j, create);
+  GRID_STRIDE(j, nops) lookup_op<1>(g, ops, j, create, g.rec_top);
 }
 
 // One CTA per growing vertex.

@@ -2845,6 +2845,7 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, const sdev::OpView
                                            uint32_t *q0, uint32_t mst, int second, const FusedRepair &fr,
                                            uint4 *scratch, const uint64_t *inl = nullptr) {
   __shared__ int s_skip;
+  __shared__ unsigned long long s_rec_top;  // (no other CTA creates records meanwhile)
   unsigned long long *c = g.ctl;
   const unsigned tid = threadIdx.x;
   // phase trace (RG_OPT_PHASE_TRACE): thread 0 stamps the device clock
@@ -2856,6 +2857,7 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, const sdev::OpView
     // the second batch of a submission does nothing after an error in the first
     s_skip = second && c[C_ERR] != 0;
     if (!s_skip) {
+      s_rec_top = *g.rec_top;
       const unsigned long long kl = c[C_KLAUNCH];
       prologue_ctl(c, sb.inv_tag, second ? nullptr : &sb.stamp);
       if (second) c[C_KLAUNCH] = kl;  // the count covers the whole submission
@@ -2894,8 +2896,13 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, const sdev::OpView
   }
   __syncthreads();
   stamp(RG_PH_UNPACK);
-  for (uint64_t j = tid; j < nops; j += FS_TPB) sdev::lookup_op(g, ops, j, add);
+  if (add) {
+    for (uint64_t j = tid; j < nops; j += FS_TPB) sdev::lookup_op<4>(g, ops, j, 1, &s_rec_top);
+  } else {
+    for (uint64_t j = tid; j < nops; j += FS_TPB) sdev::lookup_op<1>(g, ops, j, 0, &s_rec_top);
+  }
   __syncthreads();
+  if (add && tid == 0) *g.rec_top = s_rec_top;
   stamp(RG_PH_LOOKUP);
   if (add) {
     // each warp grows its own vertices (a vertex is in a grow list once); the
