@@ -250,12 +250,16 @@ int rg_phase_trace(rg_graph *g, uint64_t *ns);
  *                         default 16; 0: never) travel inside the kernel's
  *                         launch parameters instead of a staging buffer that
  *                         the kernel reads across the bus.
- *   RG_OPT_CLUSTER_EDGES  frontiers too large for one CTA but of at most 16 x
- *                         1024 vertices (8 x 1024 where the GPU schedules no
- *                         16-CTA cluster) and this many out-slots (default
- *                         65536, at most 2^20; 0: never) run their levels in
- *                         one thread-block cluster, one launch for successive
- *                         levels; a frontier that a tiny level could take goes
+ *   RG_OPT_CLUSTER_EDGES  0: tree calls run the graph-driven level loop, one
+ *                         launch or more per level (what served graphs do);
+ *                         otherwise (default 65536, at most 2^20) the levels
+ *                         and deletion repairs of a call run in one persistent
+ *                         launch over all SMs.  In profile mode, which steps
+ *                         the levels from the host, frontiers too large for
+ *                         one CTA but of at most 16 x 1024 vertices (8 x 1024
+ *                         where the GPU schedules no 16-CTA cluster) and this
+ *                         many out-slots run in one thread-block cluster; a
+ *                         frontier that a tiny level could take goes
  *                         to the cluster when it has more than 4096 slots. */
 typedef enum {
   RG_OPT_DENSE_PULL = 0,
@@ -374,9 +378,9 @@ int rg_server_create(uint64_t hbm_budget_bytes, double target_epoch_ms, uint64_t
                      rg_server **out);
 /* Admit a graph (labels already built with rg_build_tree for `algo`).
  * RG_ENOMEM_HBM when its device bytes would exceed the budget.  While
- * attached the graph runs no cluster levels (RG_OPT_CLUSTER_EDGES reads 0;
- * detach gives the value back): with other instances' epochs on the GPU a
- * level that needs a GPC of free SMs at once would wait for them. */
+ * attached the graph runs the graph-driven level loop (RG_OPT_CLUSTER_EDGES
+ * reads 0; detach gives the value back): with other instances' epochs on the
+ * GPU a launch that needs every SM would wait for them. */
 int rg_server_attach(rg_server *s, rg_graph *g, int algo, int directed, uint32_t *instance);
 int rg_server_detach(rg_server *s, uint32_t instance);
 /* Record the label history (rg_history_record of the modified vertices) after

@@ -141,7 +141,7 @@ extern "C" int rg_autotune(rg_graph *g, int algo, uint64_t root, const rg_edge *
   if ((rc = t.tune(RG_OPT_LBS_MIN, {512, 2048, 8192, 32768, 131072}, &Tuner::build_ms, &ms))) return rc;
   // small-frontier knob: builds and the sample's round trips together
   if ((rc = t.tune(RG_OPT_TINY_EDGES, {0, 8192, 32768, 131072}, &Tuner::both_ms, &ms))) return rc;
-  // mid-size frontiers in one thread-block cluster: builds and round trips together
+  // graph-driven loop (0) or grid engine: builds and round trips together
   if ((rc = t.tune(RG_OPT_CLUSTER_EDGES, {0, 16384, 65536, 262144}, &Tuner::both_ms, &ms))) return rc;
   if ((rc = t.build_ms(&out->build_ms_after))) return rc;
   if ((rc = t.apply_ms(&out->apply_ms_after))) return rc;

@@ -351,7 +351,7 @@ struct Graph {
   uint64_t fused_max = 2048;
   int phase_trace = 0;            // RG_OPT_PHASE_TRACE
   uint64_t inline_max = 16;       // RG_OPT_INLINE_MAX: largest fused batch passed in the launch parameters
-  uint64_t cluster_edges = 65536;  // RG_OPT_CLUSTER_EDGES: out-slot limit of a cluster level (0: off)
+  uint64_t cluster_edges = 65536;  // RG_OPT_CLUSTER_EDGES: 0: no grid engine, else also the out-slot limit of a cluster level
   int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
   unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
   bool ctl_on_host = false;         // the last launch writes the control block to h_ctl itself

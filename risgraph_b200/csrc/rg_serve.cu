@@ -389,9 +389,10 @@ int rg_server_attach(rg_server *s, rg_graph *g, int algo, int directed, uint32_t
     in->id = (uint32_t)s->inst.size();
     s->inst.push_back(in);
   }
-  // No cluster levels while served: the epochs of other instances keep SMs
-  // busy, and a level that needs a whole GPC's worth of free SMs at once then
-  // waits for them (p99 went from 0.4 to 4 ms in the six-instance mix).
+  // The graph-driven level loop while served (option value 0): the epochs of
+  // other instances keep SMs busy, and a launch that needs many SMs at once then
+  // waits for them (16-SM clusters alone took p99 from 0.4 to 4 ms in the
+  // six-instance mix; the grid engine needs every SM).
   in->cluster_edges = g->g.cluster_edges;
   g->g.cluster_edges = 0;
   Instance *raw = in.get();

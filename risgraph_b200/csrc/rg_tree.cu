@@ -1576,6 +1576,8 @@ __global__ void __launch_bounds__(TINY_TPB) k_push_tiny(DevGraph g, uint32_t *q_
 }
 
 // ---- cluster levels ------------------------------------------------------------
+// (Levels of the host-stepped loop, and of the graph-driven one on a GPU that
+// launches no cooperative grid; the grid engine runs the others.)
 // A frontier too large for one CTA but at most CL_TPB vertices per CTA of a
 // thread-block cluster (16 CTAs where the GPU schedules a cluster that size,
 // else 8; one per SM) runs in k_push_cluster: successive levels inside one
