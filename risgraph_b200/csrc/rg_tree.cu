@@ -3152,14 +3152,19 @@ __device__ __forceinline__ int fast_inline(const DevGraph &g, const InlineBatch 
       const uint32_t dead = is_ins ? 0u : DEAD;
       if (ro < cap_o) put(po + ro, d | dead, w);
       if (!g.symmetric && ri < cap_i) put(pi + ri, s | dead, w);
-      seed = is_ins ? better_now : lab.y == pack_parent(s, w);
     }
   }
   if (is_ins && made && lane == 0) *g.rec_top = top + made;
-  if (go && on && old_host) {
-    // both orientations of an undirected edge count alike
-    if (directed) old_host[lane] = old;
-    else if (!(lane & 1)) old_host[lane >> 1] = old;
+  if (go) {
+    // The count that comes back and makes the edge a candidate, as in edge_old:
+    // an undirected edge's is that of the orientation with the lower source
+    // (they differ where directed updates came before).
+    const uint32_t ways = __shfl_sync(FULL, old, directed ? lane : (lane & ~1u) + (((lane & 1) != 0) == (s < d)));
+    if (on && old_host) {
+      if (directed) old_host[lane] = ways;
+      else if (!(lane & 1)) old_host[lane >> 1] = ways;
+    }
+    seed = on && (is_ins ? ways == 0 && better_now : ways == 1 && lab.y == pack_parent(s, w));
   }
   // 4. seeds
   if (is_ins && seeds_ins) {
