@@ -1743,6 +1743,7 @@ __device__ __forceinline__ void prologue_words(unsigned long long *c, unsigned l
   c[C_EDGES] = 0;
   c[C_MODE] = M_EMPTY;
   c[C_KLAUNCH] = 0;
+  c[C_PULLED] = 0;
   c[C_HVR] = 0;
   c[C_HVE] = 0;
   c[C_HVP] = 0;
@@ -1834,7 +1835,9 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   const bool dense = n * cfg.dense_div >= g.V;
   unsigned long long mode = M_SPARSE;
   if (n == 0) mode = M_EMPTY;
-  else if (cfg.bottom_up && n * cfg.bu_div >= g.V) mode = M_BOTTOM_UP;
+  // (a pull level commits values deeper than the level, which a bottom-up level,
+  // looking for parents of one depth, would miss: none follows a pull)
+  else if (cfg.bottom_up && !c[C_PULLED] && n * cfg.bu_div >= g.V) mode = M_BOTTOM_UP;
   // pull once the frontier passes |V| / pull_div, and keep pulling until it
   // falls below 4x that (the frontier's first large levels are hub-heavy, its
   // last ones are not: the direction switch of Beamer et al., by vertex count)
@@ -1844,6 +1847,7 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   else if (dense) mode = M_DENSE_PUSH;
   else if (n >= cfg.lbs_min) mode = M_LBS;
   if (mode == M_DENSE_PUSH) c[C_ACT] += 1;
+  if (mode == M_PULL) c[C_PULLED] = 1;
   c[C_MODE] = mode;
   // bounds on the frontiers' values: pull levels collect theirs, others give none
   const int half = fin_n == &c[C_QN0] ? 0 : 1;
@@ -3765,7 +3769,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   }
   if (!grid_sync(g, bar)) return;
   if (a.del && !eng_del<A, W>(g, a, bar)) return;
-  bool pulled = false;
+  bool pulled = false, any_pull = false;  // the level before, any level before
   for (uint32_t k = 0;; k++) {
     const uint32_t *fin = a.q[k & 1];
     uint32_t *fout = a.q[(k & 1) ^ 1];
@@ -3790,7 +3794,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     }
     // the mode rules of k_level_begin, and a pull in place of a push that
     // would relax a large part of the graph
-    const bool bu = a.cfg.bottom_up && n * a.cfg.bu_div >= g.V;
+    const bool bu = a.cfg.bottom_up && !any_pull && n * a.cfg.bu_div >= g.V;
     bool pull = !bu && a.cfg.allow_pull && n * (pulled ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
     if (bu) {
       eng_bottom_up<W>(g, sh, lvl, fout, fout_n);
@@ -3847,6 +3851,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       }
     }
     pulled = pull;
+    any_pull = any_pull || pull;
     lvl++;
     if (!grid_sync(g, bar)) return;
   }
