@@ -3499,9 +3499,10 @@ __device__ __forceinline__ void eng_share(uint64_t S, uint64_t &e0, uint64_t &e1
 // Deletion repair over the whole grid (do_update_tree_del,
 // core/graph.hpp:1250-1511): the phases of k_rescue, k_expand, k_reset and
 // k_pull, each followed by the tasks of the long lists it met.
-// Leaves the reset set in queue 0 with its count in ctl[C_QN0].
+// Leaves the reset set in queue 0 with its count in ctl[C_QN0].  done: the
+// invalidation levels that the one-CTA repair ran before it handed over.
 template <int A, bool W>
-__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar) {
+__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar, uint64_t done) {
   unsigned long long *c = g.ctl;
   unsigned long long *hvr = a.bar + EB_HVR, *hve = a.bar + EB_HVE;  // two words each, by turns
   auto cnt = [&](uint64_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
@@ -3509,18 +3510,18 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
   const uint64_t nwarps = ((uint64_t)gridDim.x * ENG_TPB) >> 5;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   bool recompute = false;
-  for (uint64_t it = 0; it < a.max_iter; it++) {
+  for (uint64_t it = 0; done + it < a.max_iter; it++) {
     const uint32_t *fin = a.q[it & 1];
     uint32_t *fout = a.q[(it & 1) ^ 1];
     const uint64_t n = __ldcg(cnt(it));
     if (n == 0) break;
-    if (it <= 10 && __ldcg(&c[C_TREEN]) + n > a.big) {  // core/graph.hpp:1252
+    if (done + it <= 10 && __ldcg(&c[C_TREEN]) + n > a.big) {  // core/graph.hpp:1252
       recompute = true;
       break;
     }
     if (lead) {
       *cnt(it + 2) = 0;
-      c[C_INVITER] = it + 1;
+      c[C_INVITER] = done + it + 1;
     }
     RepQueue rq;
     rq.task = a.task;
@@ -3757,6 +3758,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   // what the launch before left, read before anything below may change it
   uint32_t st = (uint32_t)__ldcg(&c[C_STAMP]);
   uint64_t lvl = a.build ? 0 : __ldcg(&c[C_LEVEL]);
+  const uint64_t inv_levels = a.del ? __ldcg(&c[C_INVITER]) : 0;
   if (lead) a.bar[EB_QN2] = a.bar[EB_HVR] = a.bar[EB_HVE] = 0;
   if (a.build) {
     init_labels<A>(g, a.root, a.q[0], blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB);
@@ -3768,7 +3770,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     }
   }
   if (!grid_sync(g, bar)) return;
-  if (a.del && !eng_del<A, W>(g, a, bar)) return;
+  if (a.del && !eng_del<A, W>(g, a, bar, inv_levels)) return;
   bool pulled = false, any_pull = false;  // the level before, any level before
   for (uint32_t k = 0;; k++) {
     const uint32_t *fin = a.q[k & 1];
