@@ -355,6 +355,7 @@ struct Graph {
   uint64_t cluster_edges = 65536;  // RG_OPT_CLUSTER_EDGES: 0: no grid engine, else also the out-slot limit of a cluster level
   int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
   unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
+  uint32_t wait_polls = 1u << 24;   // polls before one of its waits gives up (ten seconds or more)
   bool ctl_on_host = false;         // the last launch writes the control block to h_ctl itself
   int cl_ctas = 0;                  // CTAs of the cluster kernel (16 where the GPU schedules it, else 8)
   unsigned long long *ptrace_buf = nullptr;  // its device buffer (allocated with the labels)
@@ -478,6 +479,9 @@ int tree_after_sync(Graph &g, int what, uint64_t *total);
 int tree_classify(Graph &g, uint64_t n_edges, int directed, const uint8_t *is_del_dev, uint8_t *unsafe_dev);
 int tree_labels(Graph &g, uint64_t *val, uint64_t *par, uint64_t *pw);
 int tree_checksum(Graph &g, uint64_t *sum);
+// What a launch of the grid engine that gave up leaves behind, put right (after
+// the stream was waited for).
+void engine_reset(Graph &g);
 int tree_alloc(Graph &g);
 // Fused small-batch apply (n <= SMALL_EDGES): storage update, candidate
 // selection and seeding in one single-CTA kernel, the repair loops behind a

@@ -466,6 +466,7 @@ int sync_ctl(Graph &g) {
     RG_CUDA(cudaStreamSynchronize(g.stream));
     if (g.h_ctl[C_KLAUNCH] != CTL_PENDING) return RG_OK;
     // (the engine gave up before its end: the reason is in the device's copy)
+    engine_reset(g);
   }
   RG_CUDA(cudaMemcpyAsync(g.h_ctl, g.d.ctl, sizeof(unsigned long long) * C_COUNT, cudaMemcpyDeviceToHost, g.stream));
   RG_CUDA(cudaStreamSynchronize(g.stream));
@@ -480,7 +481,7 @@ int storage_error(Graph &g) {
                                 : "device error");
   cudaMemsetAsync(&g.d.ctl[C_ERR], 0, 8, g.stream);
   cudaMemsetAsync(&g.d.ctl[C_AUX], 0, 8, g.stream);
-  if (code == RG_ETIMEOUT) cudaMemsetAsync(g.eng_bar, 0, EB_WORDS * 8, g.stream);  // (left half counted)
+  if (code == RG_ETIMEOUT) engine_reset(g);
   return code;
 }
 

@@ -3366,7 +3366,6 @@ constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alo
 // entries (RMAT-22 SSWP: the push of 97K vertices took 241 us, a pull level 75)
 constexpr uint64_t ENG_PULL_DIV = 12;
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
-constexpr uint32_t ENG_SPINS = 1u << 24;     // polls before a barrier gives up (ten seconds or more)
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
 static_assert(TASK_SLOTS >= CHUNK && TASK_DEG >= 2 * TASK_SLOTS, "the hub task queue holds the tasks");
@@ -3389,6 +3388,7 @@ struct EngineArgs {
   uint64_t limit, big, max_iter;  // deletion repairs
   LevelCfg cfg;
   uint32_t mst;
+  uint32_t polls;               // before a wait gives up
   int build;                    // initialise the labels first
   int del;                      // repair deletions from the invalidated frontier in queue 0 first
 };
@@ -3396,14 +3396,19 @@ struct EngineArgs {
 struct GridBar {
   unsigned long long *w;
   unsigned gen;  // thread 0's
+  uint32_t polls;
 };
 
-// All CTAs of the grid; false when the wait gave up (the caller returns).
+// All CTAs of the grid; false when the wait gave up (the caller returns).  A
+// CTA that gives up has arrived, so the others may run the phase after this
+// barrier, but none gets past the next one: what that phase lacks is not read.
+// quiet: giving up is no error (the last barrier, for all CTAs but the one that
+// still has work after it).
 // A CTA may leave a barrier long before another one has looked at what it
 // decides on next, so a word that every CTA reads after a barrier is written
 // again only past the barrier after that: counters and flags of successive
 // levels alternate between words.
-__device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b) {
+__device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b, bool quiet = false) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -3418,9 +3423,9 @@ __device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b) {
       unsigned x, spins = 0;
       do {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(gen) : "memory");
-      } while (x == b.gen && ++spins < ENG_SPINS);
+      } while (x == b.gen && ++spins < b.polls);
       if (x == b.gen) {
-        atomicCAS(&g.ctl[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
+        if (!quiet) atomicCAS(&g.ctl[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
         ok = 0;
       }
     }
@@ -3753,7 +3758,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   unsigned long long *bnd = a.bar + EB_BND;
   auto cnt = [&](uint32_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-  GridBar bar = {a.bar, 0u};
+  GridBar bar = {a.bar, 0u, a.polls};
   if (threadIdx.x == 0) bar.gen = *reinterpret_cast<volatile unsigned *>(a.bar + EB_GEN);
   // what the launch before left, read before anything below may change it
   uint32_t st = (uint32_t)__ldcg(&c[C_STAMP]);
@@ -3858,7 +3863,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     if (!grid_sync(g, bar)) return;
   }
   counts_out(g, &sh.bc);
-  if (!grid_sync(g, bar)) return;  // (every CTA has read the last queue counts)
+  if (!grid_sync(g, bar, blockIdx.x != 0)) return;  // (every CTA has read the last queue counts)
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
       c[C_QN0] = 0;
@@ -4583,6 +4588,7 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
   a.big = recompute_threshold(g);
   a.max_iter = (uint64_t)g.V + 2;
   a.mst = mod_stamp(g);
+  a.polls = g.wait_polls;
   a.build = build ? 1 : 0;
   a.del = del ? 1 : 0;
   g.h_ctl[C_KLAUNCH] = CTL_PENDING;
@@ -4655,8 +4661,7 @@ int after_sync(Graph &g, int what) {
   if (g.h_ctl[C_ERR]) {
     int code = (int)g.h_ctl[C_ERR];
     set_error(code == RG_ETIMEOUT ? "push levels did not converge" : "device error in tree update");
-    // (a barrier of the engine that gave up is left half counted)
-    cudaMemsetAsync(g.eng_bar, 0, EB_WORDS * 8, g.stream);
+    if (code == RG_ETIMEOUT) engine_reset(g);
     cudaMemsetAsync(&g.d.ctl[C_ERR], 0, 8, g.stream);
     return code;
   }
@@ -4766,6 +4771,14 @@ static void engine_setup(Graph &g) {
                     engine_fits<RG_WCC, false>(g) && engine_fits<RG_WCC, true>(g);
   g.eng_ctas = fits ? std::min(g.num_sms, ENG_MAX_CTAS) : 0;
   cudaGetLastError();
+}
+
+void engine_reset(Graph &g) {
+  // a barrier left half counted, stamps past the one in the control block, hubs'
+  // best pieces that no pull_hub_fix took
+  cudaMemsetAsync(g.eng_bar, 0, EB_WORDS * 8, g.stream);
+  cudaMemsetAsync(g.d.stamp, 0, g.V * 4 + 4, g.stream);
+  if (g.sell_hub_best) cudaMemsetAsync(g.sell_hub_best, 0xff, g.sell_hub_cap * 8, g.stream);
 }
 
 int tree_alloc(Graph &g) {
