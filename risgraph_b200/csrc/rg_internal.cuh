@@ -75,7 +75,8 @@ enum Ctl : int {
   C_OVER = 30,     // the fused apply's one-CTA deletion repair handed over to the grid-wide one
   C_LEFT = 31,     // what a fused kernel left to the host (1: insert batch's level loop [and the delete batch], 2: delete batch's repair)
   C_PULLED = 32,   // a level of the current loop pulled
-  C_COUNT = 33
+  C_BEAT = 33,     // counts up while long serial work goes on (see has_parents)
+  C_COUNT = 34
 };
 
 enum LevelMode : unsigned long long {

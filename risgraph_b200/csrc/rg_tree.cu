@@ -103,6 +103,12 @@ __device__ __forceinline__ void warp_add_result(unsigned long long local, unsign
   if (lane_id() == 0 && local) atomicAdd(dst, local);
 }
 
+// Serial work without a bound of its own that matters (a walk up a deep tree, a
+// warp's search of a vertex's whole list) beats every BEAT_STEPS steps, which
+// tells the CTAs that wait at the grid engine's barrier that it goes on.
+constexpr uint32_t BEAT_STEPS = 256;
+__device__ __forceinline__ void beat(const DevGraph &g) { atomicAdd(&g.ctl[C_BEAT], 1ull); }
+
 // Record v in the modified list (trace_modified graphs); the epoch is read
 // from the control block so cached graphs follow rg_clear_modified.
 __device__ __forceinline__ void mark_modified(const DevGraph &g, bool pred, uint32_t v, uint32_t /*on*/) {
@@ -1414,6 +1420,7 @@ __device__ __forceinline__ void bottom_up(const DevGraph &g, uint64_t d, uint32_
 #pragma unroll
         for (int i = 0; i < 2; i++) ok[i] = k + 32 * i + lane < n && is_parent(P_::nbr(e[i]));
         if (lane == l) scanned += min(64u, n - k);
+        if ((k - BU_ALONE) / 64 % BEAT_STEPS == BEAT_STEPS - 1 && lane == 0) beat(g);
         const unsigned hit = __ballot_sync(FULL, ok[0] || ok[1]);
         if (hit) {
           const int h = __ffs(hit) - 1;
@@ -2024,6 +2031,10 @@ __global__ void k_seed_del(DevGraph g, const uint32_t *os, const uint32_t *od, c
 //
 // The three words of a step are loaded together, so that a step costs one
 // round trip to memory rather than three.
+//
+// On a deep tree the walks of one lane can take many seconds: every BEAT_STEPS
+// steps a walk beats, and ends if the repair has already asked for a recompute
+// (which makes its answer void).
 __device__ __forceinline__ bool has_parents(const DevGraph &g, uint32_t x0, uint32_t tag_inv, uint64_t limit) {
   uint64_t num = 0;
   uint32_t x = x0;
@@ -2038,6 +2049,10 @@ __device__ __forceinline__ bool has_parents(const DevGraph &g, uint32_t x0, uint
     if (++num > limit) {
       atomicExch(&g.ctl[C_RECOMPUTE], 1ull);
       return true;
+    }
+    if (num % BEAT_STEPS == 0) {
+      if (__ldcg(&g.ctl[C_RECOMPUTE])) return true;
+      beat(g);
     }
   }
   x = x0;
@@ -3402,6 +3417,7 @@ struct GridBar {
 // All CTAs of the grid; false when the wait gave up (the caller returns).  A
 // CTA that gives up has arrived, so the others may run the phase after this
 // barrier, but none gets past the next one: what that phase lacks is not read.
+// It gives up after b.polls polls without a beat from the work that it waits for.
 // quiet: giving up is no error (the last barrier, for all CTAs but the one that
 // still has work after it).
 // A CTA may leave a barrier long before another one has looked at what it
@@ -3421,9 +3437,16 @@ __device__ __forceinline__ bool grid_sync(const DevGraph &g, GridBar &b, bool qu
       atomicExch(gen, b.gen + 1);
     } else {
       unsigned x, spins = 0;
-      do {
+      unsigned long long beats = 0;
+      for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(gen) : "memory");
-      } while (x == b.gen && ++spins < b.polls);
+        if (x != b.gen) break;
+        if (++spins < b.polls) continue;
+        const unsigned long long now = __ldcg(&g.ctl[C_BEAT]);
+        if (now == beats) break;
+        beats = now;
+        spins = 0;
+      }
       if (x == b.gen) {
         if (!quiet) atomicCAS(&g.ctl[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
         ok = 0;

@@ -85,3 +85,43 @@ def test_a_stopped_repair_leaves_nothing_behind(algo):
     assert stopped > 0
     g.close()
     h.close()
+
+
+def test_a_long_walk_up_the_tree_is_waited_for():
+    """The rescue of one vertex walks 20,000 parents, several times the wait limit set here, while the other CTAs wait."""
+    hops, V = 20_000, 250_000
+    a, b = 1 + np.arange(hops), 1 + hops + np.arange(hops)
+    t = 2 * hops + 1
+    chains = [np.stack([np.concatenate([[0], c[:-1]]), c], 1) for c in (a, b)]
+    pairs = np.concatenate(chains + [[[a[-1], t], [b[-1], t]]]).astype(np.uint64)
+    g = rg.Graph(V, len(pairs))
+    g.add_pairs(pairs, want_old=False)
+    g.set_option("fused_max", 0)   # the repair goes to the grid
+    g.build_tree("bfs", 0)
+    before, par, _ = g.labels()
+    assert before[t] == hops + 1
+    e = np.zeros(1, rg.EDGE_DTYPE)
+    e["src"], e["dst"] = par[t], t
+    set_polls(g, 1 << 12)
+    g.apply_del("bfs", e)
+    val, now, _ = g.labels()
+    np.testing.assert_array_equal(val, before)
+    assert now[t] == (b[-1] if par[t] == a[-1] else a[-1])
+    assert g.last_stats()["recomputes"] == 0
+    g.close()
+
+
+def test_a_long_list_in_a_bottom_up_level_is_waited_for():
+    """A vertex with three million in-edges, none from the frontier: one warp searches them while the grid waits."""
+    front, many = 50_000, 3_000_000
+    hub = 1 + front
+    pairs = np.concatenate([np.stack([np.zeros(front, int), 1 + np.arange(front)], 1),
+                            np.stack([hub + 1 + np.arange(many), np.full(many, hub)], 1)]).astype(np.uint64)
+    V = hub + 1 + many
+    g = rg.Graph(V, len(pairs))
+    g.add_pairs(pairs, want_old=False)
+    set_polls(g, 1 << 12)
+    g.build_tree("bfs", 0)
+    val = g.values()
+    assert val[0] == 0 and (val[1:hub] == 1).all() and (val[hub:] == 65536).all()
+    g.close()
