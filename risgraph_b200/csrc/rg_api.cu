@@ -336,18 +336,30 @@ int rg_apply_add_del(rg_graph *g, int algo, const rg_edge *adds, uint64_t n_add,
   int rc = check_graph(g);
   if (!rc) rc = check_algo(g->g, algo);
   if (rc) return rc;
-  const uint64_t most = std::max(n_add, n_del);
-  if (adds && dels && n_add && n_del && most > g->g.fused_max && most <= CHUNK_EDGES && !g->g.profiling) {
-    // both batches are checked, packed and on their way before the first one runs
-    Graph &gr = g->g;
-    uint64_t nops = 0;
-    rc = rg::stage_reserve(gr, false, n_add, n_del);
-    if (!rc) rc = stage_unchecked(gr, adds, nullptr, n_add, 0);
-    if (!rc) rc = stage_unchecked(gr, dels, nullptr, n_del, n_add);
-    if (!rc) rc = rg::stage_unpack(gr, false, n_add, 0, directed, &nops);
-    if (!rc) rc = batch_update(gr, n_add, nops, directed, nullptr, true, true);
-    if (!rc) rc = rg::stage_unpack(gr, false, n_del, n_add, directed, &nops);
-    return rc ? rc : batch_update(gr, n_del, nops, directed, nullptr, false, true);
+  Graph &gr = g->g;
+  const bool big_add = n_add > gr.fused_max, big_del = n_del > gr.fused_max;
+  if (adds && dels && n_add && n_del && (big_add || big_del) && std::max(n_add, n_del) <= CHUNK_EDGES &&
+      !gr.profiling) {
+    // Both batches are checked, and the grid-wide ones packed and on their way,
+    // before the first one runs.  A side that fits the fused path takes it: one
+    // delete beside 3,000 inserts cost 40 us on the grid-wide kernels (207 us a
+    // call, 167 so).  That path uses the front of the staging buffers.
+    constexpr uint64_t FRONT = 3 * rg::SMALL_EDGES * sizeof(rg_edge) / 8;  // in records of 8 bytes or more
+    const uint64_t at = big_add ? n_add : FRONT;
+    rc = rg::stage_reserve(gr, false, at, big_del ? n_del : 0);
+    auto look = [&](const rg_edge *e, uint64_t n, bool big, uint64_t after) {
+      return big ? stage_unchecked(gr, e, nullptr, n, after) : check_edges(gr, e, nullptr, n);
+    };
+    auto run = [&](const rg_edge *e, uint64_t n, bool big, uint64_t after, bool add) {
+      if (!big) return edge_updates(g, e, nullptr, n, directed, nullptr, add, true);
+      uint64_t nops = 0;
+      const int r = rg::stage_unpack(gr, false, n, after, directed, &nops);
+      return r ? r : batch_update(gr, n, nops, directed, nullptr, add, true);
+    };
+    if (!rc) rc = look(adds, n_add, big_add, 0);
+    if (!rc) rc = look(dels, n_del, big_del, at);
+    if (!rc) rc = run(adds, n_add, big_add, 0, true);
+    return rc ? rc : run(dels, n_del, big_del, at, false);
   }
   if (!rc) rc = check_edges(g->g, adds, nullptr, n_add);
   if (!rc) rc = check_edges(g->g, dels, nullptr, n_del);
