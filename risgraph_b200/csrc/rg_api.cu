@@ -347,8 +347,9 @@ int rg_apply_add_del(rg_graph *g, int algo, const rg_edge *adds, uint64_t n_add,
     constexpr uint64_t FRONT = 3 * rg::SMALL_EDGES * sizeof(rg_edge) / 8;  // in records of 8 bytes or more
     const uint64_t at = big_add ? n_add : FRONT;
     rc = rg::stage_reserve(gr, false, at, big_del ? n_del : 0);
+    int flags = 0;
     auto look = [&](const rg_edge *e, uint64_t n, bool big, uint64_t after) {
-      return big ? stage_unchecked(gr, e, nullptr, n, after) : check_edges(gr, e, nullptr, n);
+      return big ? rg::stage_copy(gr, e, nullptr, n, after, &flags) : check_edges(gr, e, nullptr, n);
     };
     auto run = [&](const rg_edge *e, uint64_t n, bool big, uint64_t after, bool add) {
       if (!big) return edge_updates(g, e, nullptr, n, directed, nullptr, add, true);
@@ -357,9 +358,14 @@ int rg_apply_add_del(rg_graph *g, int algo, const rg_edge *adds, uint64_t n_add,
       return r ? r : batch_update(gr, n, nops, directed, nullptr, add, true);
     };
     if (!rc) rc = look(adds, n_add, big_add, 0);
-    if (!rc) rc = look(dels, n_del, big_del, at);
-    if (!rc) rc = run(adds, n_add, big_add, 0, true);
-    return rc ? rc : run(dels, n_del, big_del, at, false);
+    if (!rc && !flags) rc = look(dels, n_del, big_del, at);
+    if (!flags) {
+      if (!rc) rc = run(adds, n_add, big_add, 0, true);
+      return rc ? rc : run(dels, n_del, big_del, at, false);
+    }
+    // a fault, or weights that need codes (which are given out only when both
+    // batches are found good): what was packed is not used
+    RG_CUDA(cudaStreamSynchronize(gr.stream));
   }
   if (!rc) rc = check_edges(g->g, adds, nullptr, n_add);
   if (!rc) rc = check_edges(g->g, dels, nullptr, n_del);
