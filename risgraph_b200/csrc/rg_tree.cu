@@ -3355,7 +3355,7 @@ __global__ void __launch_bounds__(FS_TPB)
 }
 
 // ---- the grid engine: levels and deletion repairs in one persistent launch ------
-// One CTA per SM, launched cooperatively, runs every level of a build or of a
+// One CTA per SM (or per two, see ENG_HALF_EDGES), launched cooperatively, runs every level of a build or of a
 // repair, with a grid barrier where the graph-driven loop has kernel
 // boundaries, a level-begin kernel and a conditional node.  That loop spends
 // 15 to 25 us of a level on launches and conditions; a barrier is about 1.5 us.
@@ -3382,6 +3382,13 @@ constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alo
 constexpr uint64_t ENG_PULL_DIV = 12;
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
+// Repairs of batches up to this size take half the SMs, so that those of two
+// graphs driven from two threads run side by side (4,000 inserts and deletes on
+// each of two RMAT-20 graphs, one call of each: 1,050 us on all SMs, 720 on half,
+// 834 for the graph-driven loop; one graph alone 707 and 676).  Larger ones take
+// all: deleting 30,000 tree edges of RMAT-20 SSSP 879 us against 935 on half,
+// 300,000 2,350 against 2,900; 3,000 the same, 470.
+constexpr uint64_t ENG_HALF_EDGES = 16384;
 static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
 static_assert(TASK_SLOTS >= CHUNK && TASK_DEG >= 2 * TASK_SLOTS, "the hub task queue holds the tasks");
 
@@ -4585,8 +4592,9 @@ bool engine_on(const Graph &g) { return g.eng_ctas && g.cluster_edges && !g.prof
 // One engine launch (see k_engine): build from scratch, or the levels of a
 // repair whose frontier is in queue 0, after the deletion repair when `del`.
 // It ends with the control block in the host's copy.
+// n_edges: the edges of the repair's batch.
 template <int A, bool W>
-int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
+int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edges) {
   EngineArgs a = {};
   a.cfg = level_cfg(g, A, build);
   if (a.cfg.allow_pull) {
@@ -4617,7 +4625,8 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root) {
   g.h_ctl[C_KLAUNCH] = CTL_PENDING;
   count_launch(g);
   void *args[] = {(void *)&g.d, (void *)&a};
-  RG_CUDA(cudaLaunchCooperativeKernel((const void *)k_engine<A, W>, dim3((unsigned)g.eng_ctas), dim3(ENG_TPB), args,
+  const int ctas = !build && n_edges <= ENG_HALF_EDGES ? (g.eng_ctas + 1) / 2 : g.eng_ctas;
+  RG_CUDA(cudaLaunchCooperativeKernel((const void *)k_engine<A, W>, dim3((unsigned)ctas), dim3(ENG_TPB), args,
                                       sizeof(EngShared), g.stream));
   g.ctl_on_host = true;
   return RG_OK;
@@ -4627,7 +4636,7 @@ template <int A, bool W>
 int build_enqueue(Graph &g, uint64_t root) {
   int rc = guard_counters(g);
   if (rc) return rc;
-  if (engine_on(g)) return engine_launch<A, W>(g, true, false, root);
+  if (engine_on(g)) return engine_launch<A, W>(g, true, false, root, 0);
   count_launch(g, 2);
   k_prologue<<<1, 1, 0, g.stream>>>(g.d, 0ull);
   k_init<A><<<g.num_sms * 16, TPB, 0, g.stream>>>(g.d, root, g.q[0]);
@@ -4645,7 +4654,7 @@ int add_enqueue(Graph &g, uint64_t n_edges, int directed, bool from_cands) {
       g.d, op_src(g), op_dst(g), op_w(g), from_cands ? op_cand(g) : nullptr, &g.d.ctl[C_CANDN], n_edges, directed,
       g.q[0], &g.d.ctl[C_QN0], mod_stamp(g));
   RG_CUDA(cudaGetLastError());
-  if (engine_on(g)) return engine_launch<A, W>(g, false, false, 0);
+  if (engine_on(g)) return engine_launch<A, W>(g, false, false, 0, n_edges);
   return push_levels<A, W>(g, false);
 }
 
@@ -4665,7 +4674,7 @@ int del_enqueue(Graph &g, uint64_t n_edges, int directed, bool from_cands) {
       g.d, op_src(g), op_dst(g), op_w(g), from_cands ? op_cand(g) : nullptr, &g.d.ctl[C_CANDN], n_edges, directed,
       g.q[0], &g.d.ctl[C_QN0]);
   RG_CUDA(cudaGetLastError());
-  if (engine_on(g)) return engine_launch<A, W>(g, false, true, 0);
+  if (engine_on(g)) return engine_launch<A, W>(g, false, true, 0, n_edges);
   if (g.profiling) {
     rc = del_repair_stepped<A, W>(g);
   } else {
@@ -5057,7 +5066,7 @@ template <int A, bool W>
 int finish_left(Graph &g, unsigned long long left) {
   int rc = RG_OK;
   if (engine_on(g)) {
-    rc = engine_launch<A, W>(g, false, left == 2 && g.h_ctl[C_OVER], 0);
+    rc = engine_launch<A, W>(g, false, left == 2 && g.h_ctl[C_OVER], 0, SMALL_EDGES);
     return rc ? rc : read_ctl(g);
   }
   if (left == 2) {
@@ -5231,7 +5240,7 @@ int apply_add_del_t(Graph &g, const rg_edge *adds, uint64_t n_add, const rg_edge
     // the insert batch's level loop, then the delete batch in its own kernel
     count_launch(g);
     if (engine_on(g)) {
-      if ((rc = engine_launch<A, W>(g, false, false, 0))) return rc;
+      if ((rc = engine_launch<A, W>(g, false, false, 0, n_add))) return rc;
       g.ctl_on_host = false;  // (the kernel after it writes the host's copy last)
       if ((rc = launch_apply_second<A, W>(g, directed))) return rc;
     } else {
