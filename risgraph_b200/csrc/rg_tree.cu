@@ -3534,10 +3534,9 @@ __device__ __forceinline__ void eng_share(uint64_t S, uint64_t &e0, uint64_t &e1
 // Deletion repair over the whole grid (do_update_tree_del,
 // core/graph.hpp:1250-1511): the phases of k_rescue, k_expand, k_reset and
 // k_pull, each followed by the tasks of the long lists it met.
-// Leaves the reset set in queue 0 with its count in ctl[C_QN0].  done: the
-// invalidation levels that the one-CTA repair ran before it handed over.
+// Leaves the reset set in queue 0 with its count in ctl[C_QN0].
 template <int A, bool W>
-__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar, uint64_t done) {
+__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar) {
   unsigned long long *c = g.ctl;
   unsigned long long *hvr = a.bar + EB_HVR, *hve = a.bar + EB_HVE;  // two words each, by turns
   auto cnt = [&](uint64_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
@@ -3545,7 +3544,11 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
   const uint64_t nwarps = ((uint64_t)gridDim.x * ENG_TPB) >> 5;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   bool recompute = false;
-  for (uint64_t it = 0; done + it < a.max_iter; it++) {
+  // the invalidation levels that the one-CTA repair ran before it handed over
+  // (every CTA reads them here: the word is written again at the end)
+  const uint64_t done = __ldcg(&c[C_INVITER]);
+  uint64_t it = 0;
+  for (; done + it < a.max_iter; it++) {
     const uint32_t *fin = a.q[it & 1];
     uint32_t *fout = a.q[(it & 1) ^ 1];
     const uint64_t n = __ldcg(cnt(it));
@@ -3554,10 +3557,7 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
       recompute = true;
       break;
     }
-    if (lead) {
-      *cnt(it + 2) = 0;
-      c[C_INVITER] = done + it + 1;
-    }
+    if (lead) *cnt(it + 2) = 0;
     RepQueue rq;
     rq.task = a.task;
     rq.n = &hvr[it & 1];
@@ -3604,6 +3604,7 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
   if (lead) {
     c[C_QN0] = recompute ? 0 : tn;
     c[C_QN1] = 0;
+    c[C_INVITER] = done + it;
     if (recompute) c[C_RECOMPUTE] = 1;
   }
   if (recompute) return grid_sync(g, bar);
@@ -3793,7 +3794,6 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   // what the launch before left, read before anything below may change it
   uint32_t st = (uint32_t)__ldcg(&c[C_STAMP]);
   uint64_t lvl = a.build ? 0 : __ldcg(&c[C_LEVEL]);
-  const uint64_t inv_levels = a.del ? __ldcg(&c[C_INVITER]) : 0;
   if (lead) a.bar[EB_QN2] = a.bar[EB_HVR] = a.bar[EB_HVE] = 0;
   if (a.build) {
     init_labels<A>(g, a.root, a.q[0], blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB);
@@ -3805,8 +3805,8 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     }
   }
   if (!grid_sync(g, bar)) return;
-  if (a.del && !eng_del<A, W>(g, a, bar, inv_levels)) return;
-  bool pulled = false, any_pull = false;  // the level before, any level before
+  if (a.del && !eng_del<A, W>(g, a, bar)) return;
+  unsigned pulled = 0;  // 1: the level before, 2: any level before (one register: two cost 1% of a build)
   for (uint32_t k = 0;; k++) {
     const uint32_t *fin = a.q[k & 1];
     uint32_t *fout = a.q[(k & 1) ^ 1];
@@ -3831,8 +3831,8 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     }
     // the mode rules of k_level_begin, and a pull in place of a push that
     // would relax a large part of the graph
-    const bool bu = a.cfg.bottom_up && !any_pull && n * a.cfg.bu_div >= g.V;
-    bool pull = !bu && a.cfg.allow_pull && n * (pulled ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
+    const bool bu = a.cfg.bottom_up && !pulled && n * a.cfg.bu_div >= g.V;
+    bool pull = !bu && a.cfg.allow_pull && n * (pulled & 1 ? (a.cfg.pull_div + 3) / 4 : a.cfg.pull_div) >= g.V;
     if (bu) {
       eng_bottom_up<W>(g, sh, lvl, fout, fout_n);
     } else if (!pull && n <= ENG_STAGE) {
@@ -3851,7 +3851,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
         if (!grid_sync(g, bar)) return;
         lvl = __ldcg(&at[0]);
         st = (uint32_t)__ldcg(&at[1]);
-        pulled = false;
+        pulled &= 2;
         continue;
       }
       uint64_t e0, e1;
@@ -3877,7 +3877,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       if (lead && !pull) atomicAdd(&sh.bc.scanned, (unsigned long long)S);
     }
     if (pull) {
-      const uint32_t m = pulled ? (uint32_t)__ldcg(&bnd[k % 3]) : a.cfg.bnd_best;
+      const uint32_t m = pulled & 1 ? (uint32_t)__ldcg(&bnd[k % 3]) : a.cfg.bnd_best;
       unsigned long long *bout = &bnd[(k + 1) % 3];
       eng_pull<A, W>(g, a, sh, a.cfg.pull_split ? PART_HUBS : PART_ALL, m, lvl == 0, bout, fout, fout_n);
       if (!grid_sync(g, bar)) return;
@@ -3887,8 +3887,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
         eng_pull<A, W>(g, a, sh, PART_REST, m, lvl == 0, bout, fout, fout_n);
       }
     }
-    pulled = pull;
-    any_pull = any_pull || pull;
+    pulled = pull ? 3 : pulled & 2;
     lvl++;
     if (!grid_sync(g, bar)) return;
   }
