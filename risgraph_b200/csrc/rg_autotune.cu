@@ -1,9 +1,9 @@
 // Autotuner of the level-mode knobs (rg_autotune in include/risgraph_b200.h).
 //
-// The level engine picks each level's kernel from the frontier size with a few
-// thresholds (rg_option): when a build level pulls, when BFS goes bottom-up,
-// when a push level is dense or edge-balanced, and up to which size a frontier
-// stays in one CTA.  The best values depend on the graph's degree distribution
+// A level's kind follows from the frontier size and a few thresholds (rg_option):
+// when a build level pulls, when BFS goes bottom-up, up to which size a frontier
+// stays in one CTA, and in the graph-driven loop when a push level is dense or
+// edge-balanced.  The best values depend on the graph's degree distribution
 // and on the algorithm, so this tuner measures them on the graph itself:
 // coordinate descent over each knob's candidate values, timing full builds
 // (and, when the caller passes a sample batch, insert+delete round trips of
@@ -112,6 +112,31 @@ struct Tuner {
     *best_ms = cur;
     return RG_OK;
   }
+
+  // Grid engine or graph-driven loop, by builds and round trips together.  Two
+  // knobs are the loop's alone: they are tuned with the loop on, before it is
+  // compared, and keep the values they had when the engine is chosen.  The
+  // graph's present setting stays unless the other one wins by more than medians
+  // of whole builds move (1 %).
+  int tune_driver() {
+    const int own[2] = {RG_OPT_DENSE_DIV, RG_OPT_LBS_MIN};
+    uint64_t had = 0, had_own[2], loop_own[2];
+    int rc = rg_get_option(g, RG_OPT_CLUSTER_EDGES, &had);
+    for (int k = 0; !rc && k < 2; k++) rc = rg_get_option(g, own[k], &had_own[k]);
+    double engine = 0, loop = 0, ms = 0;
+    if (!rc) rc = rg_set_option(g, RG_OPT_CLUSTER_EDGES, had ? had : rg::CLUSTER_EDGES_DEFAULT);
+    if (!rc) rc = both_ms(&engine);
+    const uint64_t on = g->g.cluster_edges;
+    if (!rc) rc = rg_set_option(g, RG_OPT_CLUSTER_EDGES, 0);
+    if (!rc) rc = tune(RG_OPT_DENSE_DIV, {10, 20, 40, 80}, &Tuner::build_ms, &ms);
+    if (!rc) rc = tune(RG_OPT_LBS_MIN, {512, 2048, 8192, 32768, 131072}, &Tuner::build_ms, &ms);
+    if (!rc) rc = both_ms(&loop);
+    for (int k = 0; !rc && k < 2; k++) rc = rg_get_option(g, own[k], &loop_own[k]);
+    const bool use_loop = had ? loop < 0.98 * engine : !(engine < 0.98 * loop);
+    if (!rc) rc = rg_set_option(g, RG_OPT_CLUSTER_EDGES, use_loop ? 0 : on);
+    for (int k = 0; !rc && k < 2; k++) rc = rg_set_option(g, own[k], use_loop ? loop_own[k] : had_own[k]);
+    return rc;
+  }
 };
 
 }  // namespace
@@ -137,12 +162,9 @@ extern "C" int rg_autotune(rg_graph *g, int algo, uint64_t root, const rg_edge *
     if ((rc = t.tune(RG_OPT_PULL_DIV, {16, 32, 64, 128, 256}, &Tuner::build_ms, &ms))) return rc;
   }
   if (algo != RG_BFS && (rc = t.tune(RG_OPT_PULL_SPLIT, {0, 1}, &Tuner::build_ms, &ms))) return rc;
-  if ((rc = t.tune(RG_OPT_DENSE_DIV, {10, 20, 40, 80}, &Tuner::build_ms, &ms))) return rc;
-  if ((rc = t.tune(RG_OPT_LBS_MIN, {512, 2048, 8192, 32768, 131072}, &Tuner::build_ms, &ms))) return rc;
   // small-frontier knob: builds and the sample's round trips together
   if ((rc = t.tune(RG_OPT_TINY_EDGES, {0, 8192, 32768, 131072}, &Tuner::both_ms, &ms))) return rc;
-  // graph-driven loop (0) or grid engine: builds and round trips together
-  if ((rc = t.tune(RG_OPT_CLUSTER_EDGES, {0, 16384, 65536, 262144}, &Tuner::both_ms, &ms))) return rc;
+  if ((rc = t.tune_driver())) return rc;
   if ((rc = t.build_ms(&out->build_ms_after))) return rc;
   if ((rc = t.apply_ms(&out->apply_ms_after))) return rc;
   if (out->build_ms_after + out->apply_ms_after > 1.05 * (out->build_ms_before + out->apply_ms_before)) {

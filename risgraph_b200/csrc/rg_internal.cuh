@@ -82,7 +82,7 @@ enum Ctl : int {
 enum LevelMode : unsigned long long {
   M_EMPTY = 0,      // frontier empty: every level kernel returns at once
   M_SPARSE = 1,     // k_push + k_push_hub over the frontier list
-  M_PULL = 2,       // k_pull_hubs + k_pull_sell over all in-edges
+  M_PULL = 2,       // k_pull_sell + k_pull_hub_fix over all in-edges
   M_DENSE_PUSH = 3, // k_push_dense over all out-slots of active vertices
   M_BOTTOM_UP = 4,  // k_bfs_bottom_up (full BFS builds)
   M_LBS = 5,        // edge-balanced push (degree scan + tile partition + k_push_lbs)
@@ -278,6 +278,8 @@ struct SellPlan {
   uint32_t slice[SELL_KEYS];            // first slice of key <= k
 };
 
+constexpr uint64_t CLUSTER_EDGES_DEFAULT = 65536;  // RG_OPT_CLUSTER_EDGES
+
 // A cached, instantiated level-loop graph.
 struct LoopGraph {
   cudaGraphExec_t exec = nullptr;
@@ -353,7 +355,7 @@ struct Graph {
   uint64_t fused_max = 2048;
   int phase_trace = 0;            // RG_OPT_PHASE_TRACE
   uint64_t inline_max = 16;       // RG_OPT_INLINE_MAX: largest fused batch passed in the launch parameters
-  uint64_t cluster_edges = 65536;  // RG_OPT_CLUSTER_EDGES: 0: no grid engine, else also the out-slot limit of a cluster level
+  uint64_t cluster_edges = CLUSTER_EDGES_DEFAULT;  // RG_OPT_CLUSTER_EDGES: 0: no grid engine, else also the out-slot limit of a cluster level
   int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
   unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
   uint32_t wait_polls = 1u << 24;   // polls before one of its waits gives up (ten seconds or more)
