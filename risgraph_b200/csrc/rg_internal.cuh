@@ -74,7 +74,8 @@ enum Ctl : int {
   C_HVP = 29,      // ... by the pull over the reset set
   C_OVER = 30,     // the fused apply's one-CTA deletion repair handed over to the grid-wide one
   C_LEFT = 31,     // what a fused kernel left to the host (1: insert batch's level loop [and the delete batch], 2: delete batch's repair)
-  C_PULLED = 32,   // a level of the current loop pulled
+  C_HOST = 32,     // the words above are the host's too (ctl_to_host); the rest stay on the device
+  C_PULLED = 32,   // a level of the current graph-driven loop pulled
   C_BEAT = 33,     // counts up while long serial work goes on (see has_parents)
   C_COUNT = 34
 };

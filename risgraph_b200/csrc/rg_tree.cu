@@ -1750,7 +1750,6 @@ __device__ __forceinline__ void prologue_words(unsigned long long *c, unsigned l
   c[C_EDGES] = 0;
   c[C_MODE] = M_EMPTY;
   c[C_KLAUNCH] = 0;
-  c[C_PULLED] = 0;
   c[C_HVR] = 0;
   c[C_HVE] = 0;
   c[C_HVP] = 0;
@@ -1844,7 +1843,7 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   if (n == 0) mode = M_EMPTY;
   // (a pull level commits values deeper than the level, which a bottom-up level,
   // looking for parents of one depth, would miss: none follows a pull)
-  else if (cfg.bottom_up && !c[C_PULLED] && n * cfg.bu_div >= g.V) mode = M_BOTTOM_UP;
+  else if (cfg.bottom_up && !(lvl && c[C_PULLED]) && n * cfg.bu_div >= g.V) mode = M_BOTTOM_UP;
   // pull once the frontier passes |V| / pull_div, and keep pulling until it
   // falls below 4x that (the frontier's first large levels are hub-heavy, its
   // last ones are not: the direction switch of Beamer et al., by vertex count)
@@ -1854,7 +1853,7 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   else if (dense) mode = M_DENSE_PUSH;
   else if (n >= cfg.lbs_min) mode = M_LBS;
   if (mode == M_DENSE_PUSH) c[C_ACT] += 1;
-  if (mode == M_PULL) c[C_PULLED] = 1;
+  if (lvl == 0 || mode == M_PULL) c[C_PULLED] = mode == M_PULL;
   c[C_MODE] = mode;
   // bounds on the frontiers' values: pull levels collect theirs, others give none
   const int half = fin_n == &c[C_QN0] ? 0 : 1;
@@ -2786,10 +2785,11 @@ struct FusedRepair {
 
 // The control block to the host's mapped copy, by the whole CTA after its
 // last update (the host reads it once the stream has synchronised, and the
-// kernel's end makes its writes visible).
+// kernel's end makes its writes visible).  One warp and 256 bytes: two words more
+// cost 0.7 us of a 20 us call.
 __device__ __forceinline__ void ctl_to_host(const DevGraph &g, unsigned long long *ctl_host) {
   __syncthreads();
-  if (threadIdx.x < C_COUNT) ctl_host[threadIdx.x] = g.ctl[threadIdx.x];
+  if (threadIdx.x < C_HOST) ctl_host[threadIdx.x] = g.ctl[threadIdx.x];
 }
 
 // A batch's header as the fused kernels read it.
