@@ -283,10 +283,11 @@ int stage_copy(Graph &g, const rg_edge *edges, const uint64_t *pairs, uint64_t n
   uint32_t *host = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_host) + at);
   uint32_t *dev = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_dev) + at);
   *flags = 0;
+  const int threads = n >= RG_STAGE_PARALLEL;
   for (uint64_t b = 0; b < n; b += STAGE_STEP) {
     const uint64_t m = std::min(STAGE_STEP, n - b);
-    *flags |= pairs ? rg_stage_pairs(pairs + 2 * b, m, g.V, host + words * b)
-                    : rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, host + words * b);
+    *flags |= pairs ? rg_stage_pairs(pairs + 2 * b, m, g.V, threads, host + words * b)
+                    : rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, threads, host + words * b);
     if (*flags) return RG_OK;
     RG_CUDA(cudaMemcpyAsync(dev + words * b, host + words * b, m * words * 4, cudaMemcpyHostToDevice, g.stream));
   }
@@ -310,10 +311,11 @@ static int stage_trusted(Graph &g, const rg_edge *edges, const uint64_t *pairs, 
   const uint64_t words = g.weighted && !pairs ? 3 : 2, at = stage_bytes(g, pairs != nullptr, after);
   uint32_t *host = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_host) + at);
   uint32_t *dev = reinterpret_cast<uint32_t *>(static_cast<char *>(g.stage_dev) + at);
+  const int threads = n >= RG_STAGE_PARALLEL;
   for (uint64_t b = 0; b < n; b += STAGE_STEP) {
     const uint64_t m = std::min(STAGE_STEP, n - b);
-    if (pairs) rg_stage_pairs(pairs + 2 * b, m, g.V, host + words * b);
-    else rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, host + words * b);
+    if (pairs) rg_stage_pairs(pairs + 2 * b, m, g.V, threads, host + words * b);
+    else rg_stage_edges(edges + b, m, g.V, g.weighted, W_RAW_MAX, W_LIMIT, threads, host + words * b);
     RG_CUDA(cudaMemcpyAsync(dev + words * b, host + words * b, m * words * 4, cudaMemcpyHostToDevice, g.stream));
   }
   return RG_OK;
