@@ -220,10 +220,12 @@ int rg_phase_trace(rg_graph *g, uint64_t *ns);
  *   RG_OPT_PULL_DIV       a build level pulls when frontier * div >= |V| (default 64)
  *   RG_OPT_TINY_EDGES     frontiers of at most 1024 vertices and this many out-slots
  *                         run level after level in one CTA (default 32768, max 2^20,
- *                         0 = off)
- *   RG_OPT_DENSE_DIV      a level is dense when frontier * div >= |V|
- *   RG_OPT_LBS_MIN        frontiers at least this large use the edge-balanced push
- *   RG_OPT_BFS_BOTTOM_UP  1: full BFS builds pull bottom-up on large levels
+ *                         0 = off; the persistent launch of RG_OPT_CLUSTER_EDGES
+ *                         spreads levels of more than 1024 slots over its CTAs)
+ *   RG_OPT_DENSE_DIV      a level is dense when frontier * div >= |V| (*)
+ *   RG_OPT_LBS_MIN        frontiers at least this large use the edge-balanced push (*)
+ *   RG_OPT_BFS_BOTTOM_UP  1: full BFS builds pull bottom-up on large levels, as long as
+ *                         no level of the build has pulled (RG_OPT_DENSE_PULL 1)
  *   RG_OPT_BFS_BU_DIV     a BFS build level goes bottom-up when frontier * div >= |V|
  *                         (default 64; Beamer's direction switch by frontier size)
  *   RG_OPT_RECOMPUTE_MIN  deletion repair falls back to a full build when the
@@ -239,7 +241,7 @@ int rg_phase_trace(rg_graph *g, uint64_t *ns);
  *   RG_OPT_PULL_GROUPS    launches of a split pull level (2..16, default 2): the
  *                         hub slices first, then the other rows, widest first, in
  *                         groups - 1 launches of about equal entries; each launch
- *                         reads the values the earlier ones set in this level.
+ *                         reads the values the earlier ones set in this level. (*)
  *   RG_OPT_FUSED_MAX      update batches of at most this many edges (0..2048,
  *                         default 2048) take the fused single-CTA path of
  *                         rg_apply_*: storage and small repairs in one
@@ -254,13 +256,20 @@ int rg_phase_trace(rg_graph *g, uint64_t *ns);
  *                         launch or more per level (what served graphs do);
  *                         otherwise (default 65536, at most 2^20) the levels
  *                         and deletion repairs of a call run in one persistent
- *                         launch over all SMs.  In profile mode, which steps
+ *                         launch over all SMs, repairs of at most 16,384 edges
+ *                         over half of them.  A wait inside it that sees no
+ *                         progress for about ten seconds ends the call with
+ *                         RG_ETIMEOUT, with the labels partly updated as after
+ *                         RG_OPT_MAX_LEVELS.  In profile mode, which steps
  *                         the levels from the host, frontiers too large for
  *                         one CTA but of at most 16 x 1024 vertices (8 x 1024
  *                         where the GPU schedules no 16-CTA cluster) and this
  *                         many out-slots run in one thread-block cluster; a
  *                         frontier that a tiny level could take goes
- *                         to the cluster when it has more than 4096 slots. */
+ *                         to the cluster when it has more than 4096 slots.
+ * (*) Of the graph-driven loop and profile mode only: the persistent launch
+ *     spreads every push over its CTAs by out-slots, and splits a pull level in
+ *     two parts at most. */
 typedef enum {
   RG_OPT_DENSE_PULL = 0,
   RG_OPT_DENSE_DIV = 1,
@@ -282,11 +291,14 @@ int rg_set_option(rg_graph *g, int option, uint64_t value);
 int rg_get_option(rg_graph *g, int option, uint64_t *value);
 
 /* Autotuner of the options above for this graph and algorithm: coordinate
- * descent over candidate values of the pull / bottom-up divisor, the dense
- * divisor, the edge-balanced minimum and the small-frontier size, timing `reps`
- * full builds per trial (and, when n_sample > 0, insert + delete round trips
- * of the sample batch, which leave the graph unchanged, for the small-frontier
- * size).  The chosen values stay set on the graph.  Every trial must give the
+ * descent over candidate values of the pull / bottom-up divisor, the pull split
+ * and the small-frontier size, then the persistent launch against the
+ * graph-driven loop with its dense divisor and edge-balanced minimum tuned
+ * (RG_OPT_CLUSTER_EDGES; the two keep their values unless the loop is chosen),
+ * timing `reps` full builds per trial (and, when n_sample > 0, insert + delete
+ * round trips of the sample batch, which leave the graph unchanged, for the
+ * small-frontier size and for the launch against the loop).  The chosen values
+ * stay set on the graph.  Every trial must give the
  * same values (checked by checksum); the labels end as after rg_build_tree.
  * No reference counterpart: the reference's thresholds are constants. */
 typedef struct {
@@ -380,7 +392,7 @@ int rg_server_create(uint64_t hbm_budget_bytes, double target_epoch_ms, uint64_t
  * RG_ENOMEM_HBM when its device bytes would exceed the budget.  While
  * attached the graph runs the graph-driven level loop (RG_OPT_CLUSTER_EDGES
  * reads 0; detach gives the value back): with other instances' epochs on the
- * GPU a launch that needs every SM would wait for them. */
+ * GPU a launch that needs half the SMs or all would wait for them. */
 int rg_server_attach(rg_server *s, rg_graph *g, int algo, int directed, uint32_t *instance);
 int rg_server_detach(rg_server *s, uint32_t instance);
 /* Record the label history (rg_history_record of the modified vertices) after

@@ -392,7 +392,7 @@ int rg_server_attach(rg_server *s, rg_graph *g, int algo, int directed, uint32_t
   // The graph-driven level loop while served (option value 0): the epochs of
   // other instances keep SMs busy, and a launch that needs many SMs at once then
   // waits for them (16-SM clusters alone took p99 from 0.4 to 4 ms in the
-  // six-instance mix; the grid engine needs every SM).
+  // six-instance mix; the grid engine needs half of them or all).
   in->cluster_edges = g->g.cluster_edges;
   g->g.cluster_edges = 0;
   Instance *raw = in.get();

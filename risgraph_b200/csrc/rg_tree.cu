@@ -3378,7 +3378,9 @@ constexpr uint32_t ENG_STAGE = 2048;
 constexpr int ENG_MAX_CTAS = 256;
 constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alone (4096 took 20 us a level, the grid 9)
 // a build's push level pulls instead when its out-slots are at least 1 / 12 of the copy's
-// entries (RMAT-22 SSWP: the push of 97K vertices took 241 us, a pull level 75)
+// entries (RMAT-22 SSWP: the push of 97K vertices took 241 us, a pull level 75).  Builds, us, at
+// 1/1, 1/6, 1/12 and 1/24: SSWP RMAT-22 1010, 833, 797, 800; RMAT-20 693, 678, 707, 752; RMAT-18
+// 422, 435, 441, 443; SSSP RMAT-20 440, 440, 426, 426; the same at RMAT-18 and 22
 constexpr uint64_t ENG_PULL_DIV = 12;
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
