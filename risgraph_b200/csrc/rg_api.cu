@@ -724,6 +724,13 @@ int rg_test_wait_polls(rg_graph *gh, uint64_t polls) {
   return RG_OK;
 }
 
+// For tests: out-slots from which the engine leaves a push level to the loop; 0: the default.
+int rg_test_push_slots(rg_graph *gh, uint64_t slots) {
+  if (!gh) return RG_EINVAL;
+  gh->g.push_slots = slots ? slots : Graph().push_slots;
+  return RG_OK;
+}
+
 int rg_device_bytes(rg_graph *gh, uint64_t *bytes) {
   if (!gh || !bytes) return RG_EINVAL;
   *bytes = gh->g.bytes;

@@ -52,7 +52,7 @@ enum Ctl : int {
   C_ERR = 8,       // first error code raised on the device
   C_RECOMPUTE = 9, // parent-chain guard tripped (has_parents, core/graph.hpp:1900-1903)
   C_MODN = 10,     // modified list length
-  C_CHECKSUM = 11,
+  C_ELEFT = 11,    // what the grid engine left to the host (EngineLeft)
   C_AUX = 12,
   C_EDGES = 13,    // edge slots scanned by push levels (work counter)
   C_BND0 = 14,     // bound on the values in queue 0: none of them is better than this
@@ -77,7 +77,13 @@ enum Ctl : int {
   C_HOST = 32,     // the words above are the host's too (ctl_to_host); the rest stay on the device
   C_PULLED = 32,   // a level of the current graph-driven loop pulled
   C_BEAT = 33,     // counts up while long serial work goes on (see has_parents)
-  C_COUNT = 34
+  C_CHECKSUM = 34,
+  C_COUNT = 35
+};
+
+enum EngineLeft : unsigned long long {
+  ELEFT_NONE = 0,
+  ELEFT_PUSH = 1    // the levels from the frontier in queue 0 on, to the graph-driven loop
 };
 
 enum LevelMode : unsigned long long {
@@ -360,6 +366,7 @@ struct Graph {
   int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
   unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
   uint32_t wait_polls = 1u << 24;   // polls before one of its waits gives up (ten seconds or more)
+  uint64_t push_slots = 8ull << 20;  // out-slots of a push level that it leaves to the loop (see k_engine)
   bool ctl_on_host = false;         // the last launch writes the control block to h_ctl itself
   int cl_ctas = 0;                  // CTAs of the cluster kernel (16 where the GPU schedules it, else 8)
   unsigned long long *ptrace_buf = nullptr;  // its device buffer (allocated with the labels)

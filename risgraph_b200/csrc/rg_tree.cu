@@ -1750,6 +1750,7 @@ __device__ __forceinline__ void prologue_words(unsigned long long *c, unsigned l
   c[C_EDGES] = 0;
   c[C_MODE] = M_EMPTY;
   c[C_KLAUNCH] = 0;
+  c[C_ELEFT] = 0;
   c[C_HVR] = 0;
   c[C_HVE] = 0;
   c[C_HVP] = 0;
@@ -1835,6 +1836,7 @@ __global__ void __launch_bounds__(LVB_TPB) k_level_begin(DevGraph g, const uint3
   const uint64_t n = n0;
   const uint64_t lvl = c[C_LEVEL];
   *fout_n = 0;
+  c[C_ELEFT] = 0;
   c[C_HUBN] = 0;
   c[C_STAMP] += 1;
   c[C_DEPTH] = lvl;
@@ -2875,8 +2877,9 @@ __device__ __forceinline__ int apply_batch(const DevGraph &g, const sdev::OpView
     if (tr && tid == 0) tr[k] = global_ns();
   };
   if (tid == 0) {
-    // the second batch of a submission does nothing after an error in the first
-    s_skip = second && c[C_ERR] != 0;
+    // the second batch of a submission does nothing after an error in the first,
+    // or before the levels that the engine left of the first one's repair
+    s_skip = second && (c[C_ERR] != 0 || c[C_ELEFT] != 0);
     if (!s_skip) {
       s_rec_top = *g.rec_top;
       const unsigned long long kl = c[C_KLAUNCH];
@@ -3382,6 +3385,13 @@ constexpr uint32_t ENG_TINY = 1024;          // out-slots that CTA 0 relaxes alo
 // 1/1, 1/6, 1/12 and 1/24: SSWP RMAT-22 1010, 833, 797, 800; RMAT-20 693, 678, 707, 752; RMAT-18
 // 422, 435, 441, 443; SSSP RMAT-20 440, 440, 426, 426; the same at RMAT-18 and 22
 constexpr uint64_t ENG_PULL_DIV = 12;
+// A push level of Graph::push_slots out-slots (8M) is left, with all that follow, to the graph-driven
+// loop (ELEFT_PUSH), whose edge-balanced and dense pushes keep more edges in flight per SM and win there.
+// An edge that joins the root to an RMAT-20 graph, us a call, left and not left: SSSP 1165, 1850; BFS
+// 525, 596; WCC 688, 832 (RMAT-18, 4M edges, never left: 754, 290, 366; left from 2M on: 695, 331, 390).
+// With the line at 4M, putting 300,000 tree edges of RMAT-20 SSSP back took 1438 instead of 1250.  The
+// first level of a deletion repair stays: few slots of the reset set improve anything, and the engine
+// reads them as fast (batches of 10,000 deletes with hubs among them lost 70 us each).
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 // Repairs of batches up to this size take half the SMs, so that those of two
@@ -3413,6 +3423,7 @@ struct EngineArgs {
   LevelCfg cfg;
   uint32_t mst;
   uint32_t polls;               // before a wait gives up
+  uint64_t push_slots;          // out-slots of a push level that is left to the loop
   int build;                    // initialise the labels first
   int del;                      // repair deletions from the invalidated frontier in queue 0 first
 };
@@ -3808,12 +3819,14 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   }
   if (!grid_sync(g, bar)) return;
   if (a.del && !eng_del<A, W>(g, a, bar)) return;
+  bool leave = false;
+  uint64_t n = 0;
   unsigned pulled = 0;  // 1: the level before, 2: any level before (one register: two cost 1% of a build)
   for (uint32_t k = 0;; k++) {
     const uint32_t *fin = a.q[k & 1];
     uint32_t *fout = a.q[(k & 1) ^ 1];
     unsigned long long *fout_n = cnt(k + 1);
-    const uint64_t n = __ldcg(cnt(k));
+    n = __ldcg(cnt(k));
     if (n == 0) break;
     if (lvl >= a.cfg.max_levels) {
       if (lead) atomicCAS(&c[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
@@ -3868,6 +3881,14 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       uint32_t i;
       const uint64_t S = eng_first(a, sh, scan_tmp, (uint32_t)n, per, e0, e1, i);
       pull = a.cfg.allow_pull && S * ENG_PULL_DIV >= a.plan->total;
+      if (!pull && S >= a.push_slots && !(a.del && k == 0)) {
+        // the loop starts with queue 0, which holds the frontier before last now
+        if (k & 1)
+          for (uint64_t x = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; x < n; x += (uint64_t)gridDim.x * ENG_TPB)
+            fout[x] = fin[x];
+        leave = true;
+        break;
+      }
       for (uint64_t e = e0; e < e1 && !pull;) {
         const uint32_t m = eng_stage_from(g, a, sh, fin, (uint32_t)n, per, i, S);
         const uint64_t end = min(e1, sh.p.pref[m]);
@@ -3897,8 +3918,15 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   if (!grid_sync(g, bar, blockIdx.x != 0)) return;  // (every CTA has read the last queue counts)
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
-      c[C_QN0] = 0;
+      c[C_QN0] = leave ? n : 0;
       c[C_QN1] = 0;
+      if (leave) {  // (the loop begins this level anew)
+        c[C_LEVEL] = lvl;
+        c[C_MODE] = M_EMPTY;
+        c[C_BND0] = a.cfg.bnd_best;
+        c[C_PULLED] = pulled != 0;
+        c[C_ELEFT] = ELEFT_PUSH;
+      }
       if (lvl < TRACE_CAP) g.trace[TRACE_CAP + lvl] = global_ns();
     }
     ctl_to_host(g, a.ctl_host);
@@ -4621,6 +4649,7 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edge
   a.max_iter = (uint64_t)g.V + 2;
   a.mst = mod_stamp(g);
   a.polls = g.wait_polls;
+  a.push_slots = g.push_slots;
   a.build = build ? 1 : 0;
   a.del = del ? 1 : 0;
   g.h_ctl[C_KLAUNCH] = CTL_PENDING;
@@ -4631,6 +4660,16 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edge
                                       sizeof(EngShared), g.stream));
   g.ctl_on_host = true;
   return RG_OK;
+}
+
+// The levels that the engine left, to their end.
+template <int A, bool W>
+int engine_left(Graph &g, bool build) {
+  cudaGraphExec_t exec;
+  const int rc = loop_exec<A, W>(g, build, &exec);
+  if (rc) return rc;
+  RG_CUDA(cudaGraphLaunch(exec, g.stream));
+  return read_ctl(g);
 }
 
 template <int A, bool W>
@@ -4697,6 +4736,10 @@ int after_sync(Graph &g, int what) {
     if (code == RG_ETIMEOUT) engine_reset(g);
     cudaMemsetAsync(&g.d.ctl[C_ERR], 0, 8, g.stream);
     return code;
+  }
+  if (g.h_ctl[C_ELEFT]) {
+    const int rc = engine_left<A, W>(g, what == 0);
+    return rc ? rc : after_sync<A, W>(g, what);
   }
   g.launches += g.h_ctl[C_KLAUNCH];  // kernels run inside graphs, counted on the device
   g.st_levels = g.h_ctl[C_LEVEL];
@@ -5244,6 +5287,14 @@ int apply_add_del_t(Graph &g, const rg_edge *adds, uint64_t n_add, const rg_edge
       if ((rc = engine_launch<A, W>(g, false, false, 0, n_add))) return rc;
       g.ctl_on_host = false;  // (the kernel after it writes the host's copy last)
       if ((rc = launch_apply_second<A, W>(g, directed))) return rc;
+      RG_CUDA(cudaStreamSynchronize(g.stream));
+      if (g.h_ctl[C_ELEFT] && !g.h_ctl[C_ERR]) {
+        // the engine left levels of the insert batch: the delete batch waited
+        if ((rc = engine_left<A, W>(g, false))) return rc;
+        if ((rc = storage_error(g))) return rc;
+        count_launch(g);
+        if ((rc = launch_apply_second<A, W>(g, directed))) return rc;
+      }
     } else {
       cudaGraphExec_t re;
       if ((rc = rest_exec<A, W>(g, directed, &re))) return rc;
