@@ -724,10 +724,17 @@ int rg_test_wait_polls(rg_graph *gh, uint64_t polls) {
   return RG_OK;
 }
 
-// For tests: out-slots from which the engine leaves a push level to the loop; 0: the default.
+// For tests: out-slots from which the engine leaves a push level to the loop, and
+// vertices from which it leaves off on half the SMs; 0: the default.
 int rg_test_push_slots(rg_graph *gh, uint64_t slots) {
   if (!gh) return RG_EINVAL;
   gh->g.push_slots = slots ? slots : Graph().push_slots;
+  return RG_OK;
+}
+
+int rg_test_half_vertices(rg_graph *gh, uint64_t vertices) {
+  if (!gh) return RG_EINVAL;
+  gh->g.half_vertices = vertices ? vertices : Graph().half_vertices;
   return RG_OK;
 }
 

@@ -83,7 +83,9 @@ enum Ctl : int {
 
 enum EngineLeft : unsigned long long {
   ELEFT_NONE = 0,
-  ELEFT_PUSH = 1    // the levels from the frontier in queue 0 on, to the graph-driven loop
+  ELEFT_PUSH = 1,   // the levels from the frontier in queue 0 on, to the graph-driven loop
+  ELEFT_LEVELS = 2, // the same, to a launch on all SMs
+  ELEFT_REPAIR = 3  // the deletion repair from there on, to a launch on all SMs
 };
 
 enum LevelMode : unsigned long long {
@@ -366,6 +368,7 @@ struct Graph {
   int eng_ctas = 0;                 // CTAs of the grid engine (0: it does not fit this GPU)
   unsigned long long *eng_bar = nullptr;  // its barrier words, third queue counter and bounds
   uint32_t wait_polls = 1u << 24;   // polls before one of its waits gives up (ten seconds or more)
+  uint64_t half_vertices = 32768;    // vertices at which a launch on half the SMs leaves off
   uint64_t push_slots = 8ull << 20;  // out-slots of a push level that it leaves to the loop (see k_engine)
   bool ctl_on_host = false;         // the last launch writes the control block to h_ctl itself
   int cl_ctas = 0;                  // CTAs of the cluster kernel (16 where the GPU schedules it, else 8)

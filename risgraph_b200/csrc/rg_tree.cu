@@ -3390,8 +3390,8 @@ constexpr uint64_t ENG_PULL_DIV = 12;
 // An edge that joins the root to an RMAT-20 graph, us a call, left and not left: SSSP 1165, 1850; BFS
 // 525, 596; WCC 688, 832 (RMAT-18, 4M edges, never left: 754, 290, 366; left from 2M on: 695, 331, 390).
 // With the line at 4M, putting 300,000 tree edges of RMAT-20 SSSP back took 1438 instead of 1250.  The
-// first level of a deletion repair stays: few slots of the reset set improve anything, and the engine
-// reads them as fast (batches of 10,000 deletes with hubs among them lost 70 us each).
+// first level of a deletion repair stays unless it is dense: few slots of a reset set with hubs in it
+// improve anything, and the engine reads them as fast (such batches of 10,000 deletes lost 70 us each).
 constexpr uint64_t ENG_TINY_LEVELS = 2048;   // levels it runs before the others look in again
 constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 // Repairs of batches up to this size take half the SMs, so that those of two
@@ -3399,7 +3399,11 @@ constexpr int ENG_ITEMS = 2;                 // slots a thread relaxes at a time
 // each of two RMAT-20 graphs, one call of each: 1,050 us on all SMs, 720 on half,
 // 834 for the graph-driven loop; one graph alone 707 and 676).  Larger ones take
 // all: deleting 30,000 tree edges of RMAT-20 SSSP 879 us against 935 on half,
-// 300,000 2,350 against 2,900; 3,000 the same, 470.
+// 300,000 2,350 against 2,900; 3,000 the same, 470.  A repair on half that comes to a
+// frontier or a reset set of more than Graph::half_vertices (32,768), or to a push of 32
+// times as many out-slots, goes on in a second launch, on all (deleting 3,000 edges of an
+// RMAT-20 graph, the one that joins it to the root among them, us so, on half alone and on
+// all alone: SSSP 2090, 2520, 1970; BFS 1600, 1940, 1675; WCC 2750, 3540, 2760).
 constexpr uint64_t ENG_HALF_EDGES = 16384;
 static_assert(ENG_TPB == TINY_TPB, "CTA 0 runs the one-CTA levels");
 static_assert(TASK_SLOTS >= CHUNK && TASK_DEG >= 2 * TASK_SLOTS, "the hub task queue holds the tasks");
@@ -3424,6 +3428,7 @@ struct EngineArgs {
   uint32_t mst;
   uint32_t polls;               // before a wait gives up
   uint64_t push_slots;          // out-slots of a push level that is left to the loop
+  uint64_t half_vertices, half_slots;  // vertices and out-slots at which a launch on half the SMs leaves off
   int build;                    // initialise the labels first
   int del;                      // repair deletions from the invalidated frontier in queue 0 first
 };
@@ -3490,6 +3495,10 @@ struct EngShared {
   EngStage p;
   uint32_t q[ENG_TPB / 32][PQ_CAP];
   BlockCounts bc;
+  // why the level loop ended early and with how many vertices (thread 0's; in
+  // registers they cost BFS builds 3 %)
+  unsigned long long left;
+  uint64_t left_n;
   // the kernel's parameters: the level kinds are calls and take them by
   // reference, and a reference into parameter space is read through L1, which
   // every barrier empties
@@ -3547,9 +3556,16 @@ __device__ __forceinline__ void eng_share(uint64_t S, uint64_t &e0, uint64_t &e1
 // Deletion repair over the whole grid (do_update_tree_del,
 // core/graph.hpp:1250-1511): the phases of k_rescue, k_expand, k_reset and
 // k_pull, each followed by the tasks of the long lists it met.
-// Leaves the reset set in queue 0 with its count in ctl[C_QN0].
+// Leaves the reset set in queue 0 with its count in ctl[C_QN0], or leaves off
+// with the frontier of n vertices there.
+enum DelResult : int { DEL_GAVE_UP, DEL_DONE, DEL_LEFT };
+// A frontier of queue 1 into queue 0, which holds the one before it (all CTAs).
+__device__ __noinline__ void eng_to_q0(const EngineArgs &a, uint64_t n) {
+  for (uint64_t i = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; i < n; i += (uint64_t)gridDim.x * ENG_TPB)
+    a.q[0][i] = a.q[1][i];
+}
 template <int A, bool W>
-__device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar) {
+__device__ __noinline__ DelResult eng_del(const DevGraph &g, const EngineArgs &a, GridBar &bar, uint64_t &n_left) {
   unsigned long long *c = g.ctl;
   unsigned long long *hvr = a.bar + EB_HVR, *hve = a.bar + EB_HVE;  // two words each, by turns
   auto cnt = [&](uint64_t k) { return k % 3 == 2 ? a.bar + EB_QN2 : &c[C_QN0 + k % 3]; };
@@ -3570,12 +3586,18 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
       recompute = true;
       break;
     }
+    if (n > a.half_vertices) {
+      if (it & 1) eng_to_q0(a, n);
+      if (lead) c[C_INVITER] = done + it;
+      n_left = n;
+      return DEL_LEFT;
+    }
     if (lead) *cnt(it + 2) = 0;
     RepQueue rq;
     rq.task = a.task;
     rq.n = &hvr[it & 1];
     rescue_warps<A, W>(g, fin, n, a.limit, warp, nwarps, rq);
-    if (!grid_sync(g, bar)) return false;
+    if (!grid_sync(g, bar)) return DEL_GAVE_UP;
     const uint64_t nr = __ldcg(rq.n);
     if (nr) {
       const uint32_t tag_inv = (uint32_t)c[C_INVTAG];
@@ -3589,7 +3611,7 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
         if (__shfl_sync(FULL, td, 0) != tag_inv) continue;  // rescued by another task
         rescue_one<A, W>(g, d, sd, k0, min(len, k0 + TASK_SLOTS), off, tag_inv, a.limit);
       }
-      if (!grid_sync(g, bar)) return false;
+      if (!grid_sync(g, bar)) return DEL_GAVE_UP;
     }
     if (__ldcg(&c[C_RECOMPUTE])) {  // a chain ran past the guard (nothing sets it before the next level's rescue)
       recompute = true;
@@ -3598,7 +3620,7 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
     if (lead) hvr[(it + 1) & 1] = hve[(it + 1) & 1] = 0;
     rq.n = &hve[it & 1];
     expand_warps<A, W>(g, fin, n, a.tree, fout, cnt(it + 1), warp, nwarps, rq);
-    if (!grid_sync(g, bar)) return false;
+    if (!grid_sync(g, bar)) return DEL_GAVE_UP;
     const uint64_t ne = __ldcg(rq.n);
     if (ne) {
       const uint32_t tag_inv = (uint32_t)c[C_INVTAG];
@@ -3609,28 +3631,33 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
         expand_slots<W, 4>(g, u, g.out.off[u], k0 + lane_id(), 32, min(len, k0 + TASK_SLOTS), tag_inv, fout,
                            cnt(it + 1));
       }
-      if (!grid_sync(g, bar)) return false;
+      if (!grid_sync(g, bar)) return DEL_GAVE_UP;
     }
   }
   const uint64_t tn = __ldcg(&c[C_TREEN]);
-  if (!grid_sync(g, bar)) return false;  // (every CTA has read the last counts)
+  if (!grid_sync(g, bar)) return DEL_GAVE_UP;  // (every CTA has read the last counts)
+  if (tn > a.half_vertices && !recompute) {
+    if (lead) c[C_INVITER] = done + it;
+    n_left = 0;  // (nothing is left to invalidate)
+    return DEL_LEFT;
+  }
   if (lead) {
     c[C_QN0] = recompute ? 0 : tn;
     c[C_QN1] = 0;
     c[C_INVITER] = done + it;
     if (recompute) c[C_RECOMPUTE] = 1;
   }
-  if (recompute) return grid_sync(g, bar);
+  if (recompute) return grid_sync(g, bar) ? DEL_DONE : DEL_GAVE_UP;
   // reset the invalid set; it is also the frontier of the push levels
   reset_warps<A>(g, a.tree, tn, a.mst, warp, nwarps);
   for (uint64_t i = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; i < tn; i += (uint64_t)gridDim.x * ENG_TPB)
     a.q[0][i] = a.tree[i];
-  if (!grid_sync(g, bar)) return false;
+  if (!grid_sync(g, bar)) return DEL_GAVE_UP;
   RepQueue rq;
   rq.task = a.task;
   rq.n = &c[C_HVP];
   unsigned long long local = pull_warps<A, W>(g, a.tree, tn, a.mst, warp, nwarps, rq);
-  if (!grid_sync(g, bar)) return false;
+  if (!grid_sync(g, bar)) return DEL_GAVE_UP;
   const uint64_t np = __ldcg(rq.n);
   if (np) {
     for (uint64_t t = warp; t < np; t += nwarps) {
@@ -3641,10 +3668,33 @@ __device__ __noinline__ bool eng_del(const DevGraph &g, const EngineArgs &a, Gri
       pull_slots<A, W, 4>(g, g.in.off[d], k0 + lane_id(), 32, min(len, k0 + TASK_SLOTS), p);
       local += pull_reduce<A>(g, p, d, true, 32, a.mst);
     }
-    if (!grid_sync(g, bar)) return false;
+    if (!grid_sync(g, bar)) return DEL_GAVE_UP;
   }
   warp_add_result(local, &c[C_RESULT]);
-  return true;
+  return DEL_DONE;
+}
+
+// The levels end here, with n vertices in queue k & 1 (all CTAs): the launch after
+// this one starts with queue 0.
+__device__ __noinline__ void eng_leave(const EngineArgs &a, EngShared &sh, unsigned long long what, uint32_t k,
+                                       uint64_t n) {
+  if (k & 1) eng_to_q0(a, n);
+  if (threadIdx.x == 0) {
+    sh.left = what;
+    sh.left_n = n;
+  }
+}
+
+// What the next launch needs: this level begins anew there.
+__device__ __noinline__ void eng_left_words(const DevGraph &g, const EngineArgs &a, const EngShared &sh, uint64_t lvl,
+                                            unsigned pulled) {
+  unsigned long long *c = g.ctl;
+  c[C_QN0] = sh.left_n;
+  c[C_LEVEL] = lvl;
+  c[C_MODE] = M_EMPTY;
+  c[C_BND0] = a.cfg.bnd_best;
+  c[C_PULLED] = pulled != 0;
+  c[C_ELEFT] = sh.left;
 }
 
 // The level kinds as calls: each gets the registers of a thread for itself
@@ -3794,6 +3844,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     sh.g = g_arg;
     sh.a = a_arg;
     sh.bc = BlockCounts{0, 0};
+    sh.left = ELEFT_NONE;
   }
   __syncthreads();
   const DevGraph &g = sh.g;
@@ -3807,7 +3858,7 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   // what the launch before left, read before anything below may change it
   uint32_t st = (uint32_t)__ldcg(&c[C_STAMP]);
   uint64_t lvl = a.build ? 0 : __ldcg(&c[C_LEVEL]);
-  if (lead) a.bar[EB_QN2] = a.bar[EB_HVR] = a.bar[EB_HVE] = 0;
+  if (lead) a.bar[EB_QN2] = a.bar[EB_HVR] = a.bar[EB_HVE] = c[C_ELEFT] = 0;
   if (a.build) {
     init_labels<A>(g, a.root, a.q[0], blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x, (uint64_t)gridDim.x * ENG_TPB);
     if (lead) {
@@ -3818,18 +3869,27 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
     }
   }
   if (!grid_sync(g, bar)) return;
-  if (a.del && !eng_del<A, W>(g, a, bar)) return;
-  bool leave = false;
-  uint64_t n = 0;
+  bool levels = true;
+  if (a.del) {
+    uint64_t n = 0;
+    const DelResult r = eng_del<A, W>(g, a, bar, n);
+    if (r == DEL_GAVE_UP) return;
+    levels = r == DEL_DONE;
+    if (!levels) eng_leave(a, sh, ELEFT_REPAIR, 0, n);
+  }
   unsigned pulled = 0;  // 1: the level before, 2: any level before (one register: two cost 1% of a build)
-  for (uint32_t k = 0;; k++) {
+  for (uint32_t k = 0; levels; k++) {
     const uint32_t *fin = a.q[k & 1];
     uint32_t *fout = a.q[(k & 1) ^ 1];
     unsigned long long *fout_n = cnt(k + 1);
-    n = __ldcg(cnt(k));
+    const uint64_t n = __ldcg(cnt(k));
     if (n == 0) break;
     if (lvl >= a.cfg.max_levels) {
       if (lead) atomicCAS(&c[C_ERR], 0ull, (unsigned long long)RG_ETIMEOUT);
+      break;
+    }
+    if (n > a.half_vertices) {
+      eng_leave(a, sh, ELEFT_LEVELS, k, n);
       break;
     }
     st++;
@@ -3881,12 +3941,12 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
       uint32_t i;
       const uint64_t S = eng_first(a, sh, scan_tmp, (uint32_t)n, per, e0, e1, i);
       pull = a.cfg.allow_pull && S * ENG_PULL_DIV >= a.plan->total;
-      if (!pull && S >= a.push_slots && !(a.del && k == 0)) {
-        // the loop starts with queue 0, which holds the frontier before last now
-        if (k & 1)
-          for (uint64_t x = blockIdx.x * (uint64_t)ENG_TPB + threadIdx.x; x < n; x += (uint64_t)gridDim.x * ENG_TPB)
-            fout[x] = fin[x];
-        leave = true;
+      if (!pull && S >= a.push_slots && !(a.del && k == 0 && n * 20 < g.V)) {
+        eng_leave(a, sh, ELEFT_PUSH, k, n);
+        break;
+      }
+      if (S >= a.half_slots) {
+        eng_leave(a, sh, ELEFT_LEVELS, k, n);
         break;
       }
       for (uint64_t e = e0; e < e1 && !pull;) {
@@ -3918,15 +3978,9 @@ __global__ void __launch_bounds__(ENG_TPB, 1) k_engine(const __grid_constant__ D
   if (!grid_sync(g, bar, blockIdx.x != 0)) return;  // (every CTA has read the last queue counts)
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
-      c[C_QN0] = leave ? n : 0;
+      c[C_QN0] = 0;
       c[C_QN1] = 0;
-      if (leave) {  // (the loop begins this level anew)
-        c[C_LEVEL] = lvl;
-        c[C_MODE] = M_EMPTY;
-        c[C_BND0] = a.cfg.bnd_best;
-        c[C_PULLED] = pulled != 0;
-        c[C_ELEFT] = ELEFT_PUSH;
-      }
+      if (sh.left) eng_left_words(g, a, sh, lvl, pulled);
       if (lvl < TRACE_CAP) g.trace[TRACE_CAP + lvl] = global_ns();
     }
     ctl_to_host(g, a.ctl_host);
@@ -4621,7 +4675,9 @@ bool engine_on(const Graph &g) { return g.eng_ctas && g.cluster_edges && !g.prof
 // One engine launch (see k_engine): build from scratch, or the levels of a
 // repair whose frontier is in queue 0, after the deletion repair when `del`.
 // It ends with the control block in the host's copy.
-// n_edges: the edges of the repair's batch.
+// n_edges: the edges of the repair's batch; ~0 for one that one CTA has run already
+// and that outgrew it (an edge that joins the root to an RMAT-18 graph: 750 us on all
+// SMs, 783 begun on half).
 template <int A, bool W>
 int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edges) {
   EngineArgs a = {};
@@ -4649,13 +4705,15 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edge
   a.max_iter = (uint64_t)g.V + 2;
   a.mst = mod_stamp(g);
   a.polls = g.wait_polls;
+  const int ctas = !build && n_edges <= ENG_HALF_EDGES ? (g.eng_ctas + 1) / 2 : g.eng_ctas;
   a.push_slots = g.push_slots;
+  a.half_vertices = ctas < g.eng_ctas ? g.half_vertices : ~0ull;
+  a.half_slots = ctas < g.eng_ctas ? 32 * g.half_vertices : ~0ull;
   a.build = build ? 1 : 0;
   a.del = del ? 1 : 0;
   g.h_ctl[C_KLAUNCH] = CTL_PENDING;
   count_launch(g);
   void *args[] = {(void *)&g.d, (void *)&a};
-  const int ctas = !build && n_edges <= ENG_HALF_EDGES ? (g.eng_ctas + 1) / 2 : g.eng_ctas;
   RG_CUDA(cudaLaunchCooperativeKernel((const void *)k_engine<A, W>, dim3((unsigned)ctas), dim3(ENG_TPB), args,
                                       sizeof(EngShared), g.stream));
   g.ctl_on_host = true;
@@ -4665,11 +4723,18 @@ int engine_launch(Graph &g, bool build, bool del, uint64_t root, uint64_t n_edge
 // The levels that the engine left, to their end.
 template <int A, bool W>
 int engine_left(Graph &g, bool build) {
-  cudaGraphExec_t exec;
-  const int rc = loop_exec<A, W>(g, build, &exec);
-  if (rc) return rc;
-  RG_CUDA(cudaGraphLaunch(exec, g.stream));
-  return read_ctl(g);
+  while (g.h_ctl[C_ELEFT] && !g.h_ctl[C_ERR]) {
+    int rc = RG_OK;
+    if (g.h_ctl[C_ELEFT] == ELEFT_PUSH) {
+      cudaGraphExec_t exec;
+      if ((rc = loop_exec<A, W>(g, build, &exec))) return rc;
+      RG_CUDA(cudaGraphLaunch(exec, g.stream));
+    } else {
+      rc = engine_launch<A, W>(g, build, g.h_ctl[C_ELEFT] == ELEFT_REPAIR, 0, ~0ull);
+    }
+    if (rc || (rc = read_ctl(g))) return rc;
+  }
+  return RG_OK;
 }
 
 template <int A, bool W>
@@ -5110,7 +5175,7 @@ template <int A, bool W>
 int finish_left(Graph &g, unsigned long long left) {
   int rc = RG_OK;
   if (engine_on(g)) {
-    rc = engine_launch<A, W>(g, false, left == 2 && g.h_ctl[C_OVER], 0, SMALL_EDGES);
+    rc = engine_launch<A, W>(g, false, left == 2 && g.h_ctl[C_OVER], 0, ~0ull);
     return rc ? rc : read_ctl(g);
   }
   if (left == 2) {
@@ -5284,7 +5349,7 @@ int apply_add_del_t(Graph &g, const rg_edge *adds, uint64_t n_add, const rg_edge
     // the insert batch's level loop, then the delete batch in its own kernel
     count_launch(g);
     if (engine_on(g)) {
-      if ((rc = engine_launch<A, W>(g, false, false, 0, n_add))) return rc;
+      if ((rc = engine_launch<A, W>(g, false, false, 0, ~0ull))) return rc;
       g.ctl_on_host = false;  // (the kernel after it writes the host's copy last)
       if ((rc = launch_apply_second<A, W>(g, directed))) return rc;
       RG_CUDA(cudaStreamSynchronize(g.stream));

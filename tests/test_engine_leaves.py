@@ -1,6 +1,7 @@
-"""Push levels that the grid engine leaves to the graph-driven loop, and all that
-follow: from builds and repairs, at frontiers in either queue, and from the
-insert batch of a submission whose delete batch waits for it."""
+"""Work that a launch of the grid engine leaves to another: push levels to the
+graph-driven loop, and repairs on half the SMs, at a level or in the invalidation,
+to a launch on all.  From builds and repairs, at frontiers in either queue, and
+from the insert batch of a submission whose delete batch waits for it."""
 import ctypes
 
 import numpy as np
@@ -18,8 +19,16 @@ SCALE = 15
 SLOTS = [1, 60_000, 300_000, 1 << 40]
 
 
+# vertices of a frontier or a reset set
+VERTICES = [1, 700, 6000]
+
+
 def set_slots(g, n):
     assert rg.lib().rg_test_push_slots(g._h, ctypes.c_uint64(n)) == 0
+
+
+def set_vertices(g, n):
+    assert rg.lib().rg_test_half_vertices(g._h, ctypes.c_uint64(n)) == 0
 
 
 def bridged(algo):
@@ -32,12 +41,28 @@ def bridged(algo):
 
 @pytest.mark.parametrize("algo", ALGOS)
 @pytest.mark.parametrize("slots", SLOTS)
-def test_values_are_those_of_the_loop(algo, slots):
+def test_push_levels_left_to_the_loop(algo, slots):
+    compare(algo, lambda g: set_slots(g, slots))
+
+
+@pytest.mark.parametrize("algo", ALGOS)
+@pytest.mark.parametrize("vertices", VERTICES)
+@pytest.mark.parametrize("slots", [0, 100_000])
+def test_repairs_left_to_all_sms(algo, vertices, slots):
+    def setup(g):
+        set_vertices(g, vertices)
+        set_slots(g, slots)
+
+    compare(algo, setup)
+
+
+def compare(algo, setup):
+    """Updates and builds on a graph with `setup` and on one that runs the loop alone."""
     V, pairs, bridge = bridged(algo)
     directed = algo != "wcc"
     g, h = (rg.Graph(V, len(pairs) + 4096, symmetric=not directed, weighted=WEIGHTED[algo]) for _ in range(2))
     h.set_option("cluster_edges", 0)
-    set_slots(g, slots)
+    setup(g)
     e, b = edges_of(algo, pairs), edges_of(algo, bridge)
     for x in (g, h):
         x.add_pairs(pairs, directed, want_old=False)
@@ -75,6 +100,14 @@ def test_values_are_those_of_the_loop(algo, slots):
     for x in (g, h):
         x.apply_add_del(algo, e[40:90], np.concatenate([b, e[:40]]), directed)
         x.apply_add_del(algo, np.concatenate([b, e[:3000]]), e[3000:6000], directed)
+    same()
+    for x in (g, h):      # many tree edges at once, and back
+        _, par, pw = x.labels()
+        kids = np.nonzero(par < V)[0][::7][:6000]
+        d = np.zeros(len(kids), rg.EDGE_DTYPE)
+        d["src"], d["dst"], d["data"] = par[kids], kids, pw[kids] if WEIGHTED[algo] else 0
+        x.apply_del(algo, d, directed)
+        x.apply_add(algo, d, directed)
     same()
     np.testing.assert_array_equal(g.degrees()[0], h.degrees()[0])
     for x in (g, h):
