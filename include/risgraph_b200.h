@@ -256,8 +256,9 @@ int rg_phase_trace(rg_graph *g, uint64_t *ns);
  *                         launch or more per level (what served graphs do);
  *                         otherwise (default 65536, at most 2^20) the levels
  *                         and deletion repairs of a call run in one persistent
- *                         launch over all SMs, repairs of at most 16,384 edges
- *                         over half of them.  A wait inside it that sees no
+ *                         launch over all SMs, repairs of batches from
+ *                         RG_OPT_FUSED_MAX to 16,384 edges over half of them;
+ *                         very large push levels go to the loop.  A wait inside it that sees no
  *                         progress for about ten seconds ends the call with
  *                         RG_ETIMEOUT, with the labels partly updated as after
  *                         RG_OPT_MAX_LEVELS.  In profile mode, which steps
